@@ -226,6 +226,7 @@ struct qtg_ctx {
     float *intra = nullptr;   // intramolecular forces, 18 floats per molecule and slot
     int4 *sites_fix = nullptr;  // fixed-point site fractions per slot (half-interaction real space)
     long long *rfix = nullptr;  // fixed-point real-space site forces per slot (half-interaction real space)
+    double *real64_tab = nullptr;  // FP64: the real-space pair-function table
     // real-space pair list (mixed contexts with beads beyond the half-interaction
     // kernel in boxes with r_c + 2 RL_SPREAD <= L/2): rl_ok marks the context
     // eligible, rl_form 0 runs the real space over the list there, 1 over all pairs
@@ -395,6 +396,7 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.sites = c->sites;
     a.sites_fix = c->sites_fix;
     a.rfix = c->rfix;
+    a.real64_tab = c->real64_tab;
     a.opos = c->opos;
     a.ljf = c->ljf;
     a.intra = c->intra;
@@ -1313,7 +1315,8 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     AL(ctx->ljf, ctx->total_sites / 3);
     AL(ctx->intra, 6 * ctx->total_sites);
     AL(ctx->sites_fix, ctx->total_sites);
-    if (ctx->mixed) AL(ctx->rfix, 3 * ctx->total_sites);
+    AL(ctx->rfix, (ctx->mixed ? 3 : 6) * ctx->total_sites);
+    if (!ctx->mixed) AL(ctx->real64_tab, (size_t)R64_INTERVALS * 16);
     {
         // real-space pair list: rows hold the molecules whose M sites lie within
         // r_c + RL_SKIN + 2 RL_SPREAD (the prefilter radius of k_rlist_rows), at the
@@ -1394,6 +1397,14 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         if (e == cudaSuccess && bytes) e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
     };
     cp(ctx->sys_d, ctx->sys_h.data(), sizeof(SysDev) * n_systems);
+    if (!ctx->mixed) {
+        static const std::vector<double> tab = [] {  // the same for every system: made once a process
+            std::vector<double> t((size_t)R64_INTERVALS * 16);
+            real64_table(t.data());
+            return t;
+        }();
+        cp(ctx->real64_tab, tab.data(), sizeof(double) * tab.size());
+    }
     cp(ctx->charge, chg_all.data(), sizeof(double) * chg_all.size());
     cp(ctx->mass, mass_all.data(), sizeof(double) * mass_all.size());
     {
@@ -1460,7 +1471,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);

@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(128) k_prep(EvalArgs a) {
         o.w = (R)0;
         reinterpret_cast<V4<R> *>(a.opos)[J.site_off / 3 + mol] = o;
     }
+    if (a.rfix)  // k_real64 adds into it
+        for (int k = 0; k < 6; ++k) a.rfix[6 * ((size_t)J.site_off + s) + k] = 0;
     const double chg = a.charge[S.chg_off + s];
     double frac[3];
     for (int d = 0; d < 3; ++d) {
@@ -1602,6 +1604,11 @@ __global__ void __launch_bounds__(128) k_combine(EvalArgs a) {
                 const double *sf = a.part + 3 * ((size_t)p * a.total_sites + J.site_off + 3 * m);
                 for (int k = 0; k < 9; ++k) fs[k] += sf[k];
             }
+            if (a.real_fix) {  // k_real64's two-limb sums
+                const long long *rf = a.rfix + 6 * ((size_t)J.site_off + 3 * m);
+                for (int k = 0; k < 9; ++k)
+                    fs[k] += fma((double)rf[2 * k], 0.00390625, (double)rf[2 * k + 1] * 8.673617379884035e-19);
+            }
         }
         double fa[9];
         for (int k = 0; k < 9; ++k) fa[k] = 0.0;
@@ -2485,7 +2492,11 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             launch_real_list(a, s);
             if (n) *n += 2;
         } else if (sizeof(R) == 4) k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        else k_real<R, 0><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
+        else {
+            a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
+            a.real_fix = 1;
+            launch_real64(a, s);
+        }
         launch_ksk<R, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
         launch_sk_reduce<R, 0>(a, s);
         if (sizeof(R) == 4) launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
@@ -2533,7 +2544,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
     // the shapes of the stepper's evaluation (forked in the mixed form; the
     // half-interaction real space leaves fixed-point sums instead of planes)
     a.n_rj = chunks_or(a.tune_rj, (long long)tiles * a.n_jobs, MAX_RJ);
-    if (mixed && half_ok(a)) {
+    if (!mixed || half_ok(a)) {
         a.n_rj = 0;
         a.real_fix = 1;
     }
@@ -2550,7 +2561,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         if (mixed && half_ok(a)) launch_real_half(a, s);
         else if (mixed && list_ok(a)) launch_real_list(a, s);
         else if (mixed) k_real_f32<<<gr, RT, 0, s>>>(a);
-        else k_real<double, 0><<<gr, RT, 0, s>>>(a);
+        else launch_real64(a, s);
     } else if (n == "ksk") {
         if (mixed) launch_ksk<float, 0>(a, gk, s);
         else launch_ksk<double, 0>(a, gk, s);
@@ -2578,6 +2589,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
 void init_force_kernel_attributes() {
     set_attrs<float>();
     set_attrs<double>();
+    init_real64_attributes();
 }
 
 void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *n) {

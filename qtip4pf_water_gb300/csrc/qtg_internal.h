@@ -454,6 +454,8 @@ void launch_nm_energy(const SysDev *sys, int sysi, int P, int n_dof, const doubl
 constexpr int MAX_RJ = 16;   // real-space j-chunks
 constexpr int MAX_KC = 16;   // reciprocal-space k-chunks
 constexpr int MAX_SC = 32;   // structure-factor site chunks
+constexpr int R64_LO = -16, R64_HI = 5;  // octaves of (kappa r)^2 in the FP64 pair-function table
+constexpr int R64_INTERVALS = (R64_HI - R64_LO) * 64;
 constexpr int HALF_MAX_TILES = 64;  // half-interaction real space: beads of at most 64 x 32 sites
 constexpr int HALF_MAX_CH = 8;      // its stationary-side chunks
 constexpr int MAX_RPLANES = HALF_MAX_CH + HALF_MAX_TILES / 2 > MAX_RJ ? HALF_MAX_CH + HALF_MAX_TILES / 2 : MAX_RJ;
@@ -507,8 +509,11 @@ struct EvalArgs {
     // (units of 2^-40 Hartree/bohr, [total_sites][3]; zeroed by k_prep_f32, summed by
     // integer atomics, so the sum does not depend on their order), read by
     // k_combine_f32 when real_fix is set
+    // FP64: the same of k_real64, [total_sites][3][2]: a high limb in units of 2^-8 and a
+    // low limb in units of 2^-60 (zeroed by k_prep, read by k_combine)
     long long *rfix;
     int real_fix;
+    const double *real64_tab;  // FP64: the pair-function table (real64_table)
     long long total_sites; // sites summed over all slots (plane stride of part)
     double2 *skp;          // partial S(k) [MAX_SC][total_k]
     double2 *dskp;         // partial dS(k) along the tangent direction
@@ -555,6 +560,12 @@ struct SplineArgs {
     const PairSplines *tables;  // per system
     const double *coef;
 };
+
+// real64.cu: real space of the FP64 form, and its pair-function table (R64_INTERVALS x 16 doubles, host)
+void real64_table(double *tab);
+void init_real64_attributes();
+void launch_real64(const EvalArgs &a, cudaStream_t s);
+
 void launch_pair_splines(const SplineArgs &a, bool mixed, cudaStream_t s, unsigned long long *launches);
 bool bspline_coefficients(const double *y, int n, double h, double dl, double dr, double *c);
 

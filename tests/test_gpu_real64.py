@@ -1,0 +1,45 @@
+"""FP64 real-space Ewald (k_real64) against the oracle at the edges of its tiles,
+packing and pair-function table: ragged and even/odd tile counts, orthorhombic
+cells, an Ewald tolerance whose pairs leave the table at its upper end, and a
+near-contact pair below its lower end. The bound is the FP64 parity bound of the
+force tests (1e-9 relative; summation order is the only difference)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _forces(q, N, P, box, pos, eps):
+    from oracle.binding import Oracle
+
+    o = Oracle(N, P, box, 298.0, 0.25, eps_ewald=eps)
+    s = q.System.create(N, P, box, precision=q.FP64, propagator=q.TROTTER, eps_ewald=eps)
+    point, lst, _ = o.build_lists(pos)
+    ref, got = np.zeros_like(pos), np.zeros_like(pos)
+    e_ref, _ = o.force_eval_trotter(pos, ref, point, lst)
+    e_got, _ = s.force_eval_trotter(pos, got, s.charges(), point, lst)
+    return ref, got, e_ref, e_got
+
+
+# 3N sites: 6 (one ragged tile), 30/33 (one / two tiles), 63, 66 (two, three), 129 (five), 192 (six, full)
+@pytest.mark.parametrize("N,P,eps,ratio", [(2, 1, 1e-6, 1.0), (10, 1, 1e-6, 1.0), (11, 2, 1e-6, 1.2), (21, 1, 1e-6, 1.0),
+                                           (22, 3, 1e-4, 0.9), (43, 1, 1e-6, 1.1), (64, 2, 1e-6, 1.0), (27, 1, 3e-15, 1.0)])
+def test_forces_match_the_oracle(gpu_lib, N, P, eps, ratio):
+    q = gpu_lib
+    st = q.seeded_start(N, P, 298.0, seed=N, density_g_cm3=0.6)
+    box = st.box_bohr * np.array([ratio, 1.0, 1.0 / ratio])
+    pos = np.ascontiguousarray(st.q)
+    ref, got, e_ref, e_got = _forces(q, N, P, box, pos, eps)
+    assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
+    assert abs(e_got - e_ref) < 1e-9 * max(1.0, abs(e_ref))
+
+
+def test_near_contact_pair(gpu_lib):
+    q = gpu_lib
+    st = q.seeded_start(27, 1, 298.0, seed=5)
+    pos = np.ascontiguousarray(st.q)
+    # an H of molecule 1 beside an H of molecule 0: (kappa r)^2 near 2^-22, below the table
+    pos[0, 9 + 3: 9 + 6] = pos[0, 3:6] + np.array([1e-3, 2e-4, -3e-4])
+    ref, got, e_ref, e_got = _forces(q, 27, 1, st.box_bohr, pos, 1e-6)
+    assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
+    assert abs(e_got - e_ref) < 1e-9 * abs(e_ref)
