@@ -407,6 +407,8 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.skp = c->skp;
     a.dskp = c->dskp;
     a.wsk = c->wsk;
+    a.wsk64 = c->wsk;
+    while ((15 << a.kshift) < c->max_kmax || (120 << a.kshift) < c->max_kmax * (c->max_kmax + 1) / 2) ++a.kshift;
     a.wdsk = c->wdsk;
     a.total_k = (long long)c->total_k;
     a.energy = c->energy;
@@ -806,6 +808,7 @@ qtg_status upload_charges(qtg_ctx *ctx, int sys, const double *charge) {
     double self = 0.0;
     for (int i = 0; i < S.n_sites; ++i) self += 0.5 * S.ewald_pref * charge[i] * charge[i];
     S.self_energy = self;
+    set_charge_scale(S, charge, S.n_sites);
     CK(up(ctx, ctx->charge + S.chg_off, charge, sizeof(double) * S.n_sites));
     return refresh_sys(ctx, sys);
 }
@@ -1099,6 +1102,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         double self = 0.0;
         for (int i = 0; i < 3 * N; ++i) self += 0.5 * S.ewald_pref * chg_all[S.chg_off + i] * chg_all[S.chg_off + i];
         S.self_energy = self;
+        set_charge_scale(S, chg_all.data() + S.chg_off, 3 * N);
         ctx->sys_h.push_back(S);
         ctx->max_mols = std::max(ctx->max_mols, N);
         ctx->max_kvec = std::max(ctx->max_kvec, S.n_kvec);
@@ -1110,11 +1114,11 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     // Structure-factor groups: runs of <= kz |kz| values of one column (each |kz|
     // standing for +kz and -kz), one thread each, 128 threads a block. The width
     // (3 or 4) is the one whose launch does less work by a simple model: whole
-    // blocks of threads, each paying the column factor (~7 instructions a site) and
-    // ~9 a |kz| (mixed, the three-multiplication form: ~8 and ~5), over every
-    // system's half set, sites and beads.
+    // blocks of threads, each paying the column factor (~8 instructions a site) and
+    // ~5 a |kz| (FP64, in integer multiply-adds: 16 and 12), over every system's half
+    // set, sites and beads.
     {
-        const double per_col = ctx->mixed ? 8.0 : 7.0, per_kz = ctx->mixed ? 5.0 : 9.0;
+        const double per_col = ctx->mixed ? 8.0 : 16.0, per_kz = ctx->mixed ? 5.0 : 12.0;
         double cost[2] = {0.0, 0.0};
         for (int w = 0; w < 2; ++w) {
             const int kz = 3 + w;
@@ -1347,7 +1351,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     AL(ctx->skp, (size_t)MAX_SC * ctx->total_k);
     AL(ctx->dskp, (size_t)MAX_SC * ctx->total_k);
     AL(ctx->wsk, ctx->total_k);
-    AL(ctx->wpk, 2 * ctx->total_k);
+    AL(ctx->wpk, (ctx->mixed ? 2 : 4) * ctx->total_k);
     AL(ctx->wdsk, ctx->total_k);
     AL(ctx->energy, ctx->total_slots);
     AL(ctx->energy_aux, ctx->total_slots);

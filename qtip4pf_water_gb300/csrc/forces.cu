@@ -103,101 +103,8 @@ __device__ __forceinline__ void pair_terms(double r2, double kap, double kap2, d
     *ec = erfc(kap * r);
 }
 
-// ---- k_prep (FP64 form; the FP32 form is k_prep_f32) ---------------------------
-template <typename R>
-__global__ void __launch_bounds__(128) k_prep(EvalArgs a) {
-    const Job J = a.jobs[blockIdx.y];
-    const SysDev &S = a.sys[J.sys];
-    const int ns = S.n_sites;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) a.energy[J.slot] = 0.0;
-    if (s >= ns) return;
-    const int mol = s / 3, kind = s - 3 * mol;
-    const double *q = a.pos + J.pos_off;
-    const double g = a.c.gamma_vs;
-    double x[3], u[3] = {0.0, 0.0, 0.0};
-    if (a.sites_are_input || kind != 0) {
-        for (int d = 0; d < 3; ++d) x[d] = q[3 * s + d];
-        if (J.mode == 1)
-            for (int d = 0; d < 3; ++d) u[d] = a.dir[J.pos_off + 3 * s + d];
-    } else {
-        // M site (forces.cpp:558-564)
-        for (int d = 0; d < 3; ++d)
-            x[d] = g * q[9 * mol + d] + 0.5 * (1.0 - g) * (q[9 * mol + 3 + d] + q[9 * mol + 6 + d]);
-        if (J.mode == 1) {
-            const double *v = a.dir + J.pos_off;
-            for (int d = 0; d < 3; ++d)
-                u[d] = g * v[9 * mol + d] + 0.5 * (1.0 - g) * (v[9 * mol + 3 + d] + v[9 * mol + 6 + d]);
-        }
-        // wrapped oxygen position for the Lennard-Jones kernel
-        V4<R> o;
-        double w[3];
-        for (int d = 0; d < 3; ++d) {
-            const double t = q[9 * mol + d] * S.inv_box[d];
-            w[d] = (t - floor(t)) * S.box[d];
-        }
-        o.x = (R)w[0];
-        o.y = (R)w[1];
-        o.z = (R)w[2];
-        o.w = (R)0;
-        reinterpret_cast<V4<R> *>(a.opos)[J.site_off / 3 + mol] = o;
-    }
-    if (a.rfix)  // k_real64 adds into it
-        for (int k = 0; k < 6; ++k) a.rfix[6 * ((size_t)J.site_off + s) + k] = 0;
-    const double chg = a.charge[S.chg_off + s];
-    double frac[3];
-    for (int d = 0; d < 3; ++d) {
-        const double t = x[d] * S.inv_box[d];
-        frac[d] = t - floor(t);
-    }
-    V4<R> sv;
-    sv.x = (R)(frac[0] * S.box[0]);
-    sv.y = (R)(frac[1] * S.box[1]);
-    sv.z = (R)(frac[2] * S.box[2]);
-    sv.w = (R)chg;
-    reinterpret_cast<V4<R> *>(a.sites)[J.site_off + s] = sv;
-    if (J.mode == 1) {
-        V4<R> tv;
-        tv.x = (R)u[0];
-        tv.y = (R)u[1];
-        tv.z = (R)u[2];
-        tv.w = (R)0;
-        reinterpret_cast<V4<R> *>(a.tan_sites)[J.site_off + s] = tv;
-    }
-    // phase table exp(i 2 pi m frac_d), layout [(d * (kmax+1) + m) * ns + s], by
-    // complex recursion from exp(i 2 pi frac_d) (as forces.cpp:233-240 does),
-    // reseeded every 4 powers from a directly evaluated phase whose argument
-    // 2 m frac_d is reduced in FP64, so rounding does not accumulate with m (the
-    // FP32 tables of k_prep_f32 reduce it exactly in fixed point)
-    const int km1 = S.k_max + 1;
-    V2<R> *ph = reinterpret_cast<V2<R> *>(a.phase) + J.phase_off;
-    for (int d = 0; d < 3; ++d) {
-        R s1, c1;
-        {
-            double t = 2.0 * frac[d];
-            t -= 2.0 * floor(0.5 * t + 0.5);  // in [-1, 1)
-            f_sincospi((R)t, &s1, &c1);
-        }
-        const R qd = (d == 0) ? (R)chg : (R)1;
-        R cr = (R)1, ci = (R)0;
-        for (int m = 0; m < km1; ++m) {
-            if (m > 0 && (m & 3) == 0) {
-                double t = 2.0 * m * frac[d];
-                t -= 2.0 * floor(0.5 * t + 0.5);
-                f_sincospi((R)t, &ci, &cr);
-            }
-            V2<R> e;
-            e.x = cr * qd;
-            e.y = ci * qd;
-            ph[(size_t)(d * km1 + m) * ns + s] = e;
-            const R nr = cr * c1 - ci * s1;
-            ci = cr * s1 + ci * c1;
-            cr = nr;
-        }
-    }
-}
-
-// FP32 form of k_prep with one thread per (site, dimension): each dimension of
+// ---- k_prep_f32 (mixed; the FP64 form's k_prep64 is in recip64.cu) --------------
+// One thread per (site, dimension): each dimension of
 // the M site, the box fraction, the fixed-point fraction and the phase-table
 // rows depend on that dimension alone. Blocks are dimension-major (a block's
 // threads share d), so the phase rows are written by consecutive sites.
@@ -262,7 +169,7 @@ __global__ void __launch_bounds__(128) k_prep_f32(EvalArgs a) {
         if (d == 0) tv[3] = 0.f;
     }
     // phase row d: exp(i 2 pi m frac) by complex recursion, reseeded every 4 powers
-    // from the exact fixed-point argument m F (see k_prep)
+    // from the exact fixed-point argument m F, so rounding does not accumulate with m
     const int km1 = S.k_max + 1;
     float2 *ph = reinterpret_cast<float2 *>(a.phase) + J.phase_off;
     float s1, c1;
@@ -2443,7 +2350,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     a.n_rj = chunks_or(a.tune_rj, (long long)tiles * a.n_jobs, MAX_RJ);
     a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
-    if (sizeof(R) == 4 && forks && a.mode == 0 && a.lj_full && a.ljf) {
+    if (forks && a.mode == 0 && a.lj_full && a.ljf) {
         // forked: prep; then real space | reciprocal chain | dense LJ; then combine.
         // The reciprocal chain runs beside the real-space kernel: its grids aim for
         // a third (structure factors) and half (k-force) of the blocks a kernel alone
@@ -2484,47 +2391,60 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         if (n) *n += (a.intra_plane ? 8 : 7) + (list_ok(a) ? 2 : 0);
         return;
     }
-    if constexpr (sizeof(R) == 4) launch_prep_f32(a, s);
-    else k_prep<R><<<dim3((ns + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
+    launch_prep_f32(a, s);
     if (a.mode == 0) {
-        if (sizeof(R) == 4 && half_ok(a)) launch_real_half(a, s);
-        else if (sizeof(R) == 4 && list_ok(a)) {
+        if (half_ok(a)) launch_real_half(a, s);
+        else if (list_ok(a)) {
             launch_real_list(a, s);
             if (n) *n += 2;
-        } else if (sizeof(R) == 4) k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        else {
-            a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
-            a.real_fix = 1;
-            launch_real64(a, s);
-        }
+        } else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
         launch_ksk<R, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
         launch_sk_reduce<R, 0>(a, s);
-        if (sizeof(R) == 4) launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
-        else k_kforce<R, 0><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<R>(a.max_kmax), s>>>(a);
+        launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
     } else {
         k_real<R, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
         launch_ksk<R, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
         launch_sk_reduce<R, 1>(a, s);
         k_kforce<R, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<R>(a.max_kmax), s>>>(a);
     }
-    const dim3 gm((a.max_mols + 127) / 128, a.n_jobs);
     // mixed with the dense Lennard-Jones: its oxygen forces go to their plane first,
     // so the combine writes the complete force
-    const bool plane = sizeof(R) == 4 && a.mode == 0 && a.lj_full && a.ljf;
+    const bool plane = a.mode == 0 && a.lj_full && a.ljf;
     if (plane) {
         a.lj_plane = 1;
         launch_lj_dense(a, s);
     }
-    if (sizeof(R) == 4) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
-    else k_combine<double><<<gm, 128, 0, s>>>(a);
+    k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
     if (n) *n += plane ? 7 : 6;
     if (a.mode == 0 && !plane) {
-        if (sizeof(R) == 4 && a.lj_full)
-            launch_lj_dense(a, s);
-        else if (a.lj_full) k_lj<R, 1><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
+        if (a.lj_full) launch_lj_dense(a, s);
         else k_lj<R, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
         if (n) *n += 1;
     }
+}
+
+// Chunk counts of the FP64 reciprocal space: whole 32-site shared-memory chunks of the
+// structure factors, and blocks enough to fill the GPU.
+void set_chunks64(EvalArgs &a) {
+    const int ns = 3 * a.max_mols, tiles = (ns + 127) / 128, ktiles = (a.max_grp + KT - 1) / KT;
+    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, std::min(MAX_SC, (ns + CH - 1) / CH), 6);
+    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
+}
+
+void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n) {
+    set_chunks64(a);
+    a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
+    a.real_fix = 1;
+    launch_prep64(a, s);
+    launch_real64(a, s);
+    launch_ksk64(a, s);
+    launch_sk_reduce64(a, s);
+    launch_kforce64(a, s);
+    k_combine<double><<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
+    const dim3 gl((a.max_mols + 3) / 4, a.n_jobs);
+    if (a.lj_full) k_lj<double, 1><<<gl, 128, 0, s>>>(a);
+    else k_lj<double, 0><<<gl, 128, 0, s>>>(a);
+    if (n) *n += 7;
 }
 
 }  // namespace
@@ -2548,15 +2468,16 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         a.n_rj = 0;
         a.real_fix = 1;
     }
-    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC, mixed ? 4 : 12);
-    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, mixed ? 6 : 12);
-    const dim3 gs((ns + 127) / 128, a.n_jobs), gr(tiles, a.n_rj, a.n_jobs);
+    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC, 4);
+    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
+    if (!mixed) set_chunks64(a);
+    const dim3 gr(tiles, a.n_rj, a.n_jobs);
     const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
     const dim3 gm((a.max_mols + 127) / 128, a.n_jobs), gl((a.max_mols + 3) / 4, a.n_jobs);
     const std::string n(name);
     if (n == "prep") {
         if (mixed) launch_prep_f32(a, s);
-        else k_prep<double><<<gs, 128, 0, s>>>(a);
+        else launch_prep64(a, s);
     } else if (n == "real") {
         if (mixed && half_ok(a)) launch_real_half(a, s);
         else if (mixed && list_ok(a)) launch_real_list(a, s);
@@ -2564,13 +2485,13 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         else launch_real64(a, s);
     } else if (n == "ksk") {
         if (mixed) launch_ksk<float, 0>(a, gk, s);
-        else launch_ksk<double, 0>(a, gk, s);
+        else launch_ksk64(a, s);
     } else if (n == "sk_reduce") {
         if (mixed) launch_sk_reduce<float, 0>(a, s);
-        else launch_sk_reduce<double, 0>(a, s);
+        else launch_sk_reduce64(a, s);
     } else if (n == "kforce") {
         if (mixed) launch_kforce_f32(a, gf, s);
-        else k_kforce<double, 0><<<gf, FT, kforce_smem<double>(a.max_kmax), s>>>(a);
+        else launch_kforce64(a, s);
     } else if (n == "combine") {
         if (mixed) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
         else k_combine<double><<<gm, 128, 0, s>>>(a);
@@ -2588,14 +2509,14 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
 
 void init_force_kernel_attributes() {
     set_attrs<float>();
-    set_attrs<double>();
+    init_recip64_attributes();
     init_real64_attributes();
 }
 
 void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *n) {
     if (a.n_jobs <= 0) return;
     if (!a.sr_only) {
-        launch_ewald<double>(a, s, n);
+        launch_ewald64(a, s, n);
         return;
     }
     // short-range terms only (FP64): LJ reads the raw positions, no preparation pass
@@ -2625,17 +2546,18 @@ void launch_kwald_only(const EvalArgs &a0, bool mixed, cudaStream_t s, unsigned 
     a.n_rj = 0;
     a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
-    const dim3 gs((ns + 127) / 128, a.n_jobs), gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
+    const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
     if (mixed) {
         launch_prep_f32(a, s);
         launch_ksk<float, 0>(a, gk, s);
         launch_sk_reduce<float, 0>(a, s);
         launch_kforce_f32(a, gf, s);
     } else {
-        k_prep<double><<<gs, 128, 0, s>>>(a);
-        launch_ksk<double, 0>(a, gk, s);
-        launch_sk_reduce<double, 0>(a, s);
-        k_kforce<double, 0><<<gf, FT, kforce_smem<double>(a.max_kmax), s>>>(a);
+        set_chunks64(a);
+        launch_prep64(a, s);
+        launch_ksk64(a, s);
+        launch_sk_reduce64(a, s);
+        launch_kforce64(a, s);
     }
     if (mixed) k_sum_parts<float><<<dim3((3 * ns + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
     else k_sum_parts<double><<<dim3((3 * ns + 127) / 128, a.n_jobs), 128, 0, s>>>(a);

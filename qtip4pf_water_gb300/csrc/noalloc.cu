@@ -12,7 +12,7 @@
 // allocates all of its memory up front.
 //
 // Limits: at most QTG_NOALLOC_MAX_SITES charge sites and k_max <=
-// QTG_NOALLOC_MAX_KMAX; the array is 2.76 MiB (2,895,872 bytes) and every GPU that loads the
+// QTG_NOALLOC_MAX_KMAX; the array is 3.29 MiB (3,453,952 bytes) and every GPU that loads the
 // library holds it until the process exits.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -47,13 +47,17 @@ constexpr size_t OFF_PHASE = OFF_SITES + al256(4 * sizeof(double) * NA_MAX_SITES
 constexpr size_t OFF_SKP = OFF_PHASE + al256(2 * sizeof(double) * 3 * (NA_MAX_KMAX + 1) * NA_MAX_SITES);
 constexpr size_t OFF_WSK = OFF_SKP + al256(2 * sizeof(double) * NA_SC * NA_MAX_K);
 constexpr size_t OFF_PART = OFF_WSK + al256(2 * sizeof(double) * NA_MAX_K);
-constexpr size_t OFF_STATUS = OFF_PART + al256(3 * sizeof(double) * NA_KC * NA_MAX_SITES);
+constexpr size_t OFF_WPK = OFF_PART + al256(3 * sizeof(double) * NA_KC * NA_MAX_SITES);
+constexpr size_t OFF_KPK = OFF_WPK + al256(4 * sizeof(int4) * NA_MAX_K);
+constexpr size_t OFF_KFC = OFF_KPK + al256(sizeof(int) * NA_MAX_K);
+constexpr size_t OFF_STATUS = OFF_KFC + al256(sizeof(int4) * NA_COLS);
 constexpr size_t NA_BYTES = OFF_STATUS + 256;
 
 // All scratch of qtg_kwald_noalloc. In host code this name is only a host-side
 // stand-in for the symbol: the device address comes from cudaGetSymbolAddress.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
-static_assert(NA_BYTES == 2895872, "the scratch size stated in the header and comments is out of date");
+static_assert(NA_MAX_KMAX <= 15, "the packed weights' |kz| needs a shift beyond k_max 15");
+static_assert(NA_BYTES == 3453952, "the scratch size stated in the header and comments is out of date");
 
 constexpr int NA_MAX_DEVICES = 64;
 unsigned char *g_scratch_ptr[NA_MAX_DEVICES] = {nullptr};
@@ -118,15 +122,22 @@ __device__ int block_scan_excl(int v, int *sh, int *total) {
     return sh[w] + inc - v;
 }
 
-// Builds the column-ordered k tables and the system / job records in the
-// scratch (one block of 512 threads; every table entry is rewritten, so no
+// Builds the column-ordered k tables, the charge scale and the system / job records
+// in the scratch (one block of 512 threads; every table entry is rewritten, so no
 // state survives from an earlier call) and clears the status word.
-__global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, unsigned char *base) {
+__global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, const double *charge, unsigned char *base) {
     __shared__ int sh[33];
+    __shared__ double top[16];
+    int *kpk = reinterpret_cast<int *>(base + OFF_KPK);
+    int4 *kfc = reinterpret_cast<int4 *>(base + OFF_KFC);
     KVec *kvec = reinterpret_cast<KVec *>(base + OFF_KVEC);
     KCol *kcol = reinterpret_cast<KCol *>(base + OFF_KCOL);
     KGroup *kgrp = reinterpret_cast<KGroup *>(base + OFF_KGRP);
     KBatch *kbat = reinterpret_cast<KBatch *>(base + OFF_KBATCH);
+    double qm = 0.0;  // the largest |charge| (published by the scans' barriers)
+    for (int k = threadIdx.x; k < p.S.n_sites; k += 512) qm = fmax(qm, fabs(charge[k]));
+    for (int o = 16; o > 0; o >>= 1) qm = fmax(qm, __shfl_xor_sync(0xffffffffu, qm, o));
+    if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = qm;
     const int width = 2 * p.kmax + 1, ncol_all = (p.kmax + 1) * width;
     const int t = threadIdx.x;
     int kx = 0, ky = 0, m = -1;
@@ -194,9 +205,18 @@ __global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, unsigned char
             b.k0 = kcol[c0].k_begin;
             b.k1 = kcol[c1 - 1].k_begin + 2 * kcol[c1 - 1].m + 1;
             kbat[nb++] = b;
+            int slot = 0;  // of the column's kz = 0 among the batch's packed weights
+            for (int c = c0; c < c1; ++c) {
+                kfc[c] = make_int4(kcol[c].kx, kcol[c].ky, kcol[c].m, slot);
+                slot += kcol[c].m + 1;
+            }
             c0 = c1;
         }
         SysDev S = p.S;
+        for (int k = 0; k < 16; ++k) qm = fmax(qm, top[k]);
+        const int ex = qm > 0.0 ? ((__double2hiint(qm) >> 20) & 0x7ff) - 1022 : 0;  // qm < 2^ex
+        S.q_scale = __hiloint2double((1023 + ex) << 20, 0);
+        S.inv_q_scale = __hiloint2double((1023 - ex) << 20, 0);
         S.n_kvec = nk;
         S.n_col = ncol;
         S.n_grp = ngrp;
@@ -213,6 +233,9 @@ __global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, unsigned char
         *reinterpret_cast<Job *>(base + OFF_JOB) = J;
         *reinterpret_cast<unsigned *>(base + OFF_STATUS) = 0u;
     }
+    __syncthreads();  // kfc above
+    if (n > 0)
+        for (int kz = -m; kz <= m; ++kz) kpk[kb + kz + m] = kz < 0 ? -1 : (kfc[ci].w + kz) << 8 | kz;
 }
 
 std::mutex g_setup_mutex;
@@ -288,7 +311,7 @@ extern "C" qtg_status qtg_kwald_noalloc(const double *sites, const double *charg
     const qtg_status st = scratch_for_current_device(&base);
     if (st != QTG_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-    k_noalloc_setup<<<1, 512, 0, s>>>(p, base);
+    k_noalloc_setup<<<1, 512, 0, s>>>(p, charge, base);
     EvalArgs a;
     memset(&a, 0, sizeof(a));
     a.sys = reinterpret_cast<const SysDev *>(base + OFF_SYS);
@@ -311,7 +334,11 @@ extern "C" qtg_status qtg_kwald_noalloc(const double *sites, const double *charg
     a.phase = base + OFF_PHASE;
     a.skp = reinterpret_cast<double2 *>(base + OFF_SKP);
     a.total_k = NA_MAX_K;
-    a.wsk = base + OFF_WSK;
+    a.wsk64 = reinterpret_cast<double2 *>(base + OFF_WSK);
+    a.wpk = reinterpret_cast<float4 *>(base + OFF_WPK);
+    a.kpk = reinterpret_cast<const int *>(base + OFF_KPK);
+    a.kfc = reinterpret_cast<const int4 *>(base + OFF_KFC);
+    a.kshift = 0;  // k_max <= 15
     a.part = reinterpret_cast<double *>(base + OFF_PART);
     a.total_sites = NA_MAX_SITES;
     a.energy = energy;

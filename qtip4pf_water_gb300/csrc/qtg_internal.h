@@ -51,6 +51,7 @@ struct SysDev {
     long long mass_off; // doubles: [9N] in mass
     double box[3], inv_box[3];
     double kappa, rc_sq, ewald_pref, k_pref, self_energy;
+    double q_scale, inv_q_scale;  // the power of two at or above the largest |charge|, and its inverse
     double r_cut_sq, r_skin_sq, skin_margin;
     double beta, beta_n, omega_psq, dt, halfdt, eps_sc, c1_centroid, inv_sqrt_beta_n;
     double inv_p, sqrt_inv_p, half_omega_psq, half_nd_beta;  // 1/P, sqrt(1/P), omega_P^2 / 2, n_dof / (2 beta)
@@ -69,6 +70,16 @@ struct SysDev {
     float rc2u, cexu, kau, prefu, s2u, invu;
     unsigned long long seed;
 };
+
+// The charge scale of n site charges (host).
+inline void set_charge_scale(SysDev &S, const double *charge, int n) {
+    double top = 0.0, s = 1.0;
+    for (int i = 0; i < n; ++i) top = charge[i] > top ? charge[i] : -charge[i] > top ? -charge[i] : top;
+    while (s < top && s < 1e300) s *= 2.0;
+    while (top > 0.0 && 0.5 * s >= top) s *= 0.5;
+    S.q_scale = s;
+    S.inv_q_scale = 1.0 / s;
+}
 
 // The FP32 constants above, from the FP64 ones (host).
 inline void set_float_consts(SysDev &S) {
@@ -492,7 +503,8 @@ struct EvalArgs {
     const int *kpk;        // per k (as kvec): kz >= 0: (packed slot in its force batch) << 8 | kz; kz < 0: -1
     const int4 *kfc;       // per column (as kcol): kx, ky, m, packed slot of its kz = 0 (FP32 k-force)
     const float2 *kfb;     // per column: (2 pi / L_x) kx, (2 pi / L_y) ky in FP32
-    float4 *wpk;           // per k slot: the packed +-kz weights P1, P2 of k_kforce_f32 (k_sk_reduce)
+    float4 *wpk;           // per k slot: the packed +-kz weights P1, P2 of k_kforce_f32 (k_sk_reduce);
+                           // FP64: four int4 of limbs (k_sk_reduce64)
     int max_grp, max_batch;
     void *sites;           // 4 reals per site (x, y, z, q), per slot
     int4 *sites_fix;       // mixed: per site the box fractions of x, y, z as 32-bit fixed point
@@ -517,7 +529,9 @@ struct EvalArgs {
     long long total_sites; // sites summed over all slots (plane stride of part)
     double2 *skp;          // partial S(k) [MAX_SC][total_k]
     double2 *dskp;         // partial dS(k) along the tangent direction
-    void *wsk, *wdsk;      // 2 c_k S(k) and 2 c_k dS(k), working precision, per slot
+    void *wsk, *wdsk;      // mixed: 2 c_k S(k) and 2 c_k dS(k), per slot
+    double2 *wsk64;        // FP64: per force batch (at its first k) the worth of its packed weights' unit
+    int kshift;            // FP64: the packed |kz|-weighted force weights carry kz / 2^kshift
     long long total_k;     // k-vectors summed over all slots (plane stride of skp)
     double *energy;        // per slot
     unsigned *status;
@@ -565,6 +579,13 @@ struct SplineArgs {
 void real64_table(double *tab);
 void init_real64_attributes();
 void launch_real64(const EvalArgs &a, cudaStream_t s);
+
+// recip64.cu: site preparation and reciprocal space of the FP64 form
+void init_recip64_attributes();
+void launch_prep64(const EvalArgs &a, cudaStream_t s);
+void launch_ksk64(const EvalArgs &a, cudaStream_t s);
+void launch_sk_reduce64(const EvalArgs &a, cudaStream_t s);
+void launch_kforce64(const EvalArgs &a, cudaStream_t s);
 
 void launch_pair_splines(const SplineArgs &a, bool mixed, cudaStream_t s, unsigned long long *launches);
 bool bspline_coefficients(const double *y, int n, double h, double dl, double dr, double *c);

@@ -16,7 +16,7 @@
 //     order, a lane a site, and added to the configuration's sums as two-limb fixed
 //     point by integer atomics, so the totals do not depend on the order the warps run.
 // 216 waters, 32 beads: 3283 us for k_real<double> (all pairs from both sides, library
-// functions), see launch_real64 for this kernel's times.
+// functions), 337 us here.
 #include <math.h>
 #include <string.h>
 
@@ -242,6 +242,7 @@ void init_real64_attributes() {
     cudaFuncSetAttribute(k_real64, cudaFuncAttributeMaxDynamicSharedMemorySize, RW * (int)sizeof(RWarp));
 }
 
+// 216 waters, 32 beads: 3283 us before, 337 us here; 512 waters 1.22 ms.
 // Chunks of ring distances: enough blocks for a few waves of the six that fit an SM, so
 // that small beads spread over the GPU and the last wave is short.
 void launch_real64(const EvalArgs &a, cudaStream_t s) {
