@@ -866,6 +866,279 @@ __global__ void __launch_bounds__(32 * HW) k_real_half(EvalArgs a, int n_ch) {
     if (lane == 0) atomicAdd(&a.energy[J.slot], (double)e);
 }
 
+// k_real_half for batches that fill the GPU (see launch_real_half), with two sites a
+// lane: a warp holds a tile of 64 sites and visits the half tiles of 32 sites at ring
+// distances d = 1 .. T/2 of 64-site tiles; step r of a visit pairs a lane's two sites
+// with visited site lane + r. The tile's own pairs are one more visit (0). Visits are
+// split over the blocks as blockIdx.y chunks of equal work.
+//
+// What bounds it is instruction issue (two thirds of the pairs lie beyond r_c and cost
+// the same). The two pairs of a step share the visited site's load and its accumulators'
+// shuffles, and their arithmetic is packed (fma / mul .f32x2): 35 issue slots a pair,
+// 51 with one site a lane; the scalar form of the same loop has 45 and is 5 % slower, as
+// a packed instruction holds its port for two slots. 512 waters, 32 beads: 70.0 -> 59.6 us.
+// Two FP32 values in one 64-bit register pair and the packed arithmetic on them.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pk(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpk(F2 p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// 1 where a < b, else 0
+__device__ __forceinline__ float below(float a, float b) {
+    float r;
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// The pair term's constants, in the units of the pair loop (see k_real_half2)
+struct HalfK {
+    float rc2, ka, cex, pref, X0, X1, X2;
+};
+
+// One visit without tests: 32 steps of a lane's two sites (a, b) with the visited
+// half tile's sites vr[0 .. 31] (lane's view of the warp's copy). SCALED: the box is not
+// cubic and integer differences are scaled to bohr, else they stay in fixed-point units.
+// Pairs beyond r_c are evaluated (every term is finite there) and weighted by zero.
+// TEST: a tile's neighbour, whose first sites may belong to the molecule of the tile's
+// last: visited site t of step r is left out where t - ma or t - mb (t counted from the
+// half tile's first site, ma and mb where the lane's molecules begin) is 0, 1 or 2.
+template <bool SCALED, bool TEST>
+__device__ __forceinline__ void half_visit(const int4 *vr, const int4 &a, const int4 &b, const HalfK &K, int ma, int mb,
+                                           F2 &fx, F2 &fy, F2 &fz, F2 &e, float &mx, float &my, float &mz) {
+    const F2 q2 = pk(__int_as_float(a.w), __int_as_float(b.w));
+    const F2 cex = pk(K.cex, K.cex), ka = pk(K.ka, K.ka), one = pk(1.f, 1.f), pref = pk(K.pref, K.pref);
+    const F2 X0 = pk(K.X0, K.X0), X1 = pk(K.X1, K.X1), X2 = pk(K.X2, K.X2);
+    // A&S 7.1.26, as as_poly
+    const F2 c5 = pk(1.061405429f, 1.061405429f), c4 = pk(-1.453152027f, -1.453152027f), c3 = pk(1.421413741f, 1.421413741f),
+             c2 = pk(-0.284496736f, -0.284496736f), c1 = pk(0.254829592f, 0.254829592f);
+    const int nx = (threadIdx.x + 1) & 31;
+#pragma unroll 4
+    for (int r = 0; r < 32; ++r) {
+        const int4 v = vr[r];
+        F2 dx = pk((float)(int)((unsigned)a.x - (unsigned)v.x), (float)(int)((unsigned)b.x - (unsigned)v.x));
+        F2 dy = pk((float)(int)((unsigned)a.y - (unsigned)v.y), (float)(int)((unsigned)b.y - (unsigned)v.y));
+        F2 dz = pk((float)(int)((unsigned)a.z - (unsigned)v.z), (float)(int)((unsigned)b.z - (unsigned)v.z));
+        if (SCALED) {
+            dx = mul2(dx, X0);
+            dy = mul2(dy, X1);
+            dz = mul2(dz, X2);
+        }
+        const F2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        float ra, rb;
+        unpk(r2, ra, rb);
+        const F2 iv = pk(rsqrt_approx(ra), rsqrt_approx(rb));
+        float xa, xb;
+        unpk(mul2(cex, r2), xa, xb);
+        const F2 ex = pk(ex2_approx(xa), ex2_approx(xb));
+        float ta, tb;
+        unpk(fma2(ka, mul2(r2, iv), one), ta, tb);
+        const F2 t = pk(rcp_approx(ta), rcp_approx(tb));
+        const F2 poly = fma2(fma2(fma2(fma2(c5, t, c4), t, c3), t, c2), t, c1);
+        const F2 A = mul2(mul2(mul2(t, poly), ex), iv);
+        const float qv = __int_as_float(v.w);
+        float in_a = below(ra, K.rc2), in_b = below(rb, K.rc2);
+        if (TEST) {
+            const int t = (threadIdx.x + r) & 31;
+            if ((unsigned)(t - ma) < 3u) in_a = 0.f;
+            if ((unsigned)(t - mb) < 3u) in_b = 0.f;
+        }
+        const F2 qq = mul2(mul2(q2, pk(qv, qv)), pk(in_a, in_b));
+        const F2 w = mul2(mul2(qq, fma2(pref, ex, A)), mul2(iv, iv));
+        e = fma2(qq, A, e);
+        fx = fma2(w, dx, fx);
+        fy = fma2(w, dy, fy);
+        fz = fma2(w, dz, fz);
+        float wa, wb, da, db;
+        unpk(w, wa, wb);
+        unpk(dx, da, db);
+        mx = fmaf(-wa, da, fmaf(-wb, db, mx));
+        unpk(dy, da, db);
+        my = fmaf(-wa, da, fmaf(-wb, db, my));
+        unpk(dz, da, db);
+        mz = fmaf(-wa, da, fmaf(-wb, db, mz));
+        mx = __shfl_sync(0xffffffffu, mx, nx);
+        my = __shfl_sync(0xffffffffu, my, nx);
+        mz = __shfl_sync(0xffffffffu, mz, nx);
+    }
+}
+
+// A tile's work units: its own pairs count two (they cost about two visits), then one a
+// visited half tile.
+__host__ __device__ constexpr int half_units(int T) { return 2 + 2 * (T / 2); }
+
+__global__ void __launch_bounds__(32 * HW) k_real_half2(EvalArgs a, int n_ch) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Job J = a.jobs[blockIdx.z];
+    const SysDev &S = a.sys[J.sys];
+    const int ns = S.n_sites, T = (ns + 63) / 64;
+    const int tJ = blockIdx.x * HW + warp;
+    if (tJ >= T) return;
+    const int maxd = T / 2, nu = half_units(T);
+    const int u0 = chunk_lo(nu, blockIdx.y, n_ch), u1 = chunk_lo(nu, blockIdx.y + 1, n_ch);
+    if (u0 >= u1) return;
+    const int4 *sites = a.sites_fix + J.site_off;
+    // cubic box: distances in fixed-point units u = L / 2^32 (the integer differences
+    // themselves), constants scaled to match; forces come out in units of 1 / u^2 and
+    // energies of 1 / u, rescaled after each visit
+    const bool cubic = S.fix_cubic;
+    const HalfK K = cubic ? HalfK{S.rc2u, S.kau, S.cexu, S.prefu, 1.f, 1.f, 1.f}
+                          : HalfK{S.rc_sqf, S.kaf, S.cexf, S.ewald_preff, S.fixf[0], S.fixf[1], S.fixf[2]};
+    const float fscale = cubic ? S.s2u : 1.f, escale = cubic ? S.invu : 1.f;
+    const int sa = tJ * 64 + lane, sb = sa + 32;
+    const bool va = sa < ns, vb = sb < ns;
+    __shared__ int4 vis[HW][64];  // the visited half tile twice over: step r of lane l reads entry l + r
+    int4 pa = make_int4(0, 0, 0, 0), pb = pa;
+    if (va) pa = sites[sa];
+    if (vb) pb = sites[sb];
+    // one pair with all its tests (a tile's own and neighbouring pairs, ragged tiles):
+    // w d is the force on p, the pair's energy is returned
+    auto pair = [&](const int4 &p, const int4 &m, float &dx, float &dy, float &dz, float &w) -> float {
+        dx = (float)(int)((unsigned)p.x - (unsigned)m.x) * K.X0;
+        dy = (float)(int)((unsigned)p.y - (unsigned)m.y) * K.X1;
+        dz = (float)(int)((unsigned)p.z - (unsigned)m.z) * K.X2;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        w = 0.f;
+        if (!(r2 < K.rc2)) return 0.f;
+        const float iv = rsqrt_approx(r2);
+        const float ex = ex2_approx(K.cex * r2);
+        const float t = rcp_approx(fmaf(K.ka, r2 * iv, 1.0f));
+        const float A = (t * as_poly(t)) * ex * iv;
+        const float qq = __int_as_float(p.w) * __int_as_float(m.w);
+        w = qq * fmaf(K.pref, ex, A) * (iv * iv);
+        return qq * A;
+    };
+    float Fa[3] = {0.f, 0.f, 0.f}, Fb[3] = {0.f, 0.f, 0.f}, Ca[3] = {0.f, 0.f, 0.f}, Cb[3] = {0.f, 0.f, 0.f}, e = 0.f;
+    for (int u = u0; u < u1; ++u) {
+        if (u == 1) continue;  // (part of visit 0)
+        const int v = u ? u - 1 : 0, d = (v + 1) >> 1, half = v ? (v - 1) & 1 : 0;
+        if (T % 2 == 0 && d == maxd && d > 0 && tJ >= maxd) continue;  // that pair of tiles is visited from the other
+        const int m0 = ((tJ + d) % T) * 64 + 32 * half;
+        if (m0 >= ns) continue;
+        float fa[3] = {0.f, 0.f, 0.f}, fb[3] = {0.f, 0.f, 0.f}, m[3] = {0.f, 0.f, 0.f}, ev = 0.f;
+        // full tiles: no test a pair, except against the tile's neighbour (visit 1), the only
+        // half tile that can share a molecule (three consecutive sites) with it
+        const bool plain = v > 0 && tJ * 64 + 64 <= ns && m0 + 32 <= ns;
+        if (plain) {
+            const int4 pm = sites[m0 + lane];
+            vis[warp][lane] = pm;
+            vis[warp][lane + 32] = pm;
+            __syncwarp();
+            F2 fx = pk(0.f, 0.f), fy = fx, fz = fx, e2 = fx;
+            const int4 *vr = &vis[warp][lane];
+            const int ma = sa / 3 * 3 - m0, mb = sb / 3 * 3 - m0;
+            if (v == 1) {
+                if (cubic) half_visit<false, true>(vr, pa, pb, K, ma, mb, fx, fy, fz, e2, m[0], m[1], m[2]);
+                else half_visit<true, true>(vr, pa, pb, K, ma, mb, fx, fy, fz, e2, m[0], m[1], m[2]);
+            } else {
+                if (cubic) half_visit<false, false>(vr, pa, pb, K, ma, mb, fx, fy, fz, e2, m[0], m[1], m[2]);
+                else half_visit<true, false>(vr, pa, pb, K, ma, mb, fx, fy, fz, e2, m[0], m[1], m[2]);
+            }
+            __syncwarp();
+            unpk(fx, fa[0], fb[0]);
+            unpk(fy, fa[1], fb[1]);
+            unpk(fz, fa[2], fb[2]);
+            float ea, eb;
+            unpk(e2, ea, eb);
+            ev = ea + eb;
+        } else if (v == 0) {
+            // the tile's own pairs: within each half from both sides, then b with a's half
+            for (int r = 1; r < 32; ++r) {
+                const int src = (lane + r) & 31;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int4 p = h ? pb : pa;
+                    const int s = h ? sb : sa, t = tJ * 64 + 32 * h + src;
+                    int4 q;
+                    q.x = __shfl_sync(0xffffffffu, p.x, src);
+                    q.y = __shfl_sync(0xffffffffu, p.y, src);
+                    q.z = __shfl_sync(0xffffffffu, p.z, src);
+                    q.w = __shfl_sync(0xffffffffu, p.w, src);
+                    if (s >= ns || t >= ns || t / 3 == s / 3) continue;
+                    float dx, dy, dz, w;
+                    ev += 0.5f * pair(p, q, dx, dy, dz, w);
+                    float *f = h ? fb : fa;
+                    f[0] = fmaf(w, dx, f[0]);
+                    f[1] = fmaf(w, dy, f[1]);
+                    f[2] = fmaf(w, dz, f[2]);
+                }
+            }
+            for (int r = 0; r < 32; ++r) {
+                const int src = (lane + r) & 31, t = tJ * 64 + src;
+                int4 q;
+                q.x = __shfl_sync(0xffffffffu, pa.x, src);
+                q.y = __shfl_sync(0xffffffffu, pa.y, src);
+                q.z = __shfl_sync(0xffffffffu, pa.z, src);
+                q.w = __shfl_sync(0xffffffffu, pa.w, src);
+                if (vb && t < ns && t / 3 != sb / 3) {
+                    float dx, dy, dz, w;
+                    ev += pair(pb, q, dx, dy, dz, w);
+                    fb[0] = fmaf(w, dx, fb[0]);
+                    fb[1] = fmaf(w, dy, fb[1]);
+                    fb[2] = fmaf(w, dz, fb[2]);
+                    m[0] = fmaf(-w, dx, m[0]);
+                    m[1] = fmaf(-w, dy, m[1]);
+                    m[2] = fmaf(-w, dz, m[2]);
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) m[k] = __shfl_sync(0xffffffffu, m[k], (lane + 1) & 31);
+            }
+        } else {
+            int4 q = make_int4(0, 0, 0, 0);
+            if (m0 + lane < ns) q = sites[m0 + lane];
+            const int nx = (lane + 1) & 31;
+            for (int r = 0; r < 32; ++r) {
+                const int t = m0 + ((lane + r) & 31);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int s = h ? sb : sa;
+                    if (s >= ns || t >= ns || t / 3 == s / 3) continue;
+                    float dx, dy, dz, w;
+                    ev += pair(h ? pb : pa, q, dx, dy, dz, w);
+                    float *f = h ? fb : fa;
+                    f[0] = fmaf(w, dx, f[0]);
+                    f[1] = fmaf(w, dy, f[1]);
+                    f[2] = fmaf(w, dz, f[2]);
+                    m[0] = fmaf(-w, dx, m[0]);
+                    m[1] = fmaf(-w, dy, m[1]);
+                    m[2] = fmaf(-w, dz, m[2]);
+                }
+                q.x = __shfl_sync(0xffffffffu, q.x, nx);
+                q.y = __shfl_sync(0xffffffffu, q.y, nx);
+                q.z = __shfl_sync(0xffffffffu, q.z, nx);
+                q.w = __shfl_sync(0xffffffffu, q.w, nx);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) m[k] = __shfl_sync(0xffffffffu, m[k], nx);
+            }
+        }
+        if (m0 + lane < ns)
+            rfix_add(a.rfix + 3 * ((size_t)J.site_off + m0 + lane), m[0] * fscale, m[1] * fscale, m[2] * fscale);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            kahan_add(Fa[k], Ca[k], fa[k] * fscale);
+            kahan_add(Fb[k], Cb[k], fb[k] * fscale);
+        }
+        e = fmaf(ev, escale, e);
+    }
+    if (va) rfix_add(a.rfix + 3 * ((size_t)J.site_off + sa), Fa[0] - Ca[0], Fa[1] - Ca[1], Fa[2] - Ca[2]);
+    if (vb) rfix_add(a.rfix + 3 * ((size_t)J.site_off + sb), Fb[0] - Cb[0], Fb[1] - Cb[1], Fb[2] - Cb[2]);
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (lane == 0) atomicAdd(&a.energy[J.slot], (double)e);
+}
+
 // ---- k_ksk: structure factors ---------------------------------------------------
 // One thread per group of <= 4 consecutive |kz| of one (kx, ky) column, each
 // |kz| covering the pair kz = +|kz|, -|kz|; the column factor X(kx) Y(ky) of a
@@ -2305,21 +2578,29 @@ void launch_lj_dense(const EvalArgs &a, cudaStream_t s) {
     else k_lj_dense<32><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
 }
 
-// The half-interaction real-space kernel applies to beads of at most
-// HALF_MAX_TILES tiles; its plane count is n_ch + T / 2 (n_ch from the
-// autotuner's real-space count, else sized for ~12 warps' blocks per SM).
+// The half-interaction real-space kernels apply to beads of at most HALF_MAX_TILES tiles
+// of 32 sites. Two sites a lane where that leaves some 16 warps an SM with one work unit
+// each: 216 waters, 32 beads (4224 warps) 27.1 -> 26.8 us, 512 waters, 32 beads 70.0 ->
+// 59.6 us. Smaller batches leave SMs idle either way, and the shorter chains of one
+// site a lane end sooner: 216 waters, 1 bead 15.3 us against 16.5 us.
 bool half_ok(const EvalArgs &a) { return (3 * a.max_mols + 31) / 32 <= HALF_MAX_TILES; }
-int half_chunks(const EvalArgs &a) {
-    const int T = (3 * a.max_mols + 31) / 32;
-    const long long blocks = (long long)((T + HW - 1) / HW) * a.n_jobs;
-    // the autotuner's picks on the 512-water P = 32 step: the most chunks (20 blocks an SM)
-    return chunks_or(a.tune_rj, blocks, HALF_MAX_CH, 20);
-}
 void launch_real_half(EvalArgs &a, cudaStream_t s) {
-    const int T = (3 * a.max_mols + 31) / 32, n_ch = half_chunks(a);
     a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
     a.real_fix = 1;
-    k_real_half<<<dim3((T + HW - 1) / HW, n_ch, a.n_jobs), 32 * HW, 0, s>>>(a, n_ch);
+    const int T2 = (3 * a.max_mols + 63) / 64, units = half_units(T2);
+    if ((long long)T2 * units * a.n_jobs >= 152LL * 16) {
+        const int gx = (T2 + HW - 1) / HW;
+        int n_ch = chunks_or(a.tune_rj, (long long)gx * a.n_jobs, units, 20);
+        if (a.tune_rj <= 0) {  // whole units: as many chunks as hold units / n_ch (rounded) each
+            const int per = std::max(1, (units + n_ch / 2) / n_ch);
+            n_ch = (units + per - 1) / per;
+        }
+        k_real_half2<<<dim3(gx, n_ch, a.n_jobs), 32 * HW, 0, s>>>(a, n_ch);
+        return;
+    }
+    const int T = (3 * a.max_mols + 31) / 32, gx = (T + HW - 1) / HW;
+    const int n_ch = chunks_or(a.tune_rj, (long long)gx * a.n_jobs, HALF_MAX_CH, 20);
+    k_real_half<<<dim3(gx, n_ch, a.n_jobs), 32 * HW, 0, s>>>(a, n_ch);
 }
 
 // The pair-list real space (mixed, forces, beads beyond the half-interaction

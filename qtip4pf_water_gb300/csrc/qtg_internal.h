@@ -468,9 +468,8 @@ constexpr int MAX_SC = 32;   // structure-factor site chunks
 constexpr int R64_LO = -16, R64_HI = 5;  // octaves of (kappa r)^2 in the FP64 pair-function table
 constexpr int R64_INTERVALS = (R64_HI - R64_LO) * 64;
 constexpr int HALF_MAX_TILES = 64;  // half-interaction real space: beads of at most 64 x 32 sites
-constexpr int HALF_MAX_CH = 8;      // its stationary-side chunks
-constexpr int MAX_RPLANES = HALF_MAX_CH + HALF_MAX_TILES / 2 > MAX_RJ ? HALF_MAX_CH + HALF_MAX_TILES / 2 : MAX_RJ;
-constexpr int MAX_PART = MAX_RPLANES + MAX_KC + 1;  // partial site-force planes
+constexpr int HALF_MAX_CH = 8;      // its stationary-side chunks, one site a lane
+constexpr int MAX_PART = MAX_RJ + MAX_KC + 1;  // partial site-force planes
 // Real-space pair list (mixed form, beads beyond the half-interaction kernel):
 // the distance from its molecule's M site (bohr) within which every charge site
 // of a configuration must lie for one minimum image per molecule pair to serve
