@@ -278,7 +278,8 @@ struct qtg_ctx {
     float2 *kfb = nullptr;   // per column: FP32 reciprocal-lattice components of kx, ky
     float4 *wpk = nullptr;   // packed +-kz force weights, 2 per k slot
     KCol *kcol = nullptr;
-    KGroup *kgrp = nullptr;
+    KGroup *kgrp = nullptr, *kpair = nullptr;
+    int max_pair = 0, pair_threads = 128;
     KBatch *kbatch = nullptr;
     int max_grp = 0, max_batch = 0;
     int kz = 4;  // |kz| values per structure-factor group (3 or 4, chosen at creation)
@@ -385,6 +386,9 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.kvec = c->kvec;
     a.kcol = c->kcol;
     a.kgrp = c->kgrp;
+    a.kpair = c->kpair;
+    a.max_pair = c->max_pair;
+    a.pair_threads = c->pair_threads;
     a.kbatch = c->kbatch;
     a.kpk = c->kpk;
     a.kfc = c->kfc;
@@ -938,7 +942,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     std::vector<int4> kfc_all;
     std::vector<float2> kfb_all;
     std::vector<KCol> call;
-    std::vector<KGroup> gall;
+    std::vector<KGroup> gall, pairall;
     std::vector<KBatch> ball;
     std::vector<double> nm_all;
     std::vector<ModeCoef> mode_all;
@@ -1139,13 +1143,44 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
                     g.col = c;
                     g.kz0 = az0;
                     g.n = std::min(ctx->kz, m - az0 + 1);
-                    g.pad = 0;
+                    g.col2 = -1;
                     gall.push_back(g);
                 }
             }
             S.n_grp = (int)gall.size() - S.grp_off;
             if (S.n_col_half == S.n_col) S.n_grp_half = S.n_grp;
             ctx->max_grp = std::max(ctx->max_grp, S.n_grp);
+        }
+    }
+    // Groups of column pairs (k_ksk2): up to four |kz| of (kx, ky) and (kx, -ky), the low
+    // |kz| of every pair first, so that a block's threads mostly share their |kz|. The
+    // block size is the one whose launch does least by whole blocks: some 36 issue slots a
+    // thread and site, and some 1.5 a thread for each of the 4 (k_max + 1) entries a block
+    // stages of a site.
+    if (ctx->mixed) {
+        double best = 0.0;
+        for (SysDev &S : ctx->sys_h) {
+            std::map<std::pair<int, int>, int> at;
+            for (int c = 0; c < S.n_col_half; ++c) at[{call[S.col_off + c].kx, call[S.col_off + c].ky}] = c;
+            S.pair_off = (int)pairall.size();
+            for (int kz0 = 0; kz0 <= S.k_max; kz0 += 4)
+                for (int c = 0; c < S.n_col_half; ++c) {
+                    const KCol &C = call[S.col_off + c];
+                    if (C.ky < 0 || C.m < kz0) continue;
+                    const auto other = C.ky > 0 ? at.find({C.kx, -C.ky}) : at.end();
+                    pairall.push_back({c, kz0, std::min(4, C.m - kz0 + 1), other == at.end() ? -1 : other->second});
+                }
+            S.n_pair = (int)pairall.size() - S.pair_off;
+            ctx->max_pair = std::max(ctx->max_pair, S.n_pair);
+        }
+        for (int th = 64; th <= 256; th += 32) {
+            double cost = 0.0;
+            for (const SysDev &S : ctx->sys_h)
+                cost += (double)((S.n_pair + th - 1) / th) * (th * 36.0 + 6.0 * (S.k_max + 1) * 1.0) * S.n_sites * S.n_beads;
+            if (th == 64 || cost < best) {
+                best = cost;
+                ctx->pair_threads = th;
+            }
         }
     }
     ctx->total_dof = (size_t)q_off;
@@ -1296,6 +1331,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     AL(ctx->kfb, kfb_all.size());
     AL(ctx->kcol, call.size());
     AL(ctx->kgrp, gall.size());
+    AL(ctx->kpair, pairall.size());
     AL(ctx->kbatch, ball.size());
     AL(ctx->nm, nm_all.size());
     AL(ctx->modes, mode_all.size());
@@ -1426,6 +1462,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     cp(ctx->kfb, kfb_all.data(), sizeof(float2) * kfb_all.size());
     cp(ctx->kcol, call.data(), sizeof(KCol) * call.size());
     cp(ctx->kgrp, gall.data(), sizeof(KGroup) * gall.size());
+    cp(ctx->kpair, pairall.data(), sizeof(KGroup) * pairall.size());
     cp(ctx->kbatch, ball.data(), sizeof(KBatch) * ball.size());
     cp(ctx->nm, nm_all.data(), sizeof(double) * nm_all.size());
     cp(ctx->modes, mode_all.data(), sizeof(ModeCoef) * mode_all.size());
@@ -1475,7 +1512,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);

@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <string>
 
+#include "packed.h"
 #include "qtg_internal.h"
 
 namespace qtg {
@@ -877,26 +878,6 @@ __global__ void __launch_bounds__(32 * HW) k_real_half(EvalArgs a, int n_ch) {
 // shuffles, and their arithmetic is packed (fma / mul .f32x2): 35 issue slots a pair,
 // 51 with one site a lane; the scalar form of the same loop has 45 and is 5 % slower, as
 // a packed instruction holds its port for two slots. 512 waters, 32 beads: 70.0 -> 59.6 us.
-// Two FP32 values in one 64-bit register pair and the packed arithmetic on them.
-struct F2 {
-    unsigned long long v;
-};
-__device__ __forceinline__ F2 pk(float a, float b) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpk(F2 p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
 // 1 where a < b, else 0
 __device__ __forceinline__ float below(float a, float b) {
     float r;
@@ -1145,21 +1126,6 @@ __global__ void __launch_bounds__(32 * HW) k_real_half2(EvalArgs a, int n_ch) {
 // site is formed once and multiplied by Z and conj(Z) with shared products. Sites are staged through shared memory in chunks of CH; each
 // chunk's partial sums (registers, working precision) are added to FP64 running
 // sums kept in shared memory.
-// Asynchronous global -> shared copies (cp.async) of B = 8 or 16 bytes; an invalid
-// source copies nothing and zero-fills the destination.
-template <int B>
-__device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int n = valid ? B : 0;
-    if constexpr (B == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(B), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 constexpr int KT = 128;  // threads (k groups) per block
 constexpr int CH = 32;   // sites per shared-memory chunk
 
@@ -1397,9 +1363,25 @@ __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
         if (sizeof(R) == 4 && MODE == 0) {
             // FP32 form: the site chunks' compensated pairs (S, C), summed in chunk
             // order with compensation in FP32; FP64 only for the energy
-            const float4 *pk = reinterpret_cast<const float4 *>(a.skp) + J.sk_off + k;
             float xs = 0.f, xc = 0.f, ys = 0.f, yc = 0.f;
             int sc = 0;
+            if (a.sk_sites) {  // k_ksk2's sums: no compensation beside them
+                const int n_sc = (S.n_sites + a.sk_sites - 1) / a.sk_sites;
+                const float2 *pp = reinterpret_cast<const float2 *>(a.skp) + J.sk_off + k;
+                for (int c0 = 0; c0 < n_sc; c0 += 8) {
+                    float2 p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        p[u] = c0 + u < n_sc ? pp[(size_t)(c0 + u) * a.total_k] : make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        kahan_add(xs, xc, p[u].x);
+                        kahan_add(ys, yc, p[u].y);
+                    }
+                }
+                sc = a.n_sc;
+            }
+            const float4 *pk = reinterpret_cast<const float4 *>(a.skp) + J.sk_off + k;
             for (; sc + 4 <= a.n_sc; sc += 4) {  // four chunks' loads in flight, then their sums in order
                 float4 p[4];
 #pragma unroll
@@ -2624,6 +2606,32 @@ void launch_real_list(EvalArgs &a, cudaStream_t s) {
     k_real_list<<<dim3((a.max_mols + RLW - 1) / RLW, a.n_rj, a.n_jobs), 32 * RLW, 0, s>>>(a);
 }
 
+// Whether a mixed evaluation's structure factors come from k_ksk2: batches of some 2000
+// waters' sites and more (one bead of 216 waters leaves either kernel mostly latency:
+// 6.2 us), with at most 192 sites a block within its planes.
+bool ksk2_ok(const EvalArgs &a) {
+    return a.mode == 0 && a.kpair && 3 * a.max_mols <= MAX_SC2 * 192 && a.max_kmax <= 32 &&
+           (long long)a.max_mols * a.n_jobs >= 2048;
+}
+// Its site chunks, of the same size for every system of the batch: at most 192 sites, and
+// about a block an SM (the real-space kernel runs beside it). 512 waters, 32 beads: 8 chunks
+// 199.5 us a step, 16 chunks 201.0; 343 waters, 16 beads: 8 chunks 104.5, 28 chunks 110.8.
+void set_ksk2_chunks(EvalArgs &a) {
+    const int ns = 3 * a.max_mols;
+    a.n_sc = std::max(chunks_or(a.tune_sc, (long long)ksk2_blocks(a) * a.n_jobs, MAX_SC2, 1), (ns + 191) / 192);
+    a.sk_sites = std::max(16, ((ns + a.n_sc - 1) / a.n_sc + 15) / 16 * 16);
+    a.n_sc = (ns + a.sk_sites - 1) / a.sk_sites;
+}
+
+// The reciprocal chain of a mixed evaluation, with a's chunk counts.
+void launch_recip(const EvalArgs &a, cudaStream_t s) {
+    const int ns = 3 * a.max_mols, tiles = (ns + FT - 1) / FT, ktiles = (a.max_grp + KT - 1) / KT;
+    if (ksk2_ok(a)) launch_ksk2(a, s);
+    else launch_ksk<float, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
+    launch_sk_reduce<float, 0>(a, s);
+    launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
+}
+
 template <typename R>
 void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks *forks = nullptr) {
     const int ns = 3 * a.max_mols;
@@ -2631,6 +2639,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     a.n_rj = chunks_or(a.tune_rj, (long long)tiles * a.n_jobs, MAX_RJ);
     a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
+    if (ksk2_ok(a)) set_ksk2_chunks(a);
     if (forks && a.mode == 0 && a.lj_full && a.ljf) {
         // forked: prep; then real space | reciprocal chain | dense LJ; then combine.
         // The reciprocal chain runs beside the real-space kernel: its grids aim for
@@ -2638,6 +2647,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         // would (the autotuner's picks on the 512-water P = 32 step)
         a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC, 4);
         a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
+        if (ksk2_ok(a)) set_ksk2_chunks(a);
         if (half_ok(a)) {  // k_kforce_f32's planes follow the real-space ones: none here
             a.n_rj = 0;
             a.real_fix = 1;
@@ -2652,9 +2662,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         cudaEventRecord(forks->fork, s);
         cudaStreamWaitEvent(forks->side[0], forks->fork, 0);
         cudaStreamWaitEvent(forks->side[1], forks->fork, 0);
-        launch_ksk<R, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), forks->side[0]);
-        launch_sk_reduce<R, 0>(a, forks->side[0]);
-        launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), forks->side[0]);
+        launch_recip(a, forks->side[0]);
         cudaEventRecord(forks->join[0], forks->side[0]);
         if (a.lj_list && forks->lists_ready) cudaStreamWaitEvent(forks->side[1], forks->lists_ready, 0);
         launch_lj_dense(a, forks->side[1]);
@@ -2679,9 +2687,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             launch_real_list(a, s);
             if (n) *n += 2;
         } else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        launch_ksk<R, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
-        launch_sk_reduce<R, 0>(a, s);
-        launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
+        launch_recip(a, s);
     } else {
         k_real<R, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
         launch_ksk<R, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
@@ -2752,6 +2758,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
     a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC, 4);
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
     if (!mixed) set_chunks64(a);
+    else if (ksk2_ok(a)) set_ksk2_chunks(a);
     const dim3 gr(tiles, a.n_rj, a.n_jobs);
     const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
     const dim3 gm((a.max_mols + 127) / 128, a.n_jobs), gl((a.max_mols + 3) / 4, a.n_jobs);
@@ -2765,7 +2772,8 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         else if (mixed) k_real_f32<<<gr, RT, 0, s>>>(a);
         else launch_real64(a, s);
     } else if (n == "ksk") {
-        if (mixed) launch_ksk<float, 0>(a, gk, s);
+        if (mixed && ksk2_ok(a)) launch_ksk2(a, s);
+        else if (mixed) launch_ksk<float, 0>(a, gk, s);
         else launch_ksk64(a, s);
     } else if (n == "sk_reduce") {
         if (mixed) launch_sk_reduce<float, 0>(a, s);
@@ -2790,6 +2798,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
 
 void init_force_kernel_attributes() {
     set_attrs<float>();
+    init_recip32_attributes();
     init_recip64_attributes();
     init_real64_attributes();
 }
@@ -2827,12 +2836,10 @@ void launch_kwald_only(const EvalArgs &a0, bool mixed, cudaStream_t s, unsigned 
     a.n_rj = 0;
     a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
-    const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
     if (mixed) {
+        if (ksk2_ok(a)) set_ksk2_chunks(a);
         launch_prep_f32(a, s);
-        launch_ksk<float, 0>(a, gk, s);
-        launch_sk_reduce<float, 0>(a, s);
-        launch_kforce_f32(a, gf, s);
+        launch_recip(a, s);
     } else {
         set_chunks64(a);
         launch_prep64(a, s);

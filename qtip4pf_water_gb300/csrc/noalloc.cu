@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, const double 
             G.col = ci;
             G.kz0 = 4 * g;
             G.n = min(4, m - G.kz0 + 1);
-            G.pad = 0;
+            G.col2 = -1;
             kgrp[gi + g] = G;
         }
     }

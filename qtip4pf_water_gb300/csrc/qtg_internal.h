@@ -32,6 +32,7 @@ struct SysDev {
     // conj S(k) for real charges; their kx = 0, ky > 0 partners count twice):
     // those columns come last, so the kept groups, batches and k entries are prefixes
     int n_grp_half, n_batch_half, n_kvec_half, n_col_half;
+    int pair_off, n_pair;        // the half set as groups of column pairs (k_ksk2)
     int centroid_fixed;          // 1: the centroid is held fixed (centroid-constrained PIMD)
     // Verlet-list build: cell grid of side >= r_skin / 2 (lc_n cells a side, lc_cells in
     // all; 0 cells: boxes under five cells a side scan every molecule), cell starts of
@@ -130,8 +131,10 @@ struct KCol {
 };
 // Structure-factor work item: up to 4 consecutive |kz| of one column, starting
 // at kz0 >= 0; each |kz| stands for the pair kz = +|kz|, -|kz|.
+// (Of the pair list, see k_ksk2: of the two columns (kx, ky >= 0) and (kx, -ky); col2 < 0:
+// the first alone.)
 struct KGroup {
-    int col, kz0, n, pad;
+    int col, kz0, n, col2;
 };
 // Reciprocal-force work item: whole columns [c0, c1) holding k in [k0, k1), k1 - k0 <= 128.
 struct KBatch {
@@ -465,6 +468,7 @@ void launch_nm_energy(const SysDev *sys, int sysi, int P, int n_dof, const doubl
 constexpr int MAX_RJ = 16;   // real-space j-chunks
 constexpr int MAX_KC = 16;   // reciprocal-space k-chunks
 constexpr int MAX_SC = 32;   // structure-factor site chunks
+constexpr int MAX_SC2 = 2 * MAX_SC;  // the same of k_ksk2, whose partial sums are half as large
 constexpr int R64_LO = -16, R64_HI = 5;  // octaves of (kappa r)^2 in the FP64 pair-function table
 constexpr int R64_INTERVALS = (R64_HI - R64_LO) * 64;
 constexpr int HALF_MAX_TILES = 64;  // half-interaction real space: beads of at most 64 x 32 sites
@@ -498,6 +502,8 @@ struct EvalArgs {
     const KVec *kvec;
     const KCol *kcol;
     const KGroup *kgrp;
+    const KGroup *kpair;     // mixed: groups of column pairs (k_ksk2)
+    int max_pair, pair_threads;
     const KBatch *kbatch;
     const int *kpk;        // per k (as kvec): kz >= 0: (packed slot in its force batch) << 8 | kz; kz < 0: -1
     const int4 *kfc;       // per column (as kcol): kx, ky, m, packed slot of its kz = 0 (FP32 k-force)
@@ -526,7 +532,8 @@ struct EvalArgs {
     int real_fix;
     const double *real64_tab;  // FP64: the pair-function table (real64_table)
     long long total_sites; // sites summed over all slots (plane stride of part)
-    double2 *skp;          // partial S(k) [MAX_SC][total_k]
+    double2 *skp;          // partial S(k) [MAX_SC][total_k] (k_ksk2: float2 [MAX_SC2][total_k])
+    int sk_sites;          // nonzero: skp holds k_ksk2's plain FP32 sums, of this many sites each
     double2 *dskp;         // partial dS(k) along the tangent direction
     void *wsk, *wdsk;      // mixed: 2 c_k S(k) and 2 c_k dS(k), per slot
     double2 *wsk64;        // FP64: per force batch (at its first k) the worth of its packed weights' unit
@@ -573,6 +580,11 @@ struct SplineArgs {
     const PairSplines *tables;  // per system
     const double *coef;
 };
+
+// recip32.cu: structure factors of the mixed form for batches that fill the GPU
+void init_recip32_attributes();
+int ksk2_blocks(const EvalArgs &a);
+void launch_ksk2(const EvalArgs &a, cudaStream_t s);
 
 // real64.cu: real space of the FP64 form, and its pair-function table (R64_INTERVALS x 16 doubles, host)
 void real64_table(double *tab);
