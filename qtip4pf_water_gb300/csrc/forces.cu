@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "packed.h"
 #include "qtg_internal.h"
@@ -2220,9 +2221,9 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
 //
 // Pairs whose FP32 r^2 lies in a narrow band around r_cut^2, or that sit at a
 // half-box tie where half a box is inside r_cut, must take the reference's FP64
-// arithmetic (as in k_lj). They are rare, and that FP64 code is kept out of the
-// main loop: the loop skips them and raises a block flag, and only blocks that
-// saw one run a second pass that evaluates exactly those pairs.
+// arithmetic (as in k_lj). They are rare (some three a bead of 512 waters), and that FP64
+// code is kept out of the main loop, which notes a lane's first two for afterwards; only
+// a block with a lane that met more runs a second pass to find them again.
 constexpr int LJD_CH = 1024;                // oxygens per shared-memory chunk
 
 struct LjdConst {
@@ -2231,14 +2232,16 @@ struct LjdConst {
 };
 
 // 0: outside r_cut; 1: inside, displacement in r; 2: needs the FP64 decision
+// (TIE: with the half-box tie test; without it for boxes in which no tie matters)
+template <bool TIE>
 __device__ __forceinline__ int ljd_classify(const float4 &oi, const float4 &o, const LjdConst &K, float *r,
                                             float *rr) {
     const float dx = oi.x - o.x, dy = oi.y - o.y, dz = oi.z - o.z;
     const float tx = dx * K.I[0], ty = dy * K.I[1], tz = dz * K.I[2];
     // wrapped positions lie in [0, L]: |t| <= 1, and two images tie at |t| = 1/2
-    const bool tie = ((K.tie_mask & 1) && fabsf(fabsf(tx) - 0.5f) < K.tie) ||
+    const bool tie = TIE && (((K.tie_mask & 1) && fabsf(fabsf(tx) - 0.5f) < K.tie) ||
                      ((K.tie_mask & 2) && fabsf(fabsf(ty) - 0.5f) < K.tie) ||
-                     ((K.tie_mask & 4) && fabsf(fabsf(tz) - 0.5f) < K.tie);
+                     ((K.tie_mask & 4) && fabsf(fabsf(tz) - 0.5f) < K.tie));
     r[0] = fmaf(-K.L[0], rintf(tx), dx);
     r[1] = fmaf(-K.L[1], rintf(ty), dy);
     r[2] = fmaf(-K.L[2], rintf(tz), dz);
@@ -2292,42 +2295,54 @@ __global__ void __launch_bounds__(128) k_lj_dense(EvalArgs a) {
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
     if (act) oi = opos[i];
     float fx = 0.f, fy = 0.f, fz = 0.f, el = 0.f;
-    int flagged = 0;
+    int nf = 0, f0 = 0, f1 = 0;  // pairs that need the FP64 decision: their number and the first two
+    auto pairs = [&](auto tie, int t0, int nj) {
+#pragma unroll 4
+        for (int jj = sub; jj < nj; jj += LJD_SUB) {
+            float r[3], rr;
+            const int c = ljd_classify<decltype(tie)::value>(oi, sj[jj], K, r, &rr);
+            if (c == 1 && t0 + jj != i) ljd_pair(r, rr, K, fx, fy, fz, el);
+            if (c == 2) {
+                if (nf == 0) f0 = t0 + jj;
+                else f1 = t0 + jj;
+                ++nf;
+            }
+        }
+    };
     for (int t0 = 0; t0 < N; t0 += LJD_CH) {
         const int nj = min(LJD_CH, N - t0);
         __syncthreads();
         for (int k = threadIdx.x; k < nj; k += 128) sj[k] = opos[t0 + k];
         __syncthreads();
         if (!act) continue;
-#pragma unroll 4
-        for (int jj = sub; jj < nj; jj += LJD_SUB) {
-            float r[3], rr;
-            const int c = ljd_classify(oi, sj[jj], K, r, &rr);
-            if (c == 1 && t0 + jj != i) ljd_pair(r, rr, K, fx, fy, fz, el);
-            flagged |= (c == 2);
-        }
+        // (no box side within twice the cutoff: no tie test a pair)
+        if (K.tie_mask) pairs(std::true_type{}, t0, nj);
+        else pairs(std::false_type{}, t0, nj);
     }
-    // second pass, only in blocks that saw a pair needing the FP64 decision
-    if (__syncthreads_or(flagged)) {
-        const double *q = a.pos + J.pos_off;
+    const double *q = a.pos + J.pos_off;
+    auto decide = [&](int j) {
+        double rd[3];
+        const double r2d = lj_exact_disp(q + 9 * i, q + 9 * j, S, rd);
+        if (r2d < rc2) {
+            const float r[3] = {(float)rd[0], (float)rd[1], (float)rd[2]};
+            ljd_pair(r, (float)r2d, K, fx, fy, fz, el);
+        }
+    };
+    if (nf == 1 || nf == 2) {
+        if (f0 != i) decide(f0);
+        if (nf == 2 && f1 != i) decide(f1);
+    }
+    // more than two of a lane: a second pass finds them again, in such blocks only
+    if (__syncthreads_or(nf > 2)) {
         for (int t0 = 0; t0 < N; t0 += LJD_CH) {
             const int nj = min(LJD_CH, N - t0);
             __syncthreads();
             for (int k = threadIdx.x; k < nj; k += 128) sj[k] = opos[t0 + k];
             __syncthreads();
-            if (!act || !flagged) continue;
+            if (!act || nf <= 2) continue;
             for (int jj = sub; jj < nj; jj += LJD_SUB) {
-                const int j = t0 + jj;
                 float r[3], rr;
-                if (j == i || ljd_classify(oi, sj[jj], K, r, &rr) != 2) continue;
-                double rd[3];
-                const double r2d = lj_exact_disp(q + 9 * i, q + 9 * j, S, rd);
-                if (r2d < rc2) {
-                    r[0] = (float)rd[0];
-                    r[1] = (float)rd[1];
-                    r[2] = (float)rd[2];
-                    ljd_pair(r, (float)r2d, K, fx, fy, fz, el);
-                }
+                if (t0 + jj != i && ljd_classify<true>(oi, sj[jj], K, r, &rr) == 2) decide(t0 + jj);
             }
         }
     }
@@ -2428,7 +2443,7 @@ __global__ void __launch_bounds__(128) k_lj_list_f32(EvalArgs a) {
                     continue;
                 }
                 float r[3], rr;
-                const int c = ljd_classify(oi, ov[u], K, r, &rr);
+                const int c = ljd_classify<true>(oi, ov[u], K, r, &rr);
                 if (c == 1) ljd_pair(r, rr, K, fx, fy, fz, el);
                 flagged |= (c == 2);
             }
@@ -2440,7 +2455,7 @@ __global__ void __launch_bounds__(128) k_lj_list_f32(EvalArgs a) {
             for (int n = n0 + lane; n < n1; n += 32) {
                 const int j = ls[n];
                 float r[3], rr;
-                if (j == i || j < 0 || j >= N || ljd_classify(oi, opos[j], K, r, &rr) != 2) continue;
+                if (j == i || j < 0 || j >= N || ljd_classify<true>(oi, opos[j], K, r, &rr) != 2) continue;
                 double rd[3];
                 const double r2d = lj_exact_disp(q + 9 * i, q + 9 * j, S, rd);
                 if (r2d < C.r_cut_sq) {
