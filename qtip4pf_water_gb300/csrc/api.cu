@@ -59,6 +59,7 @@ Consts make_consts() {
     K.ljf[3] = (float)(24.0 * K.epslj);
     K.ljf[4] = (float)K.e_cut;
     K.ljf[5] = (float)K.r_cut_sq;
+    K.ljf[6] = (float)K.r_cut;
     return K;
 }
 
@@ -287,6 +288,8 @@ struct qtg_ctx {
     ModeCoef *modes = nullptr;
     // per-slot scratch
     void *sites = nullptr, *tan_sites = nullptr, *phase = nullptr, *opos = nullptr;
+    float4 *opos32 = nullptr;  // FP64 evaluations: wrapped oxygens in FP32, and the Lennard-Jones forces
+    double *lj64 = nullptr;
     double *part = nullptr;           // [MAX_PART][total_sites][3]
     double2 *skp = nullptr, *dskp = nullptr;  // [MAX_SC][total_k]
     double2 *wsk = nullptr, *wdsk = nullptr;  // [total_k] (sized for FP64)
@@ -402,6 +405,8 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.rfix = c->rfix;
     a.real64_tab = c->real64_tab;
     a.opos = c->opos;
+    a.opos32 = c->opos32;
+    a.lj64 = c->lj64;
     a.ljf = c->ljf;
     a.intra = c->intra;
     a.phase = c->phase;
@@ -1348,10 +1353,12 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         ctx->phase = tmp;
     }
     {
-        double *tmp = nullptr;
-        AL(tmp, 4 * (ctx->total_sites / 3));
+        float4 *tmp = nullptr;
+        AL(tmp, ctx->total_sites / 3);
         ctx->opos = tmp;
     }
+    AL(ctx->opos32, ctx->total_sites / 3);
+    AL(ctx->lj64, 4 * (ctx->total_sites / 3));
     AL(ctx->ljf, ctx->total_sites / 3);
     AL(ctx->intra, 6 * ctx->total_sites);
     AL(ctx->sites_fix, ctx->total_sites);
@@ -1512,7 +1519,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair, ctx->opos32, ctx->lj64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);

@@ -1835,8 +1835,9 @@ __global__ void __launch_bounds__(128) k_combine(EvalArgs a) {
         }
         // M-site chain rule (forces.cpp:613-619)
         const double g = a.c.gamma_vs, h = 0.5 * (1.0 - g);
+        const double *lj = a.lj64 + 4 * ((size_t)J.site_off / 3 + m);
         for (int d = 0; d < 3; ++d) {
-            f[d] = fa[d] + g * fs[d];
+            f[d] = (fa[d] + g * fs[d]) + lj[d];
             f[3 + d] = fa[3 + d] + fs[3 + d] + h * fs[d];
             f[6 + d] = fa[6 + d] + fs[6 + d] + h * fs[d];
         }
@@ -2725,6 +2726,13 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     }
 }
 
+// A warp a block: the molecules' chains of FP64 library functions are long, and a small
+// batch's warps are spread over the SMs (512 waters, 16 configurations: 28.6 us with four
+// warps a block).
+void launch_combine64(const EvalArgs &a, cudaStream_t s) {
+    k_combine<double><<<dim3((a.max_mols + 31) / 32, a.n_jobs), 32, 0, s>>>(a);
+}
+
 // Chunk counts of the FP64 reciprocal space: whole 32-site shared-memory chunks of the
 // structure factors, and blocks enough to fill the GPU.
 void set_chunks64(EvalArgs &a) {
@@ -2742,10 +2750,8 @@ void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n) {
     launch_ksk64(a, s);
     launch_sk_reduce64(a, s);
     launch_kforce64(a, s);
-    k_combine<double><<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
-    const dim3 gl((a.max_mols + 3) / 4, a.n_jobs);
-    if (a.lj_full) k_lj<double, 1><<<gl, 128, 0, s>>>(a);
-    else k_lj<double, 0><<<gl, 128, 0, s>>>(a);
+    launch_lj64(a, s);
+    launch_combine64(a, s);
     if (n) *n += 7;
 }
 
@@ -2776,7 +2782,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
     else if (ksk2_ok(a)) set_ksk2_chunks(a);
     const dim3 gr(tiles, a.n_rj, a.n_jobs);
     const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
-    const dim3 gm((a.max_mols + 127) / 128, a.n_jobs), gl((a.max_mols + 3) / 4, a.n_jobs);
+    const dim3 gl((a.max_mols + 3) / 4, a.n_jobs);
     const std::string n(name);
     if (n == "prep") {
         if (mixed) launch_prep_f32(a, s);
@@ -2798,15 +2804,14 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         else launch_kforce64(a, s);
     } else if (n == "combine") {
         if (mixed) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
-        else k_combine<double><<<gm, 128, 0, s>>>(a);
+        else launch_combine64(a, s);
     } else if (n == "lj") {
         if (mixed) {
             if (a.lj_full && a.ljf) a.lj_plane = 1;  // as the stepper's forked evaluation
             if (a.lj_full) launch_lj_dense(a, s);
             else k_lj<float, 0><<<gl, 128, 0, s>>>(a);
         } else {
-            if (a.lj_full) k_lj<double, 1><<<gl, 128, 0, s>>>(a);
-            else k_lj<double, 0><<<gl, 128, 0, s>>>(a);
+            launch_lj64(a, s);
         }
     }
 }
@@ -2824,12 +2829,11 @@ void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *n) 
         launch_ewald64(a, s, n);
         return;
     }
-    // short-range terms only (FP64): LJ reads the raw positions, no preparation pass
-    const dim3 gm((a.max_mols + 127) / 128, a.n_jobs);
-    k_combine<double><<<gm, 128, 0, s>>>(a);
-    if (a.lj_full) k_lj<double, 1><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
-    else k_lj<double, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
-    if (n) *n += 2;
+    // short-range terms only (FP64)
+    launch_lj64_prep(a, s);
+    launch_lj64(a, s);
+    launch_combine64(a, s);
+    if (n) *n += 3;
 }
 
 void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *n, const Forks *forks) {

@@ -1,0 +1,175 @@
+// O-O Lennard-Jones of the FP64 form over the Verlet list (forces.cpp:25-59, :489-515).
+//
+// One warp per list row. What bounds it is FP64 issue (a warp's FP64 instruction takes
+// sixteen cycles of an SM), and of the list's pairs, which reach to r_skin = 1.3 r_cut,
+// only 45 % lie inside r_cut. So the entries are screened in FP32 on wrapped positions,
+// with a margin above their rounding, and the pairs that pass are packed into full warps
+// before anything is done in FP64: 216 waters, 32 beads 151 us for the former kernel,
+// which took every entry's image and cutoff in FP64 (launch_lj64 states this one's).
+//
+// The pair's displacement and the cutoff decision r^2 < r_cut^2 are the reference's: a
+// pair within 1e-12 of the cutoff, or near half a box in some dimension (where the two
+// images tie and the rounding rule picks the sign), is recomputed with its arithmetic
+// (x - L round(x / L), each operation rounded).
+//
+// FULL: the stepper's symmetric list; a row's force needs no atomics and the energy is
+// halved. Else the caller's half list (entries j > i), forces added by atomics. The oxygen
+// forces go to their own array, which k_combine adds, so that the kernel can run beside
+// the Ewald kernels.
+#include <math.h>
+
+#include "qtg_internal.h"
+
+namespace qtg {
+
+namespace {
+
+__device__ double lj64_exact(const double *qi, const double *qj, const SysDev &S, double *r) {
+    double r2 = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        double x = __dsub_rn(qi[d], qj[d]);
+        x = __dsub_rn(x, __dmul_rn(S.box[d], round(__ddiv_rn(x, S.box[d]))));
+        r[d] = x;
+        r2 = (d == 0) ? __dmul_rn(x, x) : __dadd_rn(r2, __dmul_rn(x, x));
+    }
+    return r2;
+}
+
+// Wrapped FP32 oxygens and cleared forces, where no preparation pass made them (the
+// displaced configurations of the Suzuki-Chin force gradient).
+__global__ void __launch_bounds__(128) k_lj64_prep(EvalArgs a) {
+    const Job J = a.jobs[blockIdx.y];
+    const SysDev &S = a.sys[J.sys];
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= S.n_mols) return;
+    float w[3];
+    for (int d = 0; d < 3; ++d) {
+        const double t = a.pos[J.pos_off + 9 * m + d] * S.inv_box[d];
+        w[d] = (float)((t - floor(t)) * S.box[d]);
+        a.lj64[4 * ((size_t)J.site_off / 3 + m) + d] = 0.0;
+    }
+    a.opos32[J.site_off / 3 + m] = make_float4(w[0], w[1], w[2], 0.f);
+}
+
+template <int FULL>
+__global__ void __launch_bounds__(128) k_lj64(EvalArgs a) {
+    const Job J = a.jobs[blockIdx.y];
+    const SysDev &S = a.sys[J.sys];
+    const int N = S.n_mols;
+    if (blockIdx.x * 4 >= N) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 4 + w;
+    __shared__ int queue[4][64];
+    __shared__ double red[4];
+    double e = 0.0;
+    const Consts &C = a.c;
+    const double rc2 = C.r_cut_sq;
+    if (i < (FULL ? N : N - 1)) {
+        const double *q = a.pos + J.pos_off;
+        const int cap = FULL ? 2 * S.list_size : S.list_size;
+        const int *pt = FULL ? a.point_full + S.pf_off + (size_t)J.bead * (N + 1) : a.point + S.pt_off + (size_t)J.bead * N;
+        const int *ls = FULL ? a.list_full + S.lf_off + (size_t)J.bead * cap : a.list + S.ls_off + (size_t)J.bead * cap;
+        // a row outside [0, capacity] (overflowed or caller-corrupted list) or an index
+        // outside the row's range is skipped and flagged instead of being read out of bounds
+        int n0 = pt[i], n1 = pt[i + 1];
+        if (n0 < 0 || n1 > cap || n0 > n1) {
+            if (lane == 0) atomicOr(a.status, (unsigned)ST_LIST_OVERFLOW);
+            n0 = max(0, min(n0, cap));
+            n1 = max(n0, min(n1, cap));
+        }
+        const float4 *opos = a.opos32 + J.site_off / 3;
+        double *plane = a.lj64 + 4 * ((size_t)J.site_off / 3);
+        const float4 oi = opos[i];
+        const double xi[3] = {q[9 * i], q[9 * i + 1], q[9 * i + 2]};
+        const float L[3] = {S.boxf[0], S.boxf[1], S.boxf[2]}, I[3] = {S.inv_boxf[0], S.inv_boxf[1], S.inv_boxf[2]};
+        const float lim = C.ljf[6] * (1.0f + 1e-6f) + 5e-7f * (L[0] + L[1] + L[2]), lim2 = lim * lim;
+        double f0 = 0.0, f1 = 0.0, f2 = 0.0, el = 0.0;
+        auto pair = [&](int j) {
+            const double *qj = q + 9 * j;
+            double r[3], r2 = 0.0;
+            bool exact = false;
+            for (int d = 0; d < 3; ++d) {
+                const double x = xi[d] - qj[d];
+                const float t = (float)x * I[d], n = rintf(t);
+                exact |= fabsf(fabsf(t - n) - 0.5f) < 1e-3f;
+                r[d] = n == 0.0f ? x : x - (n == 1.0f ? S.box[d] : n == -1.0f ? -S.box[d] : S.box[d] * (double)n);
+                r2 = fma(r[d], r[d], r2);
+            }
+            if (exact || fabs(r2 - rc2) <= 1e-12 * rc2) r2 = lj64_exact(xi, qj, S, r);
+            if (!(r2 < rc2)) return;
+            const double i2 = 1.0 / r2, i6 = i2 * i2 * i2;
+            const double s6 = i6 * C.sigmalj6, s12 = i6 * i6 * C.sigmalj12, en = s12 - s6;
+            el += en * (4.0 * C.epslj) - C.e_cut;
+            const double ff = (en + s12) * (24.0 * C.epslj) * i2;
+            f0 += ff * r[0];
+            f1 += ff * r[1];
+            f2 += ff * r[2];
+            if (!FULL)
+                for (int d = 0; d < 3; ++d) atomicAdd(plane + 4 * j + d, -(ff * r[d]));
+        };
+        int *qu = queue[w];
+        int cnt = 0;
+        for (int base = n0; base < n1; base += 32) {
+            const int n = base + lane;
+            int j = n < n1 ? ls[n] : i;
+            bool hit = false;
+            if (n < n1 && ((FULL ? j == i : j <= i) || j < 0 || j >= N)) {
+                atomicOr(a.status, (unsigned)ST_LIST_OVERFLOW);
+                j = i;
+            }
+            if (j != i) {
+                const float4 o = opos[j];
+                float dx = oi.x - o.x, dy = oi.y - o.y, dz = oi.z - o.z;
+                dx = fmaf(-L[0], rintf(dx * I[0]), dx);
+                dy = fmaf(-L[1], rintf(dy * I[1]), dy);
+                dz = fmaf(-L[2], rintf(dz * I[2]), dz);
+                hit = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < lim2;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            if (hit) qu[cnt + __popc(m & ((1u << lane) - 1u))] = j;
+            cnt += __popc(m);
+            __syncwarp();
+            if (cnt >= 32) {
+                pair(qu[lane]);
+                cnt -= 32;
+                const int rest = lane < cnt ? qu[32 + lane] : 0;
+                __syncwarp();
+                qu[lane] = rest;
+                __syncwarp();
+            }
+        }
+        if (lane < cnt) pair(qu[lane]);
+        __syncwarp();
+        f0 = warp_sum(f0);
+        f1 = warp_sum(f1);
+        f2 = warp_sum(f2);
+        e = warp_sum(el) * (FULL ? 0.5 : 1.0);
+        if (lane == 0) {
+            if (FULL) {
+                plane[4 * i] = f0;
+                plane[4 * i + 1] = f1;
+                plane[4 * i + 2] = f2;
+            } else {
+                atomicAdd(plane + 4 * i, f0);
+                atomicAdd(plane + 4 * i + 1, f1);
+                atomicAdd(plane + 4 * i + 2, f2);
+            }
+        }
+    }
+    if (lane == 0) red[w] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], (red[0] + red[1]) + (red[2] + red[3]));
+}
+
+}  // namespace
+
+void launch_lj64_prep(const EvalArgs &a, cudaStream_t s) {
+    k_lj64_prep<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
+}
+
+void launch_lj64(const EvalArgs &a, cudaStream_t s) {
+    const dim3 g((a.max_mols + 3) / 4, a.n_jobs);
+    if (a.lj_full) k_lj64<1><<<g, 128, 0, s>>>(a);
+    else k_lj64<0><<<g, 128, 0, s>>>(a);
+}
+
+}  // namespace qtg

@@ -18,7 +18,7 @@ struct Consts {
     double r_cut, r_cut_sq, r_skin, r_skin_sq;
     double gamma_vs, epslj, sigmalj6, sigmalj12, e_cut;
     double roheq, ar2, ar3, ar4fac, Dr, theta_eq, ktheta, qo, qh;
-    float ljf[6];  // FP32 Lennard-Jones constants: sigma^6, sigma^12, 4 eps, 24 eps, e_cut, r_cut^2
+    float ljf[7];  // FP32 Lennard-Jones constants: sigma^6, sigma^12, 4 eps, 24 eps, e_cut, r_cut^2, r_cut
 };
 
 // Per-system constants (one per replica), resident in device memory.
@@ -514,7 +514,9 @@ struct EvalArgs {
     void *sites;           // 4 reals per site (x, y, z, q), per slot
     int4 *sites_fix;       // mixed: per site the box fractions of x, y, z as 32-bit fixed point
                            // (so a wrapped integer difference is the minimum image) and q's bits
-    void *opos;            // wrapped oxygen positions, 4 reals per molecule, per slot
+    void *opos;            // mixed: wrapped oxygen positions, 4 floats per molecule, per slot
+    float4 *opos32;        // FP64 evaluations: the same, for k_lj64's screening
+    double *lj64;          // FP64 evaluations: Lennard-Jones oxygen forces, 4 doubles per molecule, per slot
     float4 *ljf;           // dense Lennard-Jones oxygen forces, per molecule, per slot (lj_plane)
     int lj_plane;          // 1: k_lj_dense writes ljf and k_combine_f32 adds it to the O force
     float *intra;          // mixed: intramolecular site and atom forces, 18 floats per molecule and slot
@@ -590,6 +592,10 @@ void launch_ksk2(const EvalArgs &a, cudaStream_t s);
 void real64_table(double *tab);
 void init_real64_attributes();
 void launch_real64(const EvalArgs &a, cudaStream_t s);
+
+// lj64.cu: Lennard-Jones of the FP64 form
+void launch_lj64_prep(const EvalArgs &a, cudaStream_t s);
+void launch_lj64(const EvalArgs &a, cudaStream_t s);
 
 // recip64.cu: site preparation and reciprocal space of the FP64 form
 void init_recip64_attributes();

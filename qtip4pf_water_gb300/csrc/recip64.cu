@@ -72,9 +72,9 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
         // M site (forces.cpp:558-564)
         x = g * q[9 * mol + d] + 0.5 * (1.0 - g) * (q[9 * mol + 3 + d] + q[9 * mol + 6 + d]);
         const double t = q[9 * mol + d] * S.inv_box[d];
-        double *o = reinterpret_cast<double *>(a.opos) + 4 * ((size_t)J.site_off / 3 + mol);
-        o[d] = (t - floor(t)) * S.box[d];
-        if (d == 0) o[3] = 0.0;
+        const size_t at = 4 * ((size_t)J.site_off / 3 + mol) + d;
+        reinterpret_cast<float *>(a.opos32)[at] = (float)((t - floor(t)) * S.box[d]);
+        a.lj64[at] = 0.0;  // k_lj64's forces
     }
     const double t = x * S.inv_box[d], frac = t - floor(t);
     const double chg = d == 0 ? a.charge[S.chg_off + s] : 0.0;
