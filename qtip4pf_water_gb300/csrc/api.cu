@@ -289,7 +289,7 @@ struct qtg_ctx {
     // per-slot scratch
     void *sites = nullptr, *tan_sites = nullptr, *phase = nullptr, *opos = nullptr;
     float4 *opos32 = nullptr;  // FP64 evaluations: wrapped oxygens in FP32, and the Lennard-Jones forces
-    double *lj64 = nullptr;
+    double *lj64 = nullptr, *intra64 = nullptr;
     double *part = nullptr;           // [MAX_PART][total_sites][3]
     double2 *skp = nullptr, *dskp = nullptr;  // [MAX_SC][total_k]
     double2 *wsk = nullptr, *wdsk = nullptr;  // [total_k] (sized for FP64)
@@ -407,6 +407,7 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.opos = c->opos;
     a.opos32 = c->opos32;
     a.lj64 = c->lj64;
+    a.intra64 = c->intra64;
     a.ljf = c->ljf;
     a.intra = c->intra;
     a.phase = c->phase;
@@ -452,7 +453,7 @@ EvalArgs aux_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, do
 // jobs of mode 1, nor to reciprocal-space-only calls).
 void launch_eval(qtg_ctx *c, const EvalArgs &a) {
     if (c->mixed) launch_eval_mixed(a, c->stream, &c->launches, &c->forks);
-    else launch_eval_fp64(a, c->stream, &c->launches);
+    else launch_eval_fp64(a, c->stream, &c->launches, &c->forks);
     if (c->spl_any && a.mode == 0 && !a.sites_are_input) {
         SplineArgs s;
         s.sys = c->sys_d;
@@ -669,10 +670,17 @@ void enqueue_forces(qtg_ctx *c, int sys, bool force_sc) {
         sa.n_jobs = n_odd;
         launch_sc_prepare(sa, c->stream, &c->launches);
         if (c->mixed) {
-            launch_eval(c, aux_args(c, tanj, tn, c->q, c->fdisp, 1, 0));
+            // the finite differences (FP64 pipe) and the derivative (FP32) side by side
             EvalArgs sr = aux_args(c, fdj, fdn, c->qdisp, c->fsr, 0, 1);
             sr.lj_full = full;
+            cudaEventRecord(c->forks.sc_fork, c->stream);
+            cudaStreamWaitEvent(c->forks.sc_stream, c->forks.sc_fork, 0);
+            std::swap(c->stream, c->forks.sc_stream);
             launch_eval(c, sr);
+            std::swap(c->stream, c->forks.sc_stream);
+            cudaEventRecord(c->forks.sc_join, c->forks.sc_stream);
+            launch_eval(c, aux_args(c, tanj, tn, c->q, c->fdisp, 1, 0));
+            cudaStreamWaitEvent(c->stream, c->forks.sc_join, 0);
         } else {
             EvalArgs fd = aux_args(c, fdj, fdn, c->qdisp, c->fdisp, 0, 0);
             fd.lj_full = full;
@@ -1299,6 +1307,9 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&ctx->forks.side[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->forks.fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->forks.sc_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->forks.sc_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->forks.sc_join, cudaEventDisableTiming);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ctx->forks.join[k], cudaEventDisableTiming);
 #define AL(ptr, n)                                  \
     if (e == cudaSuccess) e = dalloc(&(ptr), (n));
@@ -1359,6 +1370,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     }
     AL(ctx->opos32, ctx->total_sites / 3);
     AL(ctx->lj64, 4 * (ctx->total_sites / 3));
+    AL(ctx->intra64, 6 * ctx->total_sites);
     AL(ctx->ljf, ctx->total_sites / 3);
     AL(ctx->intra, 6 * ctx->total_sites);
     AL(ctx->sites_fix, ctx->total_sites);
@@ -1519,7 +1531,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair, ctx->opos32, ctx->lj64};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair, ctx->opos32, ctx->lj64, ctx->intra64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);
@@ -1532,9 +1544,9 @@ void qtg_destroy(qtg_ctx *ctx) {
     if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
     if (ctx->sur_stream) cudaStreamDestroy(ctx->sur_stream);
     for (cudaEvent_t ev : {ctx->ev_fork[0], ctx->ev_fork[1], ctx->ev_join, ctx->forks.fork, ctx->forks.join[0],
-                           ctx->forks.join[1], ctx->sur_fork, ctx->sur_join})
+                           ctx->forks.join[1], ctx->sur_fork, ctx->sur_join, ctx->forks.sc_fork, ctx->forks.sc_join})
         if (ev) cudaEventDestroy(ev);
-    for (cudaStream_t st : {ctx->forks.side[0], ctx->forks.side[1]})
+    for (cudaStream_t st : {ctx->forks.side[0], ctx->forks.side[1], ctx->forks.sc_stream})
         if (st) cudaStreamDestroy(st);
     delete ctx;
 }

@@ -1718,138 +1718,7 @@ void launch_kforce_f32(const EvalArgs &a, dim3 grid, cudaStream_t s) {
 
 // ---- k_combine: partial sums, short-range terms and the M-site chain rule ---------
 
-// Minimum image of an intramolecular vector. |r / L| is far below 1/2, where
-// round(r * (1/L)) and the reference's round(r / L) agree (both 0, or the same
-// integer for a molecule split by wrapping), so no FP64 division is needed.
-__device__ __forceinline__ void min_image3(double *r, const SysDev &S) {
-    for (int d = 0; d < 3; ++d) r[d] -= S.box[d] * round(r[d] * S.inv_box[d]);
-}
-
-// same-molecule real-space pair with erfc - 1 (forces.cpp:141-177); the
-// difference vector is formed in FP64, the pair term in R
-template <typename R>
-__device__ __forceinline__ double ewald_same_mol(const double *ri, const double *rj, double qiqj, const SysDev &S,
-                                                 double *fi, double *fj) {
-    double rd[3];
-    for (int d = 0; d < 3; ++d) rd[d] = ri[d] - rj[d];
-    min_image3(rd, S);
-    const double r2d = rd[0] * rd[0] + rd[1] * rd[1] + rd[2] * rd[2];
-    if (!(r2d < S.rc_sq)) return 0.0;
-    const R r2 = (R)r2d, rl = f_sqrt(r2), inv = (R)1 / rl, kap = (R)S.kappa;
-    const R ec = f_erfc(kap * rl) - (R)1;
-    const R e = (R)qiqj * inv * ec;
-    const R ff = (e + (R)qiqj * (R)S.ewald_pref * f_exp(-(kap * kap) * r2)) * inv * inv;
-    for (int d = 0; d < 3; ++d) {
-        fi[d] += (double)(ff * (R)rd[d]);
-        fj[d] -= (double)(ff * (R)rd[d]);
-    }
-    return (double)e;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(128) k_combine(EvalArgs a) {
-    const int jb = blockIdx.y;
-    const Job J = a.jobs[jb];
-    const SysDev &S = a.sys[J.sys];
-    const int N = S.n_mols;
-    if (blockIdx.x * blockDim.x >= N) return;
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    __shared__ double red[4];
-    double e = 0.0;
-    if (m < N) {
-        const double *q = a.pos + J.pos_off + 9 * m;
-        double *f = a.out + J.out_off + 9 * m;
-        double fs[9];
-        for (int k = 0; k < 9; ++k) fs[k] = 0.0;
-        if (!a.sr_only) {
-            const int np = a.n_rj + a.n_kc;
-            for (int p = 0; p < np; ++p) {
-                const double *sf = a.part + 3 * ((size_t)p * a.total_sites + J.site_off + 3 * m);
-                for (int k = 0; k < 9; ++k) fs[k] += sf[k];
-            }
-            if (a.real_fix) {  // k_real64's two-limb sums
-                const long long *rf = a.rfix + 6 * ((size_t)J.site_off + 3 * m);
-                for (int k = 0; k < 9; ++k)
-                    fs[k] += fma((double)rf[2 * k], 0.00390625, (double)rf[2 * k + 1] * 8.673617379884035e-19);
-            }
-        }
-        double fa[9];
-        for (int k = 0; k < 9; ++k) fa[k] = 0.0;
-        if (J.mode == 0) {
-            const Consts &C = a.c;
-            const double g = C.gamma_vs;
-            const double *chg = a.charge + S.chg_off + 3 * m;
-            double site[9];
-            for (int d = 0; d < 3; ++d) {
-                site[d] = g * q[d] + 0.5 * (1.0 - g) * (q[3 + d] + q[6 + d]);
-                site[3 + d] = q[3 + d];
-                site[6 + d] = q[6 + d];
-            }
-            e += ewald_same_mol<R>(site, site + 3, chg[0] * chg[1], S, fs, fs + 3);
-            e += ewald_same_mol<R>(site, site + 6, chg[0] * chg[2], S, fs, fs + 6);
-            e += ewald_same_mol<R>(site + 3, site + 6, chg[1] * chg[2], S, fs + 3, fs + 6);
-            // quartic Morse bonds (forces.cpp:65-93, :519-551); FP64 bond vectors
-            double rad[3], rbd[3];
-            for (int d = 0; d < 3; ++d) {
-                rad[d] = q[d] - q[3 + d];
-                rbd[d] = q[d] - q[6 + d];
-            }
-            min_image3(rad, S);
-            min_image3(rbd, S);
-            R ra[3], rb[3];
-            for (int d = 0; d < 3; ++d) {
-                ra[d] = (R)rad[d];
-                rb[d] = (R)rbd[d];
-            }
-            const double lad = sqrt(rad[0] * rad[0] + rad[1] * rad[1] + rad[2] * rad[2]);
-            const double lbd = sqrt(rbd[0] * rbd[0] + rbd[1] * rbd[1] + rbd[2] * rbd[2]);
-            const R la = (R)lad, lb = (R)lbd;
-            const R ar2 = (R)C.ar2, ar3 = (R)C.ar3, ar4 = (R)C.ar4fac, Dr = (R)C.Dr;
-            for (int bnd = 0; bnd < 2; ++bnd) {
-                const R *r = bnd ? rb : ra;
-                const R rl = bnd ? lb : la;
-                const R x = (R)((bnd ? lbd : lad) - C.roheq), x2 = x * x, x3 = x2 * x, x4 = x2 * x2;
-                e += (double)(Dr * (ar2 * x2 - ar3 * x3 + ar4 * x4));
-                const R gg = ((R)2 * ar2 * x - (R)3 * ar3 * x2 + (R)4 * ar4 * x3) * Dr / rl;
-                for (int d = 0; d < 3; ++d) {
-                    fa[d] -= (double)(gg * r[d]);
-                    fa[3 + 3 * bnd + d] += (double)(gg * r[d]);
-                }
-            }
-            // harmonic HOH angle (forces.cpp:96-138)
-            {
-                const R dot = ra[0] * rb[0] + ra[1] * rb[1] + ra[2] * rb[2];
-                const R ia = (R)1 / la, ib = (R)1 / lb, iab = ia * ib;
-                const R c = dot * iab;
-                const R dacos = (R)1 / f_sqrt((R)1 - c * c);
-                const R ca = dot * ia * ia * iab, cb = dot * ib * ib * iab;
-                const R dth = f_acos(c) - (R)C.theta_eq;
-                e += 0.5 * C.ktheta * (double)dth * (double)dth;
-                const R gp = (R)C.ktheta * dth * dacos;
-                for (int d = 0; d < 3; ++d) {
-                    fa[d] += (double)(gp * (iab * (ra[d] + rb[d]) - ca * ra[d] - cb * rb[d]));
-                    fa[3 + d] -= (double)(gp * (iab * rb[d] - ca * ra[d]));
-                    fa[6 + d] -= (double)(gp * (iab * ra[d] - cb * rb[d]));
-                }
-            }
-        }
-        // M-site chain rule (forces.cpp:613-619)
-        const double g = a.c.gamma_vs, h = 0.5 * (1.0 - g);
-        const double *lj = a.lj64 + 4 * ((size_t)J.site_off / 3 + m);
-        for (int d = 0; d < 3; ++d) {
-            f[d] = (fa[d] + g * fs[d]) + lj[d];
-            f[3 + d] = fa[3 + d] + fs[3 + d] + h * fs[d];
-            f[6 + d] = fa[6 + d] + fs[6 + d] + h * fs[d];
-        }
-    }
-    if (J.mode == 0) {
-        if (m == 0 && !a.sr_only) e -= S.self_energy;
-        const double t = block_sum(e, red);
-        if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
-    }
-}
-
-// Mixed form of k_combine: the FP32 planes are added with Kahan compensation;
+// The FP32 planes are added with Kahan compensation;
 // the atom differences are formed in FP64 and rounded to FP32 (intramolecular
 // vectors are ~1-3 bohr, so FP32 keeps them to ~1e-7 relative); the bond
 // lengths, whose offsets from r_eq set the stiff Morse force, are taken to FP64
@@ -2080,17 +1949,6 @@ __global__ void __launch_bounds__(128) k_combine_f32(EvalArgs a) {
 // relative band around r_cut^2, or whose separation is within rounding of
 // half a box in some dimension (where the two images tie and the rounding rule
 // picks the sign), is recomputed with exactly that arithmetic.
-__device__ __forceinline__ double lj_exact_disp(const double *qi, const double *qj, const SysDev &S, double *r) {
-    double r2 = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        double x = __dsub_rn(qi[d], qj[d]);
-        x = __dsub_rn(x, __dmul_rn(S.box[d], round(__ddiv_rn(x, S.box[d]))));
-        r[d] = x;
-        r2 = (d == 0) ? __dmul_rn(x, x) : __dadd_rn(r2, __dmul_rn(x, x));
-    }
-    return r2;
-}
-
 template <typename R, int FULL>
 __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     const int jb = blockIdx.y;
@@ -2705,10 +2563,21 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         } else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
         launch_recip(a, s);
     } else {
+        // the derivative: real space beside the reciprocal chain
+        cudaStream_t rs = s;
+        if (forks) {
+            rs = forks->side[0];
+            cudaEventRecord(forks->fork, s);
+            cudaStreamWaitEvent(rs, forks->fork, 0);
+        }
+        launch_ksk<R, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
+        launch_sk_reduce<R, 1>(a, rs);
+        k_kforce<R, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<R>(a.max_kmax), rs>>>(a);
         k_real<R, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        launch_ksk<R, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
-        launch_sk_reduce<R, 1>(a, s);
-        k_kforce<R, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<R>(a.max_kmax), s>>>(a);
+        if (forks) {
+            cudaEventRecord(forks->join[0], rs);
+            cudaStreamWaitEvent(s, forks->join[0], 0);
+        }
     }
     // mixed with the dense Lennard-Jones: its oxygen forces go to their plane first,
     // so the combine writes the complete force
@@ -2726,13 +2595,6 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     }
 }
 
-// A warp a block: the molecules' chains of FP64 library functions are long, and a small
-// batch's warps are spread over the SMs (512 waters, 16 configurations: 28.6 us with four
-// warps a block).
-void launch_combine64(const EvalArgs &a, cudaStream_t s) {
-    k_combine<double><<<dim3((a.max_mols + 31) / 32, a.n_jobs), 32, 0, s>>>(a);
-}
-
 // Chunk counts of the FP64 reciprocal space: whole 32-site shared-memory chunks of the
 // structure factors, and blocks enough to fill the GPU.
 void set_chunks64(EvalArgs &a) {
@@ -2741,18 +2603,37 @@ void set_chunks64(EvalArgs &a) {
     a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
 }
 
-void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n) {
+// An FP64 evaluation: real space | reciprocal chain | short-range terms on parallel
+// streams after the preparation. The first two share the FP64 and integer pipes little, and
+// in a small batch each leaves most of the GPU idle (64 waters, 1 bead: some 31, 48 and
+// 44 us).
+void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks *forks) {
     set_chunks64(a);
     a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
     a.real_fix = 1;
     launch_prep64(a, s);
+    cudaStream_t rs = s, ls = s;
+    if (forks) {
+        rs = forks->side[0];
+        ls = forks->side[1];
+        cudaEventRecord(forks->fork, s);
+        cudaStreamWaitEvent(rs, forks->fork, 0);
+        cudaStreamWaitEvent(ls, forks->fork, 0);
+    }
+    launch_ksk64(a, rs);
+    launch_sk_reduce64(a, rs);
+    launch_kforce64(a, rs);
+    launch_intra64(a, ls);
+    launch_lj64(a, ls);
     launch_real64(a, s);
-    launch_ksk64(a, s);
-    launch_sk_reduce64(a, s);
-    launch_kforce64(a, s);
-    launch_lj64(a, s);
+    if (forks) {
+        cudaEventRecord(forks->join[0], rs);
+        cudaEventRecord(forks->join[1], ls);
+        cudaStreamWaitEvent(s, forks->join[0], 0);
+        cudaStreamWaitEvent(s, forks->join[1], 0);
+    }
     launch_combine64(a, s);
-    if (n) *n += 7;
+    if (n) *n += 8;
 }
 
 }  // namespace
@@ -2823,23 +2704,24 @@ void init_force_kernel_attributes() {
     init_real64_attributes();
 }
 
-void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *n) {
+void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *n, const Forks *forks) {
     if (a.n_jobs <= 0) return;
     if (!a.sr_only) {
-        launch_ewald64(a, s, n);
+        launch_ewald64(a, s, n, forks);
         return;
     }
     // short-range terms only (FP64)
     launch_lj64_prep(a, s);
     launch_lj64(a, s);
+    launch_intra64(a, s);
     launch_combine64(a, s);
-    if (n) *n += 3;
+    if (n) *n += 4;
 }
 
 void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *n, const Forks *forks) {
     if (a.n_jobs <= 0) return;
     if (a.sr_only) {
-        launch_eval_fp64(a, s, n);  // the finite-difference short-range terms stay FP64
+        launch_eval_fp64(a, s, n, nullptr);  // the finite-difference short-range terms stay FP64
         return;
     }
     launch_ewald<float>(a, s, n, forks);

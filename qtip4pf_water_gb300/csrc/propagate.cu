@@ -722,13 +722,14 @@ __global__ void k_finalize(FinalizeArgs a) {
 }
 
 // ---- Suzuki-Chin assembly (forces.cpp:724-775) -----------------------------------
-__global__ void __launch_bounds__(256) k_sc_prepare(ScArgs a) {
+// A block per odd bead (few of them: as many threads a block as there can be).
+__global__ void __launch_bounds__(1024) k_sc_prepare(ScArgs a) {
     const int sid = a.job_sys[blockIdx.x], b = a.job_bead[blockIdx.x];
     const SysDev &S = a.sys[sid];
     const int nd = S.n_dof, P = S.n_beads;
     const double *fp = a.fphys + S.q_off + (size_t)b * nd;
     const double *im = a.inv_mass + S.mass_off;
-    __shared__ double red[8];
+    __shared__ double red[32];
     __shared__ double scl_sh;
     double fsq = 0.0, dl = 0.0;
     for (int i = threadIdx.x; i < nd; i += blockDim.x) {
@@ -881,7 +882,7 @@ void launch_finalize(const FinalizeArgs &a, cudaStream_t s, unsigned long long *
 
 void launch_sc_prepare(const ScArgs &a, cudaStream_t s, unsigned long long *n) {
     if (a.n_jobs <= 0) return;
-    k_sc_prepare<<<a.n_jobs, 256, 0, s>>>(a);
+    k_sc_prepare<<<a.n_jobs, 1024, 0, s>>>(a);
     if (n) ++*n;
 }
 

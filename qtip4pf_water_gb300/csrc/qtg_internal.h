@@ -333,6 +333,26 @@ __device__ __forceinline__ double2 normal2(const Philox4 &r) {
 // RNG stream tags (third counter word's high byte) keep draws independent.
 enum RngTag : uint32_t { RNG_MODES = 1u, RNG_CENTROID = 2u, RNG_GAMMA = 3u };
 
+// The reference's displacement of an O-O pair (forces.cpp:489-515): x - L round(x / L) with a
+// true division, each operation rounded separately. Returns r^2.
+__device__ __forceinline__ double lj_exact_disp(const double *qi, const double *qj, const SysDev &S, double *r) {
+    double r2 = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        double x = __dsub_rn(qi[d], qj[d]);
+        x = __dsub_rn(x, __dmul_rn(S.box[d], round(__ddiv_rn(x, S.box[d]))));
+        r[d] = x;
+        r2 = (d == 0) ? __dmul_rn(x, x) : __dadd_rn(r2, __dmul_rn(x, x));
+    }
+    return r2;
+}
+
+// Minimum image of an intramolecular vector. |r / L| is far below 1/2, where
+// round(r * (1/L)) and the reference's round(r / L) agree (both 0, or the same
+// integer for a molecule split by wrapping), so no FP64 division is needed.
+__device__ __forceinline__ void min_image3(double *r, const SysDev &S) {
+    for (int d = 0; d < 3; ++d) r[d] -= S.box[d] * round(r[d] * S.inv_box[d]);
+}
+
 #endif  // __CUDACC__
 
 // ---- launch interface between translation units ----------------------------
@@ -517,6 +537,7 @@ struct EvalArgs {
     void *opos;            // mixed: wrapped oxygen positions, 4 floats per molecule, per slot
     float4 *opos32;        // FP64 evaluations: the same, for k_lj64's screening
     double *lj64;          // FP64 evaluations: Lennard-Jones oxygen forces, 4 doubles per molecule, per slot
+    double *intra64;       // FP64 evaluations: intramolecular site and atom forces, 18 doubles per molecule, per slot
     float4 *ljf;           // dense Lennard-Jones oxygen forces, per molecule, per slot (lj_plane)
     int lj_plane;          // 1: k_lj_dense writes ljf and k_combine_f32 adds it to the O force
     float *intra;          // mixed: intramolecular site and atom forces, 18 floats per molecule and slot
@@ -529,7 +550,7 @@ struct EvalArgs {
     // integer atomics, so the sum does not depend on their order), read by
     // k_combine_f32 when real_fix is set
     // FP64: the same of k_real64, [total_sites][3][2]: a high limb in units of 2^-8 and a
-    // low limb in units of 2^-60 (zeroed by k_prep, read by k_combine)
+    // low limb in units of 2^-60 (zeroed by k_prep64, read by k_combine64)
     long long *rfix;
     int real_fix;
     const double *real64_tab;  // FP64: the pair-function table (real64_table)
@@ -593,9 +614,11 @@ void real64_table(double *tab);
 void init_real64_attributes();
 void launch_real64(const EvalArgs &a, cudaStream_t s);
 
-// lj64.cu: Lennard-Jones of the FP64 form
+// short64.cu: short-range terms of the FP64 form and the sum of its forces
 void launch_lj64_prep(const EvalArgs &a, cudaStream_t s);
 void launch_lj64(const EvalArgs &a, cudaStream_t s);
+void launch_intra64(const EvalArgs &a, cudaStream_t s);
+void launch_combine64(const EvalArgs &a, cudaStream_t s);
 
 // recip64.cu: site preparation and reciprocal space of the FP64 form
 void init_recip64_attributes();
@@ -637,7 +660,8 @@ void launch_fp32_probe(float *out, int blocks, int iters, cudaStream_t s);
 void launch_fp64_probe(double *out, int blocks, int iters, cudaStream_t s);
 
 // forces.cu
-void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *launches);
+struct Forks;
+void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *launches, const Forks *forks);
 // Side streams and events for a forked mixed evaluation: after k_prep, the
 // reciprocal-space chain (k_ksk, k_sk_reduce, k_kforce_f32) runs on side[0] and
 // the dense Lennard-Jones on side[1] beside the real-space kernel; both join
@@ -645,6 +669,10 @@ void launch_eval_fp64(const EvalArgs &a, cudaStream_t s, unsigned long long *lau
 struct Forks {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
+    // the short-range finite differences of the mixed Suzuki-Chin force run on sc_stream
+    // beside the Ewald derivative
+    cudaStream_t sc_stream;
+    cudaEvent_t sc_fork, sc_join;
     cudaEvent_t lists_ready;  // set: the Verlet-list rebuild runs beside the forces; the list LJ waits for it
 };
 void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *launches,

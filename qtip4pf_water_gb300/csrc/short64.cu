@@ -1,6 +1,8 @@
-// O-O Lennard-Jones of the FP64 form over the Verlet list (forces.cpp:25-59, :489-515).
+// Short-range terms of the FP64 form: O-O Lennard-Jones over the Verlet list
+// (forces.cpp:25-59, :489-515), the intramolecular terms, and the sum of a molecule's
+// forces.
 //
-// One warp per list row. What bounds it is FP64 issue (a warp's FP64 instruction takes
+// Lennard-Jones: one warp per list row. What bounds it is FP64 issue (a warp's FP64 instruction takes
 // sixteen cycles of an SM), and of the list's pairs, which reach to r_skin = 1.3 r_cut,
 // only 45 % lie inside r_cut. So the entries are screened in FP32 on wrapped positions,
 // with a margin above their rounding, and the pairs that pass are packed into full warps
@@ -14,7 +16,7 @@
 //
 // FULL: the stepper's symmetric list; a row's force needs no atomics and the energy is
 // halved. Else the caller's half list (entries j > i), forces added by atomics. The oxygen
-// forces go to their own array, which k_combine adds, so that the kernel can run beside
+// forces go to their own array, which k_combine64 adds, so that the kernel can run beside
 // the Ewald kernels.
 #include <math.h>
 
@@ -23,17 +25,6 @@
 namespace qtg {
 
 namespace {
-
-__device__ double lj64_exact(const double *qi, const double *qj, const SysDev &S, double *r) {
-    double r2 = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        double x = __dsub_rn(qi[d], qj[d]);
-        x = __dsub_rn(x, __dmul_rn(S.box[d], round(__ddiv_rn(x, S.box[d]))));
-        r[d] = x;
-        r2 = (d == 0) ? __dmul_rn(x, x) : __dadd_rn(r2, __dmul_rn(x, x));
-    }
-    return r2;
-}
 
 // Wrapped FP32 oxygens and cleared forces, where no preparation pass made them (the
 // displaced configurations of the Suzuki-Chin force gradient).
@@ -94,7 +85,7 @@ __global__ void __launch_bounds__(128) k_lj64(EvalArgs a) {
                 r[d] = n == 0.0f ? x : x - (n == 1.0f ? S.box[d] : n == -1.0f ? -S.box[d] : S.box[d] * (double)n);
                 r2 = fma(r[d], r[d], r2);
             }
-            if (exact || fabs(r2 - rc2) <= 1e-12 * rc2) r2 = lj64_exact(xi, qj, S, r);
+            if (exact || fabs(r2 - rc2) <= 1e-12 * rc2) r2 = lj_exact_disp(xi, qj, S, r);
             if (!(r2 < rc2)) return;
             const double i2 = 1.0 / r2, i6 = i2 * i2 * i2;
             const double s6 = i6 * C.sigmalj6, s12 = i6 * i6 * C.sigmalj12, en = s12 - s6;
@@ -160,7 +151,123 @@ __global__ void __launch_bounds__(128) k_lj64(EvalArgs a) {
     if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], (red[0] + red[1]) + (red[2] + red[3]));
 }
 
+// ---- k_intra64: intramolecular terms (forces.cpp:65-138, :141-177, :519-554) ----------
+// Four threads a molecule, as what bounds it is the length of the chains of FP64 library
+// functions: the three same-molecule Ewald pairs (erfc - 1) a thread each, the quartic
+// Morse bonds and the HOH angle the fourth (one thread for all of it took 30 us whatever
+// the batch). Per molecule 18 doubles, site forces (M, H1, H2) and atom forces (O, H1,
+// H2), for k_combine64; the energy with the Ewald self term into the job's slot.
+
+__global__ void __launch_bounds__(128) k_intra64(EvalArgs a) {
+    const Job J = a.jobs[blockIdx.y];
+    const SysDev &S = a.sys[J.sys];
+    const int N = S.n_mols;
+    if ((int)(blockIdx.x * blockDim.x) >= 4 * N) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t & 3, m = min(t >> 2, N - 1);
+    const bool act = (t >> 2) < N;
+    __shared__ double red[4];
+    const double *q = a.pos + J.pos_off + 9 * m;
+    double *o = a.intra64 + 18 * ((size_t)J.site_off / 3 + m);
+    const Consts &C = a.c;
+    double e = 0.0, f[3] = {0.0, 0.0, 0.0};  // k < 3: the pair's force on its first site
+    if (k < 3) {
+        const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+        const double g = C.gamma_vs;
+        double r[3];
+        for (int d = 0; d < 3; ++d) {
+            const double si = i ? q[3 * i + d] : g * q[d] + 0.5 * (1.0 - g) * (q[3 + d] + q[6 + d]);
+            r[d] = si - q[3 * j + d];
+        }
+        min_image3(r, S);
+        const double *chg = a.charge + S.chg_off + 3 * m;
+        const double qq = chg[i] * chg[j], r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        if (r2 < S.rc_sq) {
+            const double rl = sqrt(r2), inv = 1.0 / rl, kap = S.kappa;
+            e = qq * inv * (erfc(kap * rl) - 1.0);
+            const double ff = (e + qq * S.ewald_pref * exp(-(kap * kap) * r2)) * inv * inv;
+            for (int d = 0; d < 3; ++d) f[d] = ff * r[d];
+        }
+    } else {
+        double fa[9];
+        for (int d = 0; d < 9; ++d) fa[d] = 0.0;
+        // quartic Morse bonds (forces.cpp:65-93, :519-551)
+        double r[2][3], l[2];
+        for (int b = 0; b < 2; ++b) {
+            for (int d = 0; d < 3; ++d) r[b][d] = q[d] - q[3 + 3 * b + d];
+            min_image3(r[b], S);
+            l[b] = sqrt(r[b][0] * r[b][0] + r[b][1] * r[b][1] + r[b][2] * r[b][2]);
+            const double x = l[b] - C.roheq, x2 = x * x, x3 = x2 * x, x4 = x2 * x2;
+            e += C.Dr * (C.ar2 * x2 - C.ar3 * x3 + C.ar4fac * x4);
+            const double gg = (2.0 * C.ar2 * x - 3.0 * C.ar3 * x2 + 4.0 * C.ar4fac * x3) * C.Dr / l[b];
+            for (int d = 0; d < 3; ++d) {
+                fa[d] -= gg * r[b][d];
+                fa[3 + 3 * b + d] += gg * r[b][d];
+            }
+        }
+        // harmonic HOH angle (forces.cpp:96-138)
+        const double dot = r[0][0] * r[1][0] + r[0][1] * r[1][1] + r[0][2] * r[1][2];
+        const double ia = 1.0 / l[0], ib = 1.0 / l[1], iab = ia * ib, c = dot * iab;
+        const double dacos = 1.0 / sqrt(1.0 - c * c), ca = dot * ia * ia * iab, cb = dot * ib * ib * iab;
+        const double dth = acos(c) - C.theta_eq;
+        e += 0.5 * C.ktheta * dth * dth;
+        const double gp = C.ktheta * dth * dacos;
+        for (int d = 0; d < 3; ++d) {
+            fa[d] += gp * (iab * (r[0][d] + r[1][d]) - ca * r[0][d] - cb * r[1][d]);
+            fa[3 + d] -= gp * (iab * r[1][d] - ca * r[0][d]);
+            fa[6 + d] -= gp * (iab * r[0][d] - cb * r[1][d]);
+        }
+        if (act)
+            for (int d = 0; d < 9; ++d) o[9 + d] = fa[d];
+        if (m == 0 && !a.sr_only) e -= S.self_energy;
+    }
+    // site k takes its two pairs' forces: M +(0) +(1), H1 -(0) +(2), H2 -(1) -(2)
+    for (int d = 0; d < 3; ++d) {
+        const int base = threadIdx.x & 28;
+        const double p = __shfl_sync(0xffffffffu, f[d], base + (k == 2 ? 1 : 0));
+        const double s = __shfl_sync(0xffffffffu, f[d], base + (k == 0 ? 1 : 2));
+        if (act && k < 3) o[3 * k + d] = (k == 0 ? p : -p) + (k == 2 ? -s : s);
+    }
+    const double te = block_sum(act ? e : 0.0, red);
+    if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], te);
+}
+
+// ---- k_combine64 ------------------------------------------------------------------------
+// Three threads a molecule (one a dimension): the k-force planes in order, k_real64's
+// two-limb sums, the intramolecular and Lennard-Jones forces, and the M-site chain rule
+// (forces.cpp:613-619).
+__global__ void __launch_bounds__(96) k_combine64(EvalArgs a) {
+    const Job J = a.jobs[blockIdx.y];
+    const SysDev &S = a.sys[J.sys];
+    const int t = blockIdx.x * 96 + threadIdx.x, m = t / 3, d = t - 3 * m;
+    if (m >= S.n_mols) return;
+    double fs[3] = {0.0, 0.0, 0.0};
+    if (!a.sr_only) {
+        const size_t at = 3 * ((size_t)J.site_off + 3 * m) + d;
+        for (int p = 0; p < a.n_kc; ++p)
+            for (int s = 0; s < 3; ++s) fs[s] += a.part[3 * (size_t)p * a.total_sites + at + 3 * s];
+        for (int s = 0; s < 3; ++s) {
+            const long long *rf = a.rfix + 2 * (at + 3 * s);
+            fs[s] += fma((double)rf[0], 0.00390625, (double)rf[1] * 8.673617379884035e-19);
+        }
+    }
+    const size_t mol = (size_t)J.site_off / 3 + m;
+    const double *in = a.intra64 + 18 * mol + d;
+    for (int s = 0; s < 3; ++s) fs[s] += in[3 * s];
+    const double g = a.c.gamma_vs, h = 0.5 * (1.0 - g);
+    double *f = a.out + J.out_off + 9 * m + d;
+    f[0] = (in[9] + g * fs[0]) + a.lj64[4 * mol + d];
+    f[3] = in[12] + fs[1] + h * fs[0];
+    f[6] = in[15] + fs[2] + h * fs[0];
+}
+
 }  // namespace
+
+void launch_intra64(const EvalArgs &a, cudaStream_t s) {
+    k_intra64<<<dim3((a.max_mols + 31) / 32, a.n_jobs), 128, 0, s>>>(a);
+}
+void launch_combine64(const EvalArgs &a, cudaStream_t s) {
+    k_combine64<<<dim3((a.max_mols + 31) / 32, a.n_jobs), 96, 0, s>>>(a);
+}
 
 void launch_lj64_prep(const EvalArgs &a, cudaStream_t s) {
     k_lj64_prep<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, s>>>(a);
