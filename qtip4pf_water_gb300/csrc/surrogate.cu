@@ -558,10 +558,6 @@ struct TrainArgs {
 __device__ __forceinline__ void st_bf16(uint8_t *tile, uint32_t off, float v) {
     *reinterpret_cast<__nv_bfloat16 *>(tile + off) = __float2bfloat16_rn(v);
 }
-__device__ __forceinline__ float dsilu(float z) {
-    const float s = 1.0f / (1.0f + __expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
 // copy the transposed (k, n) view of a row-major [rows][cols] BF16 matrix into a
 // K-major B tile: element (n, k) = src[k][n]
 __device__ __forceinline__ void load_tile_t(uint8_t *tile, const __nv_bfloat16 *src, int rows, int cols, int K) {
@@ -571,7 +567,39 @@ __device__ __forceinline__ void load_tile_t(uint8_t *tile, const __nv_bfloat16 *
     }
 }
 
-__global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
+// This lane's row r of 16 columns from c0 on, of a tile that both a layer's GEMM and a
+// weight gradient read: BF16 values into the transposed tile, two rows a store (a lane and
+// its neighbour exchange halves: the even lane stores the even column of both rows, the
+// odd lane the odd one), and, where `rows` is given, 16 bytes a store into the tile itself.
+__device__ __forceinline__ void store_pairs_t(uint8_t *cols, int c, int r, uint32_t w) {
+    const bool odd = r & 1;
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? w & 0xffffu : w >> 16, 1);
+    *reinterpret_cast<uint32_t *>(cols + kmaj_off(c + (odd ? 1 : 0), r & ~1, TM)) =
+        odd ? got | (w & 0xffff0000u) : (w & 0xffffu) | got << 16;
+}
+__device__ __forceinline__ void store16(uint8_t *rows, int K, uint8_t *cols, int c0, int r, const float *v) {
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
+        store_pairs_t(cols, c0 + 2 * k, r, w[k]);
+    }
+    if (rows) {
+        *reinterpret_cast<uint4 *>(rows + kmaj_off(r, c0, K)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4 *>(rows + kmaj_off(r, c0 + 8, K)) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// One CTA an SM (its weight gradients stay in TMEM over all its tiles). The products are
+// small (a tile's take some hundred cycles); what bounds the kernel is the elementwise work
+// between them and the waits, so sixteen warps share a tile: warp w has the 32 rows of
+// TMEM quadrant w mod 4 and the 16 columns from 16 (w / 4) on of every layer. SiLU's
+// derivative is kept in registers from the forward pass, the transposed copies are stored
+// two rows at a time, and the next tile's inputs are loaded while this one is worked on.
+// 442368 rows: 800 us with four warps, one row a thread and two-byte stores; see
+// qtg_mlp_train_batch's launch.
+constexpr int TT = 512;
+__global__ void __launch_bounds__(TT, 1) k_mlp_train(TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float *b1 = reinterpret_cast<float *>(sm + T_B), *b2 = b1 + DH, *b3 = b2 + DH;
@@ -579,28 +607,31 @@ __global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + T_MISC + 8);
     float *red = reinterpret_cast<float *>(sm + T_MISC + 16);  // 4 warp sums
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cg = warp >> 2, c0 = 16 * cg, r = (warp & 3) * 32 + lane;  // my columns and tile row
     load_tile(sm + T_W1, a.w1, DH, DIN, 0, DH);
     load_tile(sm + T_W2, a.w2, DH, DH, 0, DH);
     load_tile(sm + T_W3, a.w3, DOUT, DH, 0, DOUT);
     // dH2 = dZ3 W3: B element (i, o) = W3[o][i] (K = 16 outputs); dH1 = dZ2 W2: B element (i, o) = W2[o][i]
     load_tile_t(sm + T_W3T, a.w3, DOUT, DH, DOUT);
     load_tile_t(sm + T_W2T, a.w2, DH, DH, DH);
-    for (int k = tid; k < DH; k += TM) {
-        b1[k] = a.b1[k];
-        b2[k] = a.b2[k];
+    if (tid < DH) {
+        b1[tid] = a.b1[tid];
+        b2[tid] = a.b2[tid];
     }
     if (tid < DOUT) b3[tid] = a.b3[tid];
     // rows of ones after the features of the A^T tiles (bias gradients)
-    st_bf16(sm + T_XT, kmaj_off(DIN, tid, TM), 1.0f);
-    st_bf16(sm + T_H1T, kmaj_off(DH, tid, TM), 1.0f);
-    st_bf16(sm + T_H2T, kmaj_off(DH, tid, TM), 1.0f);
+    if (tid < TM) {
+        st_bf16(sm + T_XT, kmaj_off(DIN, tid, TM), 1.0f);
+        st_bf16(sm + T_H1T, kmaj_off(DH, tid, TM), 1.0f);
+        st_bf16(sm + T_H2T, kmaj_off(DH, tid, TM), 1.0f);
+    }
     if (tid == 0) mbar_init(smem_u32(mbar), 1);
     if (warp == 0) tmem_alloc(smem_u32(tslot), TRAIN_COLS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tslot, lrow = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t tmem = *tslot, lrow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t phase = 0;
     bool ok = true;
     float loss = 0.f;
@@ -621,63 +652,72 @@ __global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
         ok = __syncthreads_and(w);
         tc_fence_after();
     };
+    // my chunks (8 inputs) of row r of a tile: cg, cg + 4, cg + 8
+    uint4 xv[3];
+    auto load_x = [&](int t) {
+        const bool in = t < n_tiles && t * TM + r < a.m;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            xv[k] = in ? *reinterpret_cast<const uint4 *>(a.x + (size_t)(t * TM + r) * DIN + (cg + 4 * k) * 8) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    load_x(blockIdx.x);
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++my_tiles) {
-        const int m0 = t * TM, r = tid;
+        const int m0 = t * TM;
         const bool valid = m0 + r < a.m;
         const uint32_t gacc = my_tiles > 0 ? 1u : 0u;
         // inputs: K-major X and transposed X^T
-        load_tile(sm + T_X, a.x, TM, DIN, m0, a.m);
-        for (int kg = 0; kg < DIN / 8; ++kg) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (valid) v = *reinterpret_cast<const uint4 *>(a.x + (size_t)(m0 + r) * DIN + kg * 8);
-            const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&v);
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                *reinterpret_cast<__nv_bfloat16 *>(sm + T_XT + kmaj_off(kg * 8 + e, r, TM)) = h[e];
+        for (int k = 0; k < 3; ++k) {
+            const int c = (cg + 4 * k) * 8;
+            *reinterpret_cast<uint4 *>(sm + T_X + kmaj_off(r, c, DIN)) = xv[k];
+            store_pairs_t(sm + T_XT, c, r, xv[k].x);
+            store_pairs_t(sm + T_XT, c + 2, r, xv[k].y);
+            store_pairs_t(sm + T_XT, c + 4, r, xv[k].z);
+            store_pairs_t(sm + T_XT, c + 6, r, xv[k].w);
         }
+        load_x(t + gridDim.x);
+        float tv[QTG_MLP_OUT];
+        if (cg == 0) {
+#pragma unroll
+            for (int o = 0; o < QTG_MLP_OUT; ++o) tv[o] = valid ? a.t[(size_t)(m0 + r) * DOUT + o] : 0.f;
+        }
+        float z[16], d1[16], d2[16];
+        // SiLU of my 16 pre-activations, in place, and its derivative
+        auto activate = [&](const float *bias, float *d) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float u = z[e] + bias[c0 + e], s = 1.0f / (1.0f + __expf(-u));
+                z[e] = u * s;
+                d[e] = s * (1.0f + u * (1.0f - s));
+            }
+        };
         // layer 1
         stage([&] { gemm(tmem + C_Z1, sm + T_X, sm + T_W1, DIN, IDESC_H); });
         if (!ok) break;
-        for (int c = 0; c < DH; c += 16) {
-            float z[16];
-            tmem_ld16(lrow + C_Z1 + c, z);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float h = silu(z[e] + b1[c + e]);
-                st_bf16(sm + T_H1, kmaj_off(r, c + e, DH), h);
-                st_bf16(sm + T_H1T, kmaj_off(c + e, r, TM), h);
-            }
-        }
+        tmem_ld16(lrow + C_Z1 + c0, z);
+        activate(b1, d1);
+        store16(sm + T_H1, DH, sm + T_H1T, c0, r, z);
         // layer 2
         stage([&] { gemm(tmem + C_Z2, sm + T_H1, sm + T_W2, DH, IDESC_H); });
         if (!ok) break;
-        for (int c = 0; c < DH; c += 16) {
-            float z[16];
-            tmem_ld16(lrow + C_Z2 + c, z);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float h = silu(z[e] + b2[c + e]);
-                st_bf16(sm + T_H2, kmaj_off(r, c + e, DH), h);
-                st_bf16(sm + T_H2T, kmaj_off(c + e, r, TM), h);
-            }
-        }
+        tmem_ld16(lrow + C_Z2 + c0, z);
+        activate(b2, d2);
+        store16(sm + T_H2, DH, sm + T_H2T, c0, r, z);
         // layer 3 and the loss gradient dZ3 = grad_scale (y - t) on the valid outputs
         stage([&] { gemm(tmem + C_Y, sm + T_H2, sm + T_W3, DH, IDESC_O); });
         if (!ok) break;
-        {
-            float y[16];
-            tmem_ld16(lrow + C_Y, y);
+        if (cg == 0) {
+            tmem_ld16(lrow + C_Y, z);
 #pragma unroll
             for (int o = 0; o < DOUT; ++o) {
                 float d = 0.f;
                 if (valid && o < QTG_MLP_OUT) {
-                    d = y[o] + b3[o] - a.t[(size_t)(m0 + r) * DOUT + o];
+                    d = z[o] + b3[o] - tv[o < QTG_MLP_OUT ? o : 0];
                     loss += d * d;
                 }
-                const float g = a.grad_scale * d;
-                st_bf16(sm + T_DZ3, kmaj_off(r, o, DOUT), g);
-                st_bf16(sm + T_DZ3T, kmaj_off(o, r, TM), g);
+                z[o] = a.grad_scale * d;
             }
+            store16(sm + T_DZ3, DOUT, sm + T_DZ3T, 0, r, z);
         }
         // dH2 = dZ3 W3 and dW3^T += H2^T dZ3
         stage([&] {
@@ -688,17 +728,10 @@ __global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
                          IDESC_GT_O, (gacc || kk > 0) ? 1u : 0u);
         });
         if (!ok) break;
-        for (int c = 0; c < DH; c += 16) {
-            float dh[16], z[16];
-            tmem_ld16(lrow + C_DH2 + c, dh);
-            tmem_ld16(lrow + C_Z2 + c, z);
+        tmem_ld16(lrow + C_DH2 + c0, z);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float g = valid ? dh[e] * dsilu(z[e] + b2[c + e]) : 0.f;
-                st_bf16(sm + T_DZ2, kmaj_off(r, c + e, DH), g);
-                st_bf16(sm + T_DZ2T, kmaj_off(c + e, r, TM), g);
-            }
-        }
+        for (int e = 0; e < 16; ++e) z[e] = valid ? z[e] * d2[e] : 0.f;
+        store16(sm + T_DZ2, DH, sm + T_DZ2T, c0, r, z);
         // dH1 = dZ2 W2 and dW2^T += H1^T dZ2
         stage([&] {
             gemm(tmem + C_DH1, sm + T_DZ2, sm + T_W2T, DH, IDESC_H);
@@ -708,14 +741,10 @@ __global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
                          IDESC_GT_H, (gacc || kk > 0) ? 1u : 0u);
         });
         if (!ok) break;
-        for (int c = 0; c < DH; c += 16) {
-            float dh[16], z[16];
-            tmem_ld16(lrow + C_DH1 + c, dh);
-            tmem_ld16(lrow + C_Z1 + c, z);
+        tmem_ld16(lrow + C_DH1 + c0, z);
 #pragma unroll
-            for (int e = 0; e < 16; ++e)
-                st_bf16(sm + T_DZ1T, kmaj_off(c + e, r, TM), valid ? dh[e] * dsilu(z[e] + b1[c + e]) : 0.f);
-        }
+        for (int e = 0; e < 16; ++e) z[e] = valid ? z[e] * d1[e] : 0.f;
+        store16(nullptr, DH, sm + T_DZ1T, c0, r, z);
         // dW1^T += X^T dZ1
         stage([&] {
             const uint32_t sa = smem_u32(sm + T_XT), sb = smem_u32(sm + T_DZ1T);
@@ -727,33 +756,33 @@ __global__ void __launch_bounds__(TM, 1) k_mlp_train(TrainArgs a) {
     // per-CTA partial: weight and bias gradients from the accumulators, the loss sum
     float *part = a.partial + (size_t)blockIdx.x * NPART;
     if (ok) {
-        const int i = tid;  // accumulator lane = input feature (or the bias row)
-        for (int c = 0; c < DH; c += 16) {
-            float g[16];
-            if (my_tiles > 0) tmem_ld16(lrow + C_GW1 + c, g);
-            else
-                for (int e = 0; e < 16; ++e) g[e] = 0.f;
-            for (int e = 0; e < 16; ++e) {
-                if (i < DIN) part[P_W1 + (c + e) * DIN + i] = g[e];
-                else if (i == DIN) part[P_B1 + c + e] = g[e];
-            }
-            if (my_tiles > 0) tmem_ld16(lrow + C_GW2 + c, g);
-            for (int e = 0; e < 16; ++e) {
-                if (i < DH) part[P_W2 + (c + e) * DH + i] = g[e];
-                else if (i == DH) part[P_B2 + c + e] = g[e];
-            }
-        }
+        const int i = r;  // accumulator lane = input feature (or the bias row)
         float g[16];
-        if (my_tiles > 0) tmem_ld16(lrow + C_GW3, g);
-        else
-            for (int e = 0; e < 16; ++e) g[e] = 0.f;
-        for (int o = 0; o < DOUT; ++o) {
-            const float v = o < QTG_MLP_OUT ? g[o] : 0.f;
-            if (i < DH) part[P_W3 + o * DH + i] = v;
-            else if (i == DH) part[P_B3 + o] = v;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) g[k] = 0.f;
+        if (my_tiles > 0) tmem_ld16(lrow + C_GW1 + c0, g);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (i < DIN) part[P_W1 + (c0 + k) * DIN + i] = g[k];
+            else if (i == DIN) part[P_B1 + c0 + k] = g[k];
         }
-        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-        if (lane == 0) red[warp] = loss;
+        if (my_tiles > 0) tmem_ld16(lrow + C_GW2 + c0, g);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (i < DH) part[P_W2 + (c0 + k) * DH + i] = g[k];
+            else if (i == DH) part[P_B2 + c0 + k] = g[k];
+        }
+        if (cg == 0) {
+            if (my_tiles > 0) tmem_ld16(lrow + C_GW3, g);
+#pragma unroll
+            for (int o = 0; o < DOUT; ++o) {
+                const float v = o < QTG_MLP_OUT ? g[o] : 0.f;
+                if (i < DH) part[P_W3 + o * DH + i] = v;
+                else if (i == DH) part[P_B3 + o] = v;
+            }
+            for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+            if (lane == 0) red[warp] = loss;
+        }
         __syncthreads();
         if (tid == 0) part[NPAR] = red[0] + red[1] + red[2] + red[3];
     } else {
@@ -770,7 +799,14 @@ __global__ void k_reduce_partials(const float *partial, int n_cta, float *out) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= NPART) return;
     float s = 0.f;
-    for (int c = 0; c < n_cta; ++c) s += partial[(size_t)c * NPART + e];
+    for (int c0 = 0; c0 < n_cta; c0 += 16) {  // sixteen loads in flight, then their sums in order
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = c0 + k < n_cta ? partial[(size_t)(c0 + k) * NPART + e] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (c0 + k < n_cta) s += v[k];
+    }
     out[e] = s;
 }
 
@@ -1037,8 +1073,8 @@ qtg_status qtg_mlp_train_batch(const qtg_mlp_weights *w, const void *x_bf16, con
     int grid = grid_for(tiles, 1);
     if (grid > max_ctas) grid = max_ctas;
     cudaStream_t s = (cudaStream_t)stream;
-    qtg::k_mlp_train<<<grid, qtg::TM, train_smem(), s>>>(a);
-    qtg::k_reduce_partials<<<(qtg::NPART + 255) / 256, 256, 0, s>>>(partial, grid, grad_out);
+    qtg::k_mlp_train<<<grid, qtg::TT, train_smem(), s>>>(a);
+    qtg::k_reduce_partials<<<(qtg::NPART + 63) / 64, 64, 0, s>>>(partial, grid, grad_out);
     return cudaGetLastError() == cudaSuccess ? QTG_OK : QTG_ERR_CUDA;
 }
 
