@@ -1584,7 +1584,58 @@ __global__ void __launch_bounds__(FT) k_kforce(EvalArgs a) {
 // -- take eight FMAs per +-kz pair, and A enters once per column:
 // sum v = pi (U1 + W0x) + pr (U2 - W0y), sum kz v = pi U3 + pr U4 (W0: kz = 0).
 // The batch's weights are staged as (sx, dy, dx, sy) and kz (dx, sy, sx, dy);
-// a site's Z(1 .. ZM) stays in registers, its X and Y rows in shared memory.
+// a site's Z(1 .. ZM) stays in registers, its Y rows in shared memory (X, reloaded where
+// the columns' kx changes, in registers: with it in shared memory too, and a test before
+// each |kz|, 4096 waters took 44 us, now 33; 512 waters, 32 beads 39.7 either way, where
+// the step gained 2 us from the room left to the kernels beside it).
+template <int ZM, typename F>
+__device__ __forceinline__ void kz_rows(int m, const F &rows) {  // rows(m), m <= ZM <= 14
+    switch (m) {
+        case 1:
+            if constexpr (ZM >= 1) rows(std::integral_constant<int, 1>{});
+            break;
+        case 2:
+            if constexpr (ZM >= 2) rows(std::integral_constant<int, 2>{});
+            break;
+        case 3:
+            if constexpr (ZM >= 3) rows(std::integral_constant<int, 3>{});
+            break;
+        case 4:
+            if constexpr (ZM >= 4) rows(std::integral_constant<int, 4>{});
+            break;
+        case 5:
+            if constexpr (ZM >= 5) rows(std::integral_constant<int, 5>{});
+            break;
+        case 6:
+            if constexpr (ZM >= 6) rows(std::integral_constant<int, 6>{});
+            break;
+        case 7:
+            if constexpr (ZM >= 7) rows(std::integral_constant<int, 7>{});
+            break;
+        case 8:
+            if constexpr (ZM >= 8) rows(std::integral_constant<int, 8>{});
+            break;
+        case 9:
+            if constexpr (ZM >= 9) rows(std::integral_constant<int, 9>{});
+            break;
+        case 10:
+            if constexpr (ZM >= 10) rows(std::integral_constant<int, 10>{});
+            break;
+        case 11:
+            if constexpr (ZM >= 11) rows(std::integral_constant<int, 11>{});
+            break;
+        case 12:
+            if constexpr (ZM >= 12) rows(std::integral_constant<int, 12>{});
+            break;
+        case 13:
+            if constexpr (ZM >= 13) rows(std::integral_constant<int, 13>{});
+            break;
+        case 14:
+            if constexpr (ZM >= 14) rows(std::integral_constant<int, 14>{});
+            break;
+    }
+}
+
 template <int ZM, int SPT>  // SPT: sites per thread (the block's weights serve SPT x FT sites)
 __global__ void __launch_bounds__(FT) k_kforce_f32(EvalArgs a) {
     constexpr int NS = SPT * FT;  // sites per block
@@ -1598,15 +1649,17 @@ __global__ void __launch_bounds__(FT) k_kforce_f32(EvalArgs a) {
     __shared__ float4 P1[KB], P2[KB];
     __shared__ int4 cs[KB];      // kx, ky, m, packed slot of kz = 0
     __shared__ float2 cb[KB];    // b_x kx, b_y ky
-    extern __shared__ float2 xyrow[];  // [2 km1][NS]: this block's sites' X(0 .. k_max), Y(0 .. k_max)
+    extern __shared__ float2 yrow[];  // [km1][NS]: this block's sites' Y(0 .. k_max)
     const float2 *ph = reinterpret_cast<const float2 *>(a.phase) + J.phase_off;
     int site[SPT];
-    float2 z[SPT][ZM];
+    float2 z[SPT][ZM], x[SPT];  // x: X(kx) of the columns at hand, which come sorted by kx
+    int kx = bt0 < bt1 ? a.kfc[S.col_off + a.kbatch[S.batch_off + bt0].c0].x : 0;
 #pragma unroll
     for (int u = 0; u < SPT; ++u) {
         site[u] = blockIdx.x * NS + u * FT + threadIdx.x;
         const int ii = site[u] < ns ? site[u] : 0;
-        for (int r = 0; r < 2 * km1; ++r) xyrow[r * NS + u * FT + threadIdx.x] = ph[(size_t)r * ns + ii];
+        x[u] = ph[(size_t)kx * ns + ii];
+        for (int r = 0; r < km1; ++r) yrow[r * NS + u * FT + threadIdx.x] = ph[(size_t)(km1 + r) * ns + ii];
 #pragma unroll
         for (int az = 1; az <= ZM; ++az) {
             z[u][az - 1] = make_float2(0.f, 0.f);
@@ -1640,33 +1693,43 @@ __global__ void __launch_bounds__(FT) k_kforce_f32(EvalArgs a) {
         for (int u = 0; u < SPT; ++u) fx[u] = fy[u] = fz[u] = 0.f;
         for (int cc = 0; cc < ncol; ++cc) {
             const int4 C = cs[cc];
+            if (C.x != kx) {
+                kx = C.x;
+#pragma unroll
+                for (int u = 0; u < SPT; ++u) x[u] = ph[(size_t)kx * ns + min(site[u], ns - 1)];
+            }
             const float4 w0 = P1[C.w];
             float pr[SPT], pi[SPT], u1[SPT], u2[SPT], u3[SPT], u4[SPT];
 #pragma unroll
             for (int u = 0; u < SPT; ++u) {
-                const float2 x = xyrow[C.x * NS + u * FT + threadIdx.x];
-                const float2 y = xyrow[(km1 + abs(C.y)) * NS + u * FT + threadIdx.x];
+                const float2 y = yrow[abs(C.y) * NS + u * FT + threadIdx.x];
                 const float yi = C.y < 0 ? -y.y : y.y;
-                pr[u] = x.x * y.x - x.y * yi;
-                pi[u] = x.x * yi + x.y * y.x;
+                pr[u] = fmaf(x[u].x, y.x, -__fmul_rn(x[u].y, yi));
+                pi[u] = fmaf(x[u].y, y.x, __fmul_rn(x[u].x, yi));
                 u1[u] = w0.x;
                 u2[u] = -w0.y;
                 u3[u] = 0.f;
                 u4[u] = 0.f;
             }
+            // az = 1 .. m: for the usual k_max a body a value of m, straight through (all its
+            // weight loads can start at once); the loop with its test a step beyond
+            auto rows = [&](auto m) {
 #pragma unroll
-            for (int az = 1; az <= ZM; ++az) {
-                if (az > C.z) break;
-                const float4 p1 = P1[C.w + az], p2 = P2[C.w + az];
+                for (int az = 1; az <= decltype(m)::value; ++az) {
+                    if (ZM > 14 && az > C.z) break;
+                    const float4 p1 = P1[C.w + az], p2 = P2[C.w + az];
 #pragma unroll
-                for (int u = 0; u < SPT; ++u) {
-                    const float zx = z[u][az - 1].x, zy = z[u][az - 1].y;
-                    u1[u] = fmaf(zx, p1.x, fmaf(zy, p1.y, u1[u]));
-                    u2[u] = fmaf(zy, p1.z, fmaf(-zx, p1.w, u2[u]));
-                    u3[u] = fmaf(zx, p2.x, fmaf(zy, p2.y, u3[u]));
-                    u4[u] = fmaf(zy, p2.z, fmaf(-zx, p2.w, u4[u]));
+                    for (int u = 0; u < SPT; ++u) {
+                        const float zx = z[u][az - 1].x, zy = z[u][az - 1].y;
+                        u1[u] = fmaf(zx, p1.x, fmaf(zy, p1.y, u1[u]));
+                        u2[u] = fmaf(zy, p1.z, fmaf(-zx, p1.w, u2[u]));
+                        u3[u] = fmaf(zx, p2.x, fmaf(zy, p2.y, u3[u]));
+                        u4[u] = fmaf(zy, p2.z, fmaf(-zx, p2.w, u4[u]));
+                    }
                 }
-            }
+            };
+            if constexpr (ZM > 14) rows(std::integral_constant<int, ZM>{});
+            else kz_rows<ZM>(C.z, rows);
             const float2 b = cb[cc];
 #pragma unroll
             for (int u = 0; u < SPT; ++u) {
@@ -1705,11 +1768,12 @@ void launch_ksk(const EvalArgs &a, dim3 grid, cudaStream_t s) {
 // the FP32 k-force kernel for the largest |kz| of the batch (the general form beyond 32)
 void launch_kforce_f32(const EvalArgs &a, dim3 grid, cudaStream_t s) {
     // two sites a thread (the block covers 2 FT sites: grid.x halves)
-    const size_t sm = (size_t)2 * (a.max_kmax + 1) * 2 * FT * sizeof(float2);
+    const size_t sm = (size_t)(a.max_kmax + 1) * 2 * FT * sizeof(float2);
     dim3 g2 = grid;
     g2.x = (grid.x + 1) / 2;
     if (a.kpk && a.max_kmax <= 8) launch_pdl(k_kforce_f32<8, 2>, g2, dim3(FT), sm, s, a);
-    else if (a.kpk && a.max_kmax <= 12) launch_pdl(k_kforce_f32<12, 2>, g2, dim3(FT), sm, s, a);
+    else if (a.kpk && a.max_kmax <= 10) launch_pdl(k_kforce_f32<10, 2>, g2, dim3(FT), sm, s, a);
+    else if (a.kpk && a.max_kmax <= 14) launch_pdl(k_kforce_f32<14, 2>, g2, dim3(FT), sm, s, a);
     else if (a.kpk && a.max_kmax <= 16) launch_pdl(k_kforce_f32<16, 2>, g2, dim3(FT), sm, s, a);
     else if (a.kpk && a.max_kmax <= 24) launch_pdl(k_kforce_f32<24, 2>, g2, dim3(FT), sm, s, a);
     else if (a.kpk && a.max_kmax <= 32) launch_pdl(k_kforce_f32<32, 2>, g2, dim3(FT), sm, s, a);
@@ -2396,7 +2460,8 @@ template <typename R>
 void set_attrs() {
     const int big = 200 * 1024;
     cudaFuncSetAttribute(k_kforce_f32<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_kforce_f32<12, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_kforce_f32<10, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_kforce_f32<14, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_kforce_f32<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_kforce_f32<24, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_kforce_f32<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
