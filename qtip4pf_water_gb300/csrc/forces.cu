@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(128) k_prep_f32(EvalArgs a) {
         float *o = reinterpret_cast<float *>(a.opos) + 4 * ((size_t)J.site_off / 3 + mol);
         o[d] = (float)FO * S.fixf[d];
         if (d == 0) o[3] = 0.f;
+        if (a.lj_half) a.lj64[4 * ((size_t)J.site_off / 3 + mol) + d] = 0.0;  // k_lj adds into it
     }
     const unsigned F = (unsigned)__double2ll_rn(x * S.fix_scale[d]);
     float *sv = reinterpret_cast<float *>(a.sites) + 4 * ((size_t)J.site_off + s);
@@ -1977,16 +1978,18 @@ __global__ void __launch_bounds__(128) k_combine_f32(EvalArgs a) {
         // M-site chain rule (forces.cpp:613-619); the dense Lennard-Jones force of a
         // forked evaluation joins the oxygen here
         const float g = (float)a.c.gamma_vs, h = 0.5f * (1.0f - g);
-        float lj[3] = {0.f, 0.f, 0.f};
+        double lj[3] = {0.0, 0.0, 0.0};
         if (a.lj_plane && J.mode == 0) {
             const float4 l = a.ljf[J.site_off / 3 + m];
-            lj[0] = l.x;
-            lj[1] = l.y;
-            lj[2] = l.z;
+            lj[0] = (double)l.x;
+            lj[1] = (double)l.y;
+            lj[2] = (double)l.z;
+        } else if (a.lj_half && J.mode == 0) {
+            for (int d = 0; d < 3; ++d) lj[d] = a.lj64[4 * ((size_t)J.site_off / 3 + m) + d];
         }
         double *f2 = a.out_prop ? a.out_prop + J.out_off + 9 * m : nullptr;
         for (int d = 0; d < 3; ++d) {
-            const double fo = (double)(fa[d] + g * fs[d]) + (double)lj[d];
+            const double fo = (double)(fa[d] + g * fs[d]) + lj[d];
             const double f1 = (double)(fa[3 + d] + fs[3 + d] + h * fs[d]);
             const double f2v = (double)(fa[6 + d] + fs[6 + d] + h * fs[d]);
             f[d] = fo;
@@ -2034,7 +2037,9 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     // a row's force needs no atomics and the energy is halved
     if (i < (FULL ? N : N - 1)) {
         const double *q = a.pos + J.pos_off;
-        double *f = a.out + J.out_off;
+        // the forces, or their own array (lj_half: the kernel runs beside the others)
+        double *f = !FULL && a.lj_half ? a.lj64 + 4 * ((size_t)J.site_off / 3) : a.out + J.out_off;
+        const int fs = !FULL && a.lj_half ? 4 : 9;
         const int cap = FULL ? 2 * S.list_size : S.list_size;
         const int *pt = FULL ? a.point_full + S.pf_off + (size_t)J.bead * (N + 1)
                              : a.point + S.pt_off + (size_t)J.bead * N;
@@ -2102,9 +2107,9 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
                 fi1 += ff * r[1];
                 fi2 += ff * r[2];
                 if (!FULL) {
-                    atomicAdd(&f[9 * j], -(double)(ff * r[0]));
-                    atomicAdd(&f[9 * j + 1], -(double)(ff * r[1]));
-                    atomicAdd(&f[9 * j + 2], -(double)(ff * r[2]));
+                    atomicAdd(&f[fs * j], -(double)(ff * r[0]));
+                    atomicAdd(&f[fs * j + 1], -(double)(ff * r[1]));
+                    atomicAdd(&f[fs * j + 2], -(double)(ff * r[2]));
                 }
             }
         }
@@ -2118,9 +2123,9 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
                 f[9 * i + 1] += d1;
                 f[9 * i + 2] += d2;
             } else {
-                atomicAdd(&f[9 * i], d0);
-                atomicAdd(&f[9 * i + 1], d1);
-                atomicAdd(&f[9 * i + 2], d2);
+                atomicAdd(&f[fs * i], d0);
+                atomicAdd(&f[fs * i + 1], d1);
+                atomicAdd(&f[fs * i + 2], d2);
             }
         } else {
             e = 0.0;
@@ -2571,16 +2576,13 @@ void launch_recip(const EvalArgs &a, cudaStream_t s) {
     launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
 }
 
-template <typename R>
-void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks *forks = nullptr) {
+void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks *forks) {
     const int ns = 3 * a.max_mols;
     const int tiles = (ns + RT - 1) / RT, ktiles = (a.max_grp + KT - 1) / KT;
     a.n_rj = chunks_or(a.tune_rj, (long long)tiles * a.n_jobs, MAX_RJ);
-    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
-    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
-    if (ksk2_ok(a)) set_ksk2_chunks(a);
-    if (forks && a.mode == 0 && a.lj_full && a.ljf) {
-        // forked: prep; then real space | reciprocal chain | dense LJ; then combine.
+    if (a.mode == 0) {
+        // forked: prep; then real space | reciprocal chain | LJ (every pair, or the caller's
+        // half list by atomics); then combine.
         // The reciprocal chain runs beside the real-space kernel: its grids aim for
         // a third (structure factors) and half (k-force) of the blocks a kernel alone
         // would (the autotuner's picks on the 512-water P = 32 step)
@@ -2592,7 +2594,8 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             a.real_fix = 1;
         }
         else if (list_ok(a)) a.n_rj = list_chunks(a);  // k_kforce_f32's planes follow the real-space ones
-        a.lj_plane = 1;
+        if (a.lj_full) a.lj_plane = 1;
+        else a.lj_half = 1;
         launch_prep_f32(a, s);
         // capture order: the reciprocal chain (the critical path: three dependent
         // kernels) first, then the Lennard-Jones branch, the real-space kernel last
@@ -2604,7 +2607,8 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         launch_recip(a, forks->side[0]);
         cudaEventRecord(forks->join[0], forks->side[0]);
         if (a.lj_list && forks->lists_ready) cudaStreamWaitEvent(forks->side[1], forks->lists_ready, 0);
-        launch_lj_dense(a, forks->side[1]);
+        if (a.lj_full) launch_lj_dense(a, forks->side[1]);
+        else k_lj<float, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         if (a.intra) {
             a.intra_plane = 1;
             k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
@@ -2619,45 +2623,21 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         if (n) *n += (a.intra_plane ? 8 : 7) + (list_ok(a) ? 2 : 0);
         return;
     }
+    // the derivative: real space beside the reciprocal chain
+    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
+    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
     launch_prep_f32(a, s);
-    if (a.mode == 0) {
-        if (half_ok(a)) launch_real_half(a, s);
-        else if (list_ok(a)) {
-            launch_real_list(a, s);
-            if (n) *n += 2;
-        } else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        launch_recip(a, s);
-    } else {
-        // the derivative: real space beside the reciprocal chain
-        cudaStream_t rs = s;
-        if (forks) {
-            rs = forks->side[0];
-            cudaEventRecord(forks->fork, s);
-            cudaStreamWaitEvent(rs, forks->fork, 0);
-        }
-        launch_ksk<R, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
-        launch_sk_reduce<R, 1>(a, rs);
-        k_kforce<R, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<R>(a.max_kmax), rs>>>(a);
-        k_real<R, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
-        if (forks) {
-            cudaEventRecord(forks->join[0], rs);
-            cudaStreamWaitEvent(s, forks->join[0], 0);
-        }
-    }
-    // mixed with the dense Lennard-Jones: its oxygen forces go to their plane first,
-    // so the combine writes the complete force
-    const bool plane = a.mode == 0 && a.lj_full && a.ljf;
-    if (plane) {
-        a.lj_plane = 1;
-        launch_lj_dense(a, s);
-    }
+    cudaStream_t rs = forks->side[0];
+    cudaEventRecord(forks->fork, s);
+    cudaStreamWaitEvent(rs, forks->fork, 0);
+    launch_ksk<float, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
+    launch_sk_reduce<float, 1>(a, rs);
+    k_kforce<float, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<float>(a.max_kmax), rs>>>(a);
+    k_real<float, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
+    cudaEventRecord(forks->join[0], rs);
+    cudaStreamWaitEvent(s, forks->join[0], 0);
     k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
-    if (n) *n += plane ? 7 : 6;
-    if (a.mode == 0 && !plane) {
-        if (a.lj_full) launch_lj_dense(a, s);
-        else k_lj<R, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
-        if (n) *n += 1;
-    }
+    if (n) *n += 6;
 }
 
 // Chunk counts of the FP64 reciprocal space: whole 32-site shared-memory chunks of the
@@ -2789,7 +2769,7 @@ void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *n,
         launch_eval_fp64(a, s, n, nullptr);  // the finite-difference short-range terms stay FP64
         return;
     }
-    launch_ewald<float>(a, s, n, forks);
+    launch_ewald(a, s, n, forks);
 }
 
 // Reciprocal space only, on caller-supplied charge sites: out (site forces,

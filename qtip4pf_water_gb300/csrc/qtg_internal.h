@@ -537,6 +537,7 @@ struct EvalArgs {
     void *opos;            // mixed: wrapped oxygen positions, 4 floats per molecule, per slot
     float4 *opos32;        // FP64 evaluations: the same, for k_lj64's screening
     double *lj64;          // FP64 evaluations: Lennard-Jones oxygen forces, 4 doubles per molecule, per slot
+    int lj_half;           // mixed, forked, half lists: 1: k_lj adds into lj64 (zeroed by k_prep_f32)
     double *intra64;       // FP64 evaluations: intramolecular site and atom forces, 18 doubles per molecule, per slot
     float4 *ljf;           // dense Lennard-Jones oxygen forces, per molecule, per slot (lj_plane)
     int lj_plane;          // 1: k_lj_dense writes ljf and k_combine_f32 adds it to the O force
@@ -675,8 +676,7 @@ struct Forks {
     cudaEvent_t sc_fork, sc_join;
     cudaEvent_t lists_ready;  // set: the Verlet-list rebuild runs beside the forces; the list LJ waits for it
 };
-void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *launches,
-                       const Forks *forks = nullptr);
+void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *launches, const Forks *forks);
 void launch_kwald_only(const EvalArgs &a, bool mixed, cudaStream_t s, unsigned long long *launches);
 
 // one-time kernel attribute set-up (shared-memory limits); called at context creation
