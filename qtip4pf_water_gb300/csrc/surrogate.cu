@@ -409,21 +409,21 @@ __device__ __forceinline__ void load_tile(uint8_t *tile, const __nv_bfloat16 *sr
     }
 }
 
-// bias + SiLU on this thread's row of a 64-column accumulator, into a BF16 A tile;
-// z keeps the pre-activations
-__device__ __forceinline__ void epilogue_silu(uint32_t tmem_row, const float *bias, uint8_t *tile, int r,
-                                              float *z) {
+// Sixteen warps share a tile: warp w has the 32 rows of TMEM quadrant w mod 4 and 16 of a
+// layer's 64 columns, from 16 (w / 4) on (four warps, one row a thread, spent 24 us on the
+// 64 tiles of 4096 waters, nearly all of it in the layers' elementwise work).
+constexpr int TT = 512;
+
+// bias + SiLU on 16 columns of row r from a 64-column accumulator, into a BF16 A tile
+__device__ __forceinline__ void epilogue_silu(uint32_t tmem_at, const float *bias, uint8_t *tile, int r, int c0) {
+    float z[16];
+    tmem_ld16(tmem_at, z);
 #pragma unroll
-    for (int c = 0; c < DH; c += 16) tmem_ld16(tmem_row + c, z + c);
-#pragma unroll
-    for (int kg = 0; kg < DH / 8; ++kg) {
+    for (int kg = 0; kg < 2; ++kg) {
         float h[8];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            z[kg * 8 + t] += bias[kg * 8 + t];
-            h[t] = silu(z[kg * 8 + t]);
-        }
-        *reinterpret_cast<uint4 *>(tile + kmaj_off(r, kg * 8, DH)) =
+        for (int t = 0; t < 8; ++t) h[t] = silu(z[kg * 8 + t] + bias[c0 + kg * 8 + t]);
+        *reinterpret_cast<uint4 *>(tile + kmaj_off(r, c0 + kg * 8, DH)) =
             make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
     }
 }
@@ -435,21 +435,21 @@ __device__ __forceinline__ void gemm(uint32_t d_tmem, const uint8_t *a, const ui
         mma_bf16(d_tmem, sdesc(sa + kk * 256, 128, sbo), sdesc(sb + kk * 256, 128, sbo), idesc, kk > 0 ? 1u : 0u);
 }
 
-// One CTA of 128 threads per tile of 128 molecules (persistent over tiles);
-// thread r owns row r of the tile, which is TMEM lane r.
-__global__ void __launch_bounds__(TM) k_mlp_fwd(MlpArgs a) {
+// One CTA per tile of 128 molecules (persistent over tiles); row r of the tile is TMEM lane r.
+__global__ void __launch_bounds__(TT) k_mlp_fwd(MlpArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float *b1 = reinterpret_cast<float *>(sm + F_B), *b2 = b1 + DH, *b3 = b2 + DH;
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm + F_MISC);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + F_MISC + 8);
     const int tid = threadIdx.x, warp = tid >> 5;
+    const int c0 = 16 * (warp >> 2), r = (warp & 3) * 32 + (tid & 31);  // my columns and tile row
     load_tile(sm + F_W1, a.w1, DH, DIN, 0, DH);
     load_tile(sm + F_W2, a.w2, DH, DH, 0, DH);
     load_tile(sm + F_W3, a.w3, DOUT, DH, 0, DOUT);
-    for (int k = tid; k < DH; k += TM) {
-        b1[k] = a.b1[k];
-        b2[k] = a.b2[k];
+    if (tid < DH) {
+        b1[tid] = a.b1[tid];
+        b2[tid] = a.b2[tid];
     }
     if (tid < DOUT) b3[tid] = a.b3[tid];
     if (tid == 0) mbar_init(smem_u32(mbar), 1);
@@ -458,14 +458,13 @@ __global__ void __launch_bounds__(TM) k_mlp_fwd(MlpArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tslot, lane_base = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem = *tslot, lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t phase = 0;
     bool ok = true;
     const int n_tiles = (a.m + TM - 1) / TM;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         const int m0 = t * TM;
         load_tile(sm + F_X, a.x, TM, DIN, m0, a.m);
-        float z[DH];
         const uint8_t *ain[3] = {sm + F_X, sm + F_H1, sm + F_H2};
         const uint8_t *bw[3] = {sm + F_W1, sm + F_W2, sm + F_W3};
         const int kin[3] = {DIN, DH, DH};
@@ -485,13 +484,13 @@ __global__ void __launch_bounds__(TM) k_mlp_fwd(MlpArgs a) {
             if (!ok) break;
             tc_fence_after();
             const uint32_t row = tmem + lane_base + dcol[layer];
-            if (layer == 0) epilogue_silu(row, b1, sm + F_H1, tid, z);
-            else if (layer == 1) epilogue_silu(row, b2, sm + F_H2, tid, z);
-            else {
+            if (layer == 0) epilogue_silu(row + c0, b1, sm + F_H1, r, c0);
+            else if (layer == 1) epilogue_silu(row + c0, b2, sm + F_H2, r, c0);
+            else if (c0 == 0) {
                 float o[DOUT];
                 tmem_ld16(row, o);
-                if (m0 + tid < a.m) {
-                    float4 *dst = reinterpret_cast<float4 *>(a.y + (size_t)(m0 + tid) * DOUT);
+                if (m0 + r < a.m) {
+                    float4 *dst = reinterpret_cast<float4 *>(a.y + (size_t)(m0 + r) * DOUT);
 #pragma unroll
                     for (int c = 0; c < DOUT; c += 4)
                         dst[c / 4] = make_float4(o[c] + b3[c], o[c + 1] + b3[c + 1], o[c + 2] + b3[c + 2],
@@ -598,7 +597,6 @@ __device__ __forceinline__ void store16(uint8_t *rows, int K, uint8_t *cols, int
 // two rows at a time, and the next tile's inputs are loaded while this one is worked on.
 // 442368 rows: 800 us with four warps, one row a thread and two-byte stores; see
 // qtg_mlp_train_batch's launch.
-constexpr int TT = 512;
 __global__ void __launch_bounds__(TT, 1) k_mlp_train(TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -938,7 +936,7 @@ void launch_surrogate_prepare(const SurrogateRun &r, cudaStream_t s, unsigned lo
     a.y = r.y;
     a.status = r.status;
     const int tiles = (2 * N + TM - 1) / TM;
-    k_mlp_fwd<<<tiles < 2 * r.n_sm ? tiles : 2 * r.n_sm, TM, (size_t)F_END + 1024, s>>>(a);
+    k_mlp_fwd<<<tiles < 2 * r.n_sm ? tiles : 2 * r.n_sm, TT, (size_t)F_END + 1024, s>>>(a);
     k_frames<<<(N + 127) / 128, 128, 0, s>>>(r.pos, N, r.box[0], r.box[1], r.box[2], r.frames);
     if (launches) *launches += 5;
 }
@@ -1036,7 +1034,7 @@ qtg_status qtg_mlp_forward(const qtg_mlp_weights *w, const void *x_bf16, int m, 
     a.y = y;
     a.status = st;
     const int tiles = (m + qtg::TM - 1) / qtg::TM;
-    qtg::k_mlp_fwd<<<grid_for(tiles, 2), qtg::TM, fwd_smem(), (cudaStream_t)stream>>>(a);
+    qtg::k_mlp_fwd<<<grid_for(tiles, 2), qtg::TT, fwd_smem(), (cudaStream_t)stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? QTG_OK : QTG_ERR_CUDA;
 }
 
