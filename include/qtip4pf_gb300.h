@@ -102,6 +102,9 @@ qtg_status qtg_set_masses(qtg_ctx *ctx, int sys, const double *mass);
  * Bit-identical CSR list; the bead's disp slice is zeroed. */
 qtg_status qtg_neighbour_list(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list,
                               double *disp, int bead);
+/* The same for every bead of the system by one build (the reference loops over the beads). */
+qtg_status qtg_neighbour_lists(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list,
+                               double *disp);
 /* forces.cpp:468-630  double get_forces_nospline(pos, f, charge, point, list, bead)
  * Writes the bead's slice of f and the bead's potential energy. */
 qtg_status qtg_get_forces(qtg_ctx *ctx, int sys, const double *pos, double *f,

@@ -92,6 +92,7 @@ def load(build_if_missing: bool = True):
         "qtg_set_charges": ([V, C.c_int, D], C.c_int),
         "qtg_set_masses": ([V, C.c_int, D], C.c_int),
         "qtg_neighbour_list": ([V, C.c_int, D, I, I, D, C.c_int], C.c_int),
+        "qtg_neighbour_lists": ([V, C.c_int, D, I, I, D], C.c_int),
         "qtg_get_forces": ([V, C.c_int, D, D, D, I, I, C.c_int, D], C.c_int),
         "qtg_kwald": ([V, C.c_int, D, D, D, C.c_int, D], C.c_int),
         "qtg_force_eval_sc": ([V, C.c_int, D, D, D, D, I, I, D, D, D], C.c_int),
@@ -386,8 +387,7 @@ class System:
 
     def build_lists(self, pos):
         point, lst, disp = self.new_lists()
-        for b in range(self.P):
-            self.neighbour_list(pos, point, lst, disp, b)
+        self._c(self.ctx.L.qtg_neighbour_lists(self.ctx.h, self.idx, _d(pos), _i(point), _i(lst), _d(disp)))
         return point, lst, disp
 
     def get_forces_nospline(self, pos, f, charge, point, lst, bead=0):

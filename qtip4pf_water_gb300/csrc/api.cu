@@ -765,10 +765,13 @@ qtg_status status_error(qtg_ctx *ctx, unsigned st) {
     return QTG_OK;
 }
 
+// The status word comes back through the pinned mailbox, so that one stream
+// synchronisation resolves it with everything else on its way there (each copy to
+// pageable memory waits for the stream by itself: some 9 us).
 qtg_status sync_status(qtg_ctx *ctx) {
+    CK(cudaMemcpyAsync(&ctx->box->status, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    unsigned st = 0;
-    CK(cudaMemcpy(&st, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    const unsigned st = ctx->box->status;
     if (st) CK(cudaMemset(ctx->status, 0, sizeof(unsigned)));
     return status_error(ctx, st);
 }
@@ -1794,32 +1797,80 @@ qtg_status qtg_set_masses(qtg_ctx *ctx, int sys, const double *mass) {
 
 // ---- tier 1 ------------------------------------------------------------------------
 
-qtg_status qtg_neighbour_list(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list, double *disp,
-                              int bead) {
-    CKS(check_sys(ctx, sys));
+// Beads [bead, bead + nb): one build for them all, one copy back for each array. A
+// forced build leaves zero displacements: the caller's are cleared here.
+static qtg_status build_bead_lists(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list, double *disp,
+                                   int bead, int nb) {
     const SysDev &S = ctx->sys_h[sys];
-    if (!pos || !point || !list || !disp || bead < 0 || bead >= S.n_beads) return fail(ctx, QTG_ERR_ARG, "bad argument");
-    const size_t nd = S.n_dof;
-    CK(up(ctx, ctx->q + S.q_off + bead * nd, pos + bead * nd, sizeof(double) * nd));
-    launch_skin_rebuild(list_args(ctx, S.job_base + bead, 1, 1), ctx->stream, &ctx->launches);
-    CK(down(ctx, point + (size_t)bead * S.n_mols, ctx->point + S.pt_off + (size_t)bead * S.n_mols, sizeof(int) * S.n_mols));
-    CK(down(ctx, list + (size_t)bead * S.list_size, ctx->list + S.ls_off + (size_t)bead * S.list_size,
-            sizeof(int) * S.list_size));
-    CK(down(ctx, disp + (size_t)bead * 3 * S.n_mols, ctx->disp + S.d_off + (size_t)bead * 3 * S.n_mols,
-            sizeof(double) * 3 * S.n_mols));
+    const size_t nd = S.n_dof, N = S.n_mols, cap = S.list_size;
+    CK(up(ctx, ctx->q + S.q_off + bead * nd, pos + bead * nd, sizeof(double) * nd * nb));
+    launch_skin_rebuild(list_args(ctx, S.job_base + bead, nb, 1), ctx->stream, &ctx->launches);
     CK(cudaMemsetAsync(ctx->acc + sys, 0, sizeof(SysAcc), ctx->stream));
+    memset(disp + bead * 3 * N, 0, sizeof(double) * 3 * N * nb);
+    CK(down(ctx, point + bead * N, ctx->point + S.pt_off + bead * N, sizeof(int) * N * nb));
+    CK(down(ctx, list + bead * cap, ctx->list + S.ls_off + bead * cap, sizeof(int) * cap * nb));
     return sync_status(ctx);
 }
 
-static qtg_status upload_lists(qtg_ctx *ctx, int sys, const int *point, const int *list, int bead_lo, int bead_hi) {
+qtg_status qtg_neighbour_list(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list, double *disp,
+                              int bead) {
+    CKS(check_sys(ctx, sys));
+    if (!pos || !point || !list || !disp || bead < 0 || bead >= ctx->sys_h[sys].n_beads)
+        return fail(ctx, QTG_ERR_ARG, "bad argument");
+    return build_bead_lists(ctx, sys, pos, point, list, disp, bead, 1);
+}
+
+qtg_status qtg_neighbour_lists(qtg_ctx *ctx, int sys, const double *pos, int *point, int *list, double *disp) {
+    CKS(check_sys(ctx, sys));
+    if (!pos || !point || !list || !disp) return fail(ctx, QTG_ERR_ARG, "bad argument");
+    return build_bead_lists(ctx, sys, pos, point, list, disp, 0, ctx->sys_h[sys].n_beads);
+}
+
+// The caller's lists go up as far as their rows reach: up to the largest entry of
+// point (a valid list fills about half of list_size), one strided copy for the beads.
+static cudaError_t copy_lists_up(qtg_ctx *ctx, int sys, const int *point, const int *list, int bead_lo, int bead_hi,
+                                 cudaStream_t s) {
     const SysDev &S = ctx->sys_h[sys];
-    const int nb = bead_hi - bead_lo;
-    CK(up(ctx, ctx->point + S.pt_off + (size_t)bead_lo * S.n_mols, point + (size_t)bead_lo * S.n_mols,
-          sizeof(int) * S.n_mols * nb));
-    CK(up(ctx, ctx->list + S.ls_off + (size_t)bead_lo * S.list_size, list + (size_t)bead_lo * S.list_size,
-          sizeof(int) * (size_t)S.list_size * nb));
+    const size_t N = S.n_mols, cap = S.list_size, nb = bead_hi - bead_lo, b0 = bead_lo;
+    const int *pt = point + b0 * N;
+    const cudaError_t e = cudaMemcpyAsync(ctx->point + S.pt_off + b0 * N, pt, sizeof(int) * N * nb,
+                                          cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    const int top = *std::max_element(pt, pt + N * nb);
+    const size_t width = std::min<size_t>(cap, std::max(top, 0));
+    ctx->h2d_bytes += sizeof(int) * (N + width) * nb;
+    if (width == 0) return cudaSuccess;
+    return cudaMemcpy2DAsync(ctx->list + S.ls_off + b0 * cap, sizeof(int) * cap, list + b0 * cap, sizeof(int) * cap,
+                             sizeof(int) * width, nb, cudaMemcpyHostToDevice, s);
+}
+static qtg_status upload_lists(qtg_ctx *ctx, int sys, const int *point, const int *list, int bead_lo, int bead_hi) {
+    CK(copy_lists_up(ctx, sys, point, list, bead_lo, bead_hi, ctx->stream));
     return QTG_OK;
 }
+
+// A force call over the caller's lists. Only the Lennard-Jones term reads them: in
+// this object's scope the next evaluation puts them up on that term's branch, while
+// the Ewald kernels run.
+struct CallLists {
+    qtg_ctx *ctx;
+    int sys;
+    const int *point, *list;
+    int bead_lo, bead_hi;
+    cudaError_t err;
+    CallLists(qtg_ctx *c, int s, const int *pt, const int *ls, int lo, int hi)
+        : ctx(c), sys(s), point(pt), list(ls), bead_lo(lo), bead_hi(hi), err(cudaSuccess) {
+        c->forks.put_lists = put;
+        c->forks.put_arg = this;
+    }
+    ~CallLists() { ctx->forks.put_lists = nullptr; }
+    CallLists(const CallLists &) = delete;
+    CallLists &operator=(const CallLists &) = delete;
+    static void put(void *arg, cudaStream_t s) {
+        CallLists *l = static_cast<CallLists *>(arg);
+        l->ctx->forks.put_lists = nullptr;  // once
+        l->err = copy_lists_up(l->ctx, l->sys, l->point, l->list, l->bead_lo, l->bead_hi, s);
+    }
+};
 
 qtg_status qtg_get_forces(qtg_ctx *ctx, int sys, const double *pos, double *f, const double *charge,
                           const int *point, const int *list, int bead, double *energy) {
@@ -1829,14 +1880,14 @@ qtg_status qtg_get_forces(qtg_ctx *ctx, int sys, const double *pos, double *f, c
     const size_t nd = S.n_dof;
     if (charge) CKS(upload_charges(ctx, sys, charge));
     CK(up(ctx, ctx->q + S.q_off + bead * nd, pos + bead * nd, sizeof(double) * nd));
-    CKS(upload_lists(ctx, sys, point, list, bead, bead + 1));
     const int jb = S.job_base + bead;
+    CallLists lists(ctx, sys, point, list, bead, bead + 1);
     launch_eval(ctx, eval_args(ctx, ctx->base.d + jb, 1, ctx->q, ctx->fphys, 0, 0));
+    CK(lists.err);
+    CK(down(ctx, ctx->box_energy, ctx->energy + jb, sizeof(double)));
     CK(down(ctx, f + bead * nd, ctx->fphys + S.q_off + bead * nd, sizeof(double) * nd));
-    double e = 0.0;
-    CK(down(ctx, &e, ctx->energy + jb, sizeof(double)));
     CKS(sync_status(ctx));
-    if (energy) *energy = e;
+    if (energy) *energy = ctx->box_energy[0];
     return QTG_OK;
 }
 
@@ -1854,22 +1905,26 @@ qtg_status qtg_kwald(qtg_ctx *ctx, int sys, const double *sites, double *f_sites
     EvalArgs a = eval_args(ctx, ctx->base.d + jb, 1, ctx->qdisp, ctx->stage, 0, 0);
     a.sites_are_input = 1;
     launch_kwald_only(a, ctx->mixed, ctx->stream, &ctx->launches);
+    CK(down(ctx, ctx->box_energy, ctx->energy + jb, sizeof(double)));
     CK(down(ctx, f_sites + bead * nd, ctx->stage + S.q_off + bead * nd, sizeof(double) * nd));
-    double e = 0.0;
-    CK(down(ctx, &e, ctx->energy + jb, sizeof(double)));
     CKS(sync_status(ctx));
-    if (energy) *energy = e;
+    if (energy) *energy = ctx->box_energy[0];
     return QTG_OK;
 }
 
+// enqueue the energies and accumulators of a force call (to the mailbox) and the
+// accumulators' clearing; read_energies takes them after the synchronisation
+static qtg_status post_energies(qtg_ctx *ctx, int sys) {
+    const SysDev &S = ctx->sys_h[sys];
+    CK(down(ctx, ctx->box_energy, ctx->energy + S.job_base, sizeof(double) * S.n_beads));
+    CK(down(ctx, &ctx->box->acc, ctx->acc + sys, sizeof(SysAcc)));
+    CK(cudaMemsetAsync(ctx->acc + sys, 0, sizeof(SysAcc), ctx->stream));
+    return QTG_OK;
+}
 static qtg_status read_energies(qtg_ctx *ctx, int sys, double *vsum, double *veven, double *sc_extra) {
     const SysDev &S = ctx->sys_h[sys];
-    std::vector<double> e(S.n_beads);
-    SysAcc acc;
-    CK(down(ctx, e.data(), ctx->energy + S.job_base, sizeof(double) * S.n_beads));
-    CK(down(ctx, &acc, ctx->acc + sys, sizeof(SysAcc)));
     CKS(sync_status(ctx));
-    CK(cudaMemsetAsync(ctx->acc + sys, 0, sizeof(SysAcc), ctx->stream));
+    const double *e = ctx->box_energy;
     double vs = 0.0, ve = 0.0;
     for (int b = 0; b < S.n_beads; ++b) {
         vs += e[b];
@@ -1877,7 +1932,7 @@ static qtg_status read_energies(qtg_ctx *ctx, int sys, double *vsum, double *vev
     }
     *vsum = vs;
     *veven = ve;
-    *sc_extra = acc.sc_extra;
+    *sc_extra = ctx->box->acc.sc_extra;
     return QTG_OK;
 }
 
@@ -1891,9 +1946,11 @@ qtg_status qtg_force_eval_sc(qtg_ctx *ctx, int sys, const double *pos, double *f
     if (charge) CKS(upload_charges(ctx, sys, charge));
     if (mass) CKS(upload_masses(ctx, sys, mass));
     CK(up(ctx, ctx->q + S.q_off, pos, sizeof(double) * nt));
-    CKS(upload_lists(ctx, sys, point, list, 0, S.n_beads));
     CK(cudaMemsetAsync(ctx->acc + sys, 0, sizeof(SysAcc), ctx->stream));
+    CallLists lists(ctx, sys, point, list, 0, S.n_beads);
     enqueue_forces(ctx, sys, true);
+    CK(lists.err);
+    CKS(post_energies(ctx, sys));
     CK(down(ctx, f, ctx->f + S.q_off, sizeof(double) * nt));
     CK(down(ctx, fphys, ctx->fphys + S.q_off, sizeof(double) * nt));
     double vs, ve, extra;
@@ -1911,8 +1968,10 @@ qtg_status qtg_force_eval_trotter(qtg_ctx *ctx, int sys, const double *pos, doub
     const size_t nt = (size_t)S.n_beads * S.n_dof;
     if (charge) CKS(upload_charges(ctx, sys, charge));
     CK(up(ctx, ctx->q + S.q_off, pos, sizeof(double) * nt));
-    CKS(upload_lists(ctx, sys, point, list, 0, S.n_beads));
+    CallLists lists(ctx, sys, point, list, 0, S.n_beads);
     launch_eval(ctx, eval_args(ctx, ctx->base.d + S.job_base, S.n_beads, ctx->q, ctx->fphys, 0, 0));
+    CK(lists.err);
+    CKS(post_energies(ctx, sys));
     CK(down(ctx, f, ctx->fphys + S.q_off, sizeof(double) * nt));
     double vs, ve, extra;
     CKS(read_energies(ctx, sys, &vs, &ve, &extra));

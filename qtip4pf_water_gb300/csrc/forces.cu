@@ -2607,16 +2607,22 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         launch_recip(a, forks->side[0]);
         cudaEventRecord(forks->join[0], forks->side[0]);
         if (a.lj_list && forks->lists_ready) cudaStreamWaitEvent(forks->side[1], forks->lists_ready, 0);
+        auto real = [&] {
+            if (half_ok(a)) launch_real_half(a, s);
+            else if (list_ok(a)) launch_real_list(a, s);
+            else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
+        };
+        if (a.intra) a.intra_plane = 1;
+        const bool put = forks->put_lists;
+        if (put) {
+            real();
+            forks->put_lists(forks->put_arg, forks->side[1]);
+        }
         if (a.lj_full) launch_lj_dense(a, forks->side[1]);
         else k_lj<float, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
-        if (a.intra) {
-            a.intra_plane = 1;
-            k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
-        }
+        if (a.intra) k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         cudaEventRecord(forks->join[1], forks->side[1]);
-        if (half_ok(a)) launch_real_half(a, s);
-        else if (list_ok(a)) launch_real_list(a, s);
-        else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
+        if (!put) real();
         cudaStreamWaitEvent(s, forks->join[0], 0);
         cudaStreamWaitEvent(s, forks->join[1], 0);
         k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
@@ -2669,8 +2675,13 @@ void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n, const For
     launch_sk_reduce64(a, rs);
     launch_kforce64(a, rs);
     launch_intra64(a, ls);
+    const bool put = forks && forks->put_lists;
+    if (put) {
+        launch_real64(a, s);
+        forks->put_lists(forks->put_arg, ls);
+    }
     launch_lj64(a, ls);
-    launch_real64(a, s);
+    if (!put) launch_real64(a, s);
     if (forks) {
         cudaEventRecord(forks->join[0], rs);
         cudaEventRecord(forks->join[1], ls);

@@ -675,6 +675,10 @@ struct Forks {
     cudaStream_t sc_stream;
     cudaEvent_t sc_fork, sc_join;
     cudaEvent_t lists_ready;  // set: the Verlet-list rebuild runs beside the forces; the list LJ waits for it
+    // set: enqueues the caller's lists on the branch of the Lennard-Jones term, which the
+    // host launches last then (a copy from pageable memory holds the host until it is done)
+    void (*put_lists)(void *arg, cudaStream_t s);
+    void *put_arg;
 };
 void launch_eval_mixed(const EvalArgs &a, cudaStream_t s, unsigned long long *launches, const Forks *forks);
 void launch_kwald_only(const EvalArgs &a, bool mixed, cudaStream_t s, unsigned long long *launches);
