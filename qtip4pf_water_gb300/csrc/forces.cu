@@ -1326,21 +1326,24 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
     }
 }
 
-// Sum of the structure-factor partials of every k (FP64, fixed order), the
-// reciprocal-space energy sum_k c_k |S(k)|^2, and the force weights 2 c_k S(k)
-// (and 2 c_k dS(k)) in the working precision for k_kforce. One thread per k.
-template <typename R, int MODE>
+// Sum of the structure-factor partials of every k in chunk order, the reciprocal-space
+// energy sum_k c_k |S(k)|^2, and the force weights 2 c_k S(k) (MODE 1, the derivative:
+// and 2 c_k dS(k)) for the k-force. One thread per k. Bound by latency: what does not
+// depend on k_ksk is read before the wait for it, and the partials come sixteen (MODE 1:
+// eight) loads at a time (four, resp. one, took 9.9 us at 216 waters, 1 bead against 7.4,
+// resp. 18 us for the derivative of 512 waters, 16 beads).
+// MODE 0: k_ksk's partials; MODE 2: k_ksk2's, which need fewer registers.
+template <int MODE>
 __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
     pdl_launch_dependents();  // the k-force may start its staging of the phase rows
-    pdl_wait();               // the structure-factor partials of k_ksk
     const int jb = blockIdx.y;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
-    // FP32 energy/force form: the half set, each kx = 0, ky > 0 vector standing for
+    // energy/force forms: the half set, each kx = 0, ky > 0 vector standing for
     // itself and its conjugate partner (|S|^2 and the force are the same for both),
     // one block per force batch (whole columns, <= 128 vectors), so that the block
     // also packs the batch's +-kz weights for k_kforce_f32
-    const bool half = sizeof(R) == 4 && MODE == 0;
+    constexpr bool half = MODE != 1;
     int k, nk, kb0 = 0;
     if (half) {
         if ((int)blockIdx.x >= S.n_batch_half) return;
@@ -1353,91 +1356,86 @@ __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
         if (blockIdx.x * 128 >= nk) return;
         k = blockIdx.x * 128 + threadIdx.x;
     }
-    __shared__ double red[4];
     __shared__ float2 wl[128];
     __shared__ float redf[4];
-    double e = 0.0;
-    float ef = 0.f;  // FP32 form: the k's energy term, summed over the block in FP32
+    float ef = 0.f;  // the k's energy term, summed over the block in FP32
+    const bool pack = half && a.wpk && a.kpk;
+    int code = -1;
+    double w = 0.0;
     if (k < nk) {
         const KVec kv = a.kvec[S.kvec_off + k];
-        const double w = 2.0 * kv.coef * ((half && kv.twin) ? 2.0 : 1.0);
-        double sr = 0.0, si = 0.0, dr = 0.0, di = 0.0;
-        if (sizeof(R) == 4 && MODE == 0) {
-            // FP32 form: the site chunks' compensated pairs (S, C), summed in chunk
-            // order with compensation in FP32; FP64 only for the energy
+        w = 2.0 * kv.coef * ((half && kv.twin) ? 2.0 : 1.0);
+        if (pack) code = a.kpk[S.kvec_off + k];
+    }
+    pdl_wait();  // the structure-factor partials of k_ksk
+    if (k < nk) {
+        if (half) {
+            // the site chunks' sums, in chunk order with compensation in FP32
             float xs = 0.f, xc = 0.f, ys = 0.f, yc = 0.f;
-            int sc = 0;
-            if (a.sk_sites) {  // k_ksk2's sums: no compensation beside them
+            if (MODE == 2) {  // no compensation beside them
                 const int n_sc = (S.n_sites + a.sk_sites - 1) / a.sk_sites;
                 const float2 *pp = reinterpret_cast<const float2 *>(a.skp) + J.sk_off + k;
-                for (int c0 = 0; c0 < n_sc; c0 += 8) {
-                    float2 p[8];
+                for (int c0 = 0; c0 < n_sc; c0 += 16) {
+                    float2 p[16];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        p[u] = c0 + u < n_sc ? pp[(size_t)(c0 + u) * a.total_k] : make_float2(0.f, 0.f);
+                    for (int u = 0; u < 16; ++u)
+                        if (c0 + u < n_sc) p[u] = pp[(size_t)(c0 + u) * a.total_k];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        kahan_add(xs, xc, p[u].x);
-                        kahan_add(ys, yc, p[u].y);
-                    }
+                    for (int u = 0; u < 16; ++u)
+                        if (c0 + u < n_sc) {
+                            kahan_add(xs, xc, p[u].x);
+                            kahan_add(ys, yc, p[u].y);
+                        }
                 }
-                sc = a.n_sc;
-            }
-            const float4 *pk = reinterpret_cast<const float4 *>(a.skp) + J.sk_off + k;
-            for (; sc + 4 <= a.n_sc; sc += 4) {  // four chunks' loads in flight, then their sums in order
-                float4 p[4];
+            } else {  // compensated pairs (S, C)
+                const float4 *pk = reinterpret_cast<const float4 *>(a.skp) + J.sk_off + k;
+                for (int c0 = 0; c0 < a.n_sc; c0 += 16) {
+                    float4 p[16];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) p[u] = pk[(size_t)(sc + u) * a.total_k];
+                    for (int u = 0; u < 16; ++u)
+                        if (c0 + u < a.n_sc) p[u] = pk[(size_t)(c0 + u) * a.total_k];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    kahan_add(xs, xc, p[u].x - p[u].z);
-                    kahan_add(ys, yc, p[u].y - p[u].w);
+                    for (int u = 0; u < 16; ++u)
+                        if (c0 + u < a.n_sc) {
+                            kahan_add(xs, xc, p[u].x - p[u].z);
+                            kahan_add(ys, yc, p[u].y - p[u].w);
+                        }
                 }
-            }
-            for (; sc < a.n_sc; ++sc) {
-                const float4 p = pk[(size_t)sc * a.total_k];
-                kahan_add(xs, xc, p.x - p.z);
-                kahan_add(ys, yc, p.y - p.w);
             }
             const float fr = xs - xc, fi = ys - yc, wf = (float)w;
             ef = 0.5f * wf * fmaf(fr, fr, fi * fi);
-            V2<R> v;
-            v.x = (R)(wf * fr);
-            v.y = (R)(wf * fi);
-            reinterpret_cast<V2<R> *>(a.wsk)[J.sk_off + k] = v;
-            wl[threadIdx.x] = make_float2(wf * fr, wf * fi);
+            const float2 v = make_float2(wf * fr, wf * fi);
+            reinterpret_cast<float2 *>(a.wsk)[J.sk_off + k] = v;
+            wl[threadIdx.x] = v;
         } else {
-        for (int sc = 0; sc < a.n_sc; ++sc) {
-            const size_t at = (size_t)sc * a.total_k + J.sk_off + k;
-            const double2 p = a.skp[at];
-            sr += p.x;
-            si += p.y;
-            if (MODE == 1) {
-                const double2 d = a.dskp[at];
-                dr += d.x;
-                di += d.y;
+            double sr = 0.0, si = 0.0, dr = 0.0, di = 0.0;
+            for (int c0 = 0; c0 < a.n_sc; c0 += 8) {
+                double2 p[8], d[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (c0 + u < a.n_sc) {
+                        const size_t at = (size_t)(c0 + u) * a.total_k + J.sk_off + k;
+                        p[u] = a.skp[at];
+                        d[u] = a.dskp[at];
+                    }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (c0 + u < a.n_sc) {
+                        sr += p[u].x;
+                        si += p[u].y;
+                        dr += d[u].x;
+                        di += d[u].y;
+                    }
             }
-        }
-        e = 0.5 * w * (sr * sr + si * si);
-        V2<R> *ws = reinterpret_cast<V2<R> *>(a.wsk) + J.sk_off;
-        V2<R> v;
-        v.x = (R)(w * sr);
-        v.y = (R)(w * si);
-        ws[k] = v;
-        if (MODE == 1) {
-            V2<R> *wd = reinterpret_cast<V2<R> *>(a.wdsk) + J.sk_off;
-            v.x = (R)(w * dr);
-            v.y = (R)(w * di);
-            wd[k] = v;
-        }
+            reinterpret_cast<float2 *>(a.wsk)[J.sk_off + k] = make_float2((float)(w * sr), (float)(w * si));
+            reinterpret_cast<float2 *>(a.wdsk)[J.sk_off + k] = make_float2((float)(w * dr), (float)(w * di));
         }
     }
-    if (half && a.wpk && a.kpk) {
+    if (pack) {
         // the batch's packed weights: slot of |kz| = az of a column holds, with
         // s = W(+az) + W(-az) and d = W(+az) - W(-az), P1 = (s.x, d.y, d.x, s.y) and
         // P2 = az (d.x, s.y, s.x, d.y) (az = 0: P1 = (W, 0, 0))
         __syncthreads();
-        const int code = k < nk ? a.kpk[S.kvec_off + k] : -1;
         if (code >= 0) {
             const int slot = code >> 8, az = code & 255;
             const float2 wp = wl[threadIdx.x];
@@ -1454,23 +1452,19 @@ __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
         }
     }
     if (half) {  // the block's FP32 partial, added to the FP64 energy
-        float t = warp_sum(ef);
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        if (lane == 0) redf[w] = t;
+        const float t = warp_sum(ef);
+        const int lane = threadIdx.x & 31, w4 = threadIdx.x >> 5;
+        if (lane == 0) redf[w4] = t;
         __syncthreads();
         if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], (double)(((redf[0] + redf[1]) + redf[2]) + redf[3]));
-    } else if (MODE == 0) {
-        const double t = block_sum(e, red);
-        if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
     }
 }
 
-// k_sk_reduce's grid: FP32 energy/force form one block per force batch, else per 128 k
-template <typename R, int MODE>
+// k_sk_reduce's grid: energy/force forms one block per force batch, else per 128 k
+template <int MODE>
 void launch_sk_reduce(const EvalArgs &a, cudaStream_t s) {
-    const bool half = sizeof(R) == 4 && MODE == 0;
-    const dim3 g(half ? a.max_batch : (a.max_kvec + 127) / 128, a.n_jobs);
-    launch_pdl(k_sk_reduce<R, MODE>, g, dim3(128), 0, s, a);
+    const dim3 g(MODE == 1 ? (a.max_kvec + 127) / 128 : a.max_batch, a.n_jobs);
+    launch_pdl(k_sk_reduce<MODE>, g, dim3(128), 0, s, a);
 }
 
 // ---- k_kforce: reciprocal-space site forces -------------------------------------
@@ -1488,7 +1482,7 @@ __global__ void __launch_bounds__(FT) k_kforce(EvalArgs a) {
     const int kc = blockIdx.y, jb = blockIdx.z;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
-    // FP32 energy/force form: the half set, whose weights k_sk_reduce<float, 0> writes
+    // FP32 energy/force form: the half set, whose weights k_sk_reduce writes
     const int nb = (sizeof(R) == 4 && MODE == 0) ? S.n_batch_half : S.n_batch, ns = S.n_sites, km1 = S.k_max + 1;
     if (blockIdx.x * FT >= ns) return;
     const int i = blockIdx.x * FT + threadIdx.x;
@@ -1643,7 +1637,7 @@ __global__ void __launch_bounds__(FT) k_kforce_f32(EvalArgs a) {
     const int kc = blockIdx.y, jb = blockIdx.z;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
-    // the half set, whose weights k_sk_reduce<float, 0> writes
+    // the half set, whose weights k_sk_reduce writes
     const int nb = S.n_batch_half, ns = S.n_sites, km1 = S.k_max + 1;
     if (blockIdx.x * NS >= ns) return;
     const int bt0 = chunk_lo(nb, kc, a.n_kc), bt1 = chunk_lo(nb, kc + 1, a.n_kc);
@@ -1914,13 +1908,15 @@ __global__ void __launch_bounds__(128) k_intra_f32(EvalArgs a) {
     if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
 }
 
-// CMB molecules per 128-thread block: first every thread sums site-force
-// components over the partial planes (one component a thread, plane order,
-// Kahan-compensated: the same sums as one thread per molecule would form, spread
-// over the block), then one thread per molecule adds the intramolecular and
-// Lennard-Jones terms and applies the M-site chain rule.
-constexpr int CMB = 32;
-__global__ void __launch_bounds__(128) k_combine_f32(EvalArgs a) {
+// CMB molecules a block: each thread sums one site-force component over the partial
+// planes (plane order, Kahan-compensated), then three threads a molecule, one a
+// dimension, add the intramolecular and Lennard-Jones terms and apply the M-site chain
+// rule. Bound by latency at every size: one wave of loads, since a thread has one
+// component and the second part's inputs are on their way during the first
+// (128 threads with up to three components in turn, then one thread a molecule: 9.2 us at
+// 512 waters, 32 beads and 9.8 at 216 waters, 1 bead, cold caches; now 6.5 and 8.6).
+constexpr int CMB = 32, CMT = 9 * CMB;
+__global__ void __launch_bounds__(CMT) k_combine_f32(EvalArgs a) {
     pdl_launch_dependents();  // the end step may load positions and masses meanwhile
     const int jb = blockIdx.y;
     const Job J = a.jobs[jb];
@@ -1929,82 +1925,54 @@ __global__ void __launch_bounds__(128) k_combine_f32(EvalArgs a) {
     const int m0 = blockIdx.x * CMB;
     if (m0 >= N) return;
     const int nm = min(CMB, N - m0);
-    const int m = m0 + threadIdx.x;
-    __shared__ double red[4];
-    __shared__ float fsum[CMB * 9];
-    {
+    __shared__ float fsum[CMT];
+    const int o = threadIdx.x, m = m0 + o / 3, d = o % 3;
+    const bool own = o < 3 * nm;
+    float fi[3] = {0.f, 0.f, 0.f}, fa[3] = {0.f, 0.f, 0.f};
+    double lj = 0.0;
+    if (own && J.mode == 0) {
+        const size_t mol = (size_t)J.site_off / 3 + m;
+        const float *in = a.intra + 18 * mol + d;  // k_intra_f32's
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            fi[k] = in[3 * k];
+            fa[k] = in[9 + 3 * k];
+        }
+        if (a.lj_plane) lj = (double)reinterpret_cast<const float *>(a.ljf + mol)[d];
+        else if (a.lj_half) lj = a.lj64[4 * mol + d];
+    }
+    if (o < 9 * nm) {
         const int np = a.n_rj + a.n_kc;
         const size_t stride = 3 * (size_t)a.total_sites;
-        const float *pl = reinterpret_cast<const float *>(a.part) + 3 * ((size_t)J.site_off + 3 * m0);
-        const long long *rf = a.real_fix ? a.rfix + 3 * ((size_t)J.site_off + 3 * m0) : nullptr;
-        for (int o = threadIdx.x; o < 9 * nm; o += blockDim.x) {
-            float sum = 0.f, comp = 0.f;
-            // the half-interaction real space's fixed-point sums (2^-40 units), loaded
-            // beside the planes
-            const long long rv = rf ? rf[o] : 0ll;
-            for (int p = 0; p < np; p += 16) {  // up to sixteen planes' loads in flight, then their sums in order
-                float v[16];
+        const float *pl = reinterpret_cast<const float *>(a.part) + 3 * ((size_t)J.site_off + 3 * m0) + o;
+        // the half-interaction real space's fixed-point sums (2^-40 units), loaded
+        // beside the planes
+        const long long rv = a.real_fix ? a.rfix[3 * ((size_t)J.site_off + 3 * m0) + o] : 0ll;
+        float sum = 0.f, comp = 0.f;
+        for (int p = 0; p < np; p += 16) {  // up to sixteen planes' loads in flight, then their sums in order
+            float v[16];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) v[u] = p + u < np ? pl[(p + u) * stride + o] : 0.f;
+            for (int u = 0; u < 16; ++u) v[u] = p + u < np ? pl[(p + u) * stride] : 0.f;
 #pragma unroll
-                for (int u = 0; u < 16; ++u)
-                    if (p + u < np) kahan_add(sum, comp, v[u]);
-            }
-            if (rf) kahan_add(sum, comp, (float)((double)rv * 9.094947017729282e-13));
-            fsum[o] = sum - comp;
+            for (int u = 0; u < 16; ++u)
+                if (p + u < np) kahan_add(sum, comp, v[u]);
         }
+        if (a.real_fix) kahan_add(sum, comp, (float)((double)rv * 9.094947017729282e-13));
+        fsum[o] = sum - comp;
     }
     __syncthreads();
-    double e = 0.0;
-    if ((int)threadIdx.x < nm) {
-        double *f = a.out + J.out_off + 9 * m;
-        float fs[9];
-        for (int k = 0; k < 9; ++k) fs[k] = fsum[9 * threadIdx.x + k];
-        float fa[9];
-        for (int k = 0; k < 9; ++k) fa[k] = 0.f;
-        if (J.mode == 0 && a.intra_plane) {  // computed beside the pair kernels (k_intra_f32)
-            const float *o = a.intra + 18 * ((size_t)J.site_off / 3 + m);
-            for (int k = 0; k < 9; ++k) {
-                fs[k] += o[k];
-                fa[k] = o[9 + k];
-            }
-        } else if (J.mode == 0) {  // the same sums in the same order as k_intra_f32's
-            float fi[9];
-            for (int k = 0; k < 9; ++k) fi[k] = 0.f;
-            e += intra_f32(a, J, S, m, fi, fa);
-            if (m == 0) e -= S.self_energy;
-            for (int k = 0; k < 9; ++k) fs[k] += fi[k];
-        }
-        // M-site chain rule (forces.cpp:613-619); the dense Lennard-Jones force of a
-        // forked evaluation joins the oxygen here
-        const float g = (float)a.c.gamma_vs, h = 0.5f * (1.0f - g);
-        double lj[3] = {0.0, 0.0, 0.0};
-        if (a.lj_plane && J.mode == 0) {
-            const float4 l = a.ljf[J.site_off / 3 + m];
-            lj[0] = (double)l.x;
-            lj[1] = (double)l.y;
-            lj[2] = (double)l.z;
-        } else if (a.lj_half && J.mode == 0) {
-            for (int d = 0; d < 3; ++d) lj[d] = a.lj64[4 * ((size_t)J.site_off / 3 + m) + d];
-        }
-        double *f2 = a.out_prop ? a.out_prop + J.out_off + 9 * m : nullptr;
-        for (int d = 0; d < 3; ++d) {
-            const double fo = (double)(fa[d] + g * fs[d]) + lj[d];
-            const double f1 = (double)(fa[3 + d] + fs[3 + d] + h * fs[d]);
-            const double f2v = (double)(fa[6 + d] + fs[6 + d] + h * fs[d]);
-            f[d] = fo;
-            f[3 + d] = f1;
-            f[6 + d] = f2v;
-            if (f2) {
-                f2[d] = fo;
-                f2[3 + d] = f1;
-                f2[6 + d] = f2v;
-            }
-        }
-    }
-    if (J.mode == 0 && !a.intra_plane) {
-        const double t = block_sum(e, red);
-        if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
+    if (!own) return;
+    const float *fs0 = fsum + 9 * (o / 3) + d;
+    const float fs[3] = {fs0[0] + fi[0], fs0[3] + fi[1], fs0[6] + fi[2]};
+    // M-site chain rule (forces.cpp:613-619); the Lennard-Jones force joins the oxygen here
+    const float g = (float)a.c.gamma_vs, h = 0.5f * (1.0f - g);
+    const double f[3] = {(double)(fa[0] + g * fs[0]) + lj, (double)(fa[1] + fs[1] + h * fs[0]),
+                         (double)(fa[2] + fs[2] + h * fs[0])};
+    const long long at = J.out_off + 9 * m + d;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a.out[at + 3 * k] = f[k];
+        if (a.out_prop) a.out_prop[at + 3 * k] = f[k];
     }
 }
 
@@ -2572,7 +2540,8 @@ void launch_recip(const EvalArgs &a, cudaStream_t s) {
     const int ns = 3 * a.max_mols, tiles = (ns + FT - 1) / FT, ktiles = (a.max_grp + KT - 1) / KT;
     if (ksk2_ok(a)) launch_ksk2(a, s);
     else launch_ksk<float, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
-    launch_sk_reduce<float, 0>(a, s);
+    if (a.sk_sites) launch_sk_reduce<2>(a, s);
+    else launch_sk_reduce<0>(a, s);
     launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
 }
 
@@ -2612,7 +2581,6 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             else if (list_ok(a)) launch_real_list(a, s);
             else k_real_f32<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
         };
-        if (a.intra) a.intra_plane = 1;
         const bool put = forks->put_lists;
         if (put) {
             real();
@@ -2620,13 +2588,13 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         }
         if (a.lj_full) launch_lj_dense(a, forks->side[1]);
         else k_lj<float, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
-        if (a.intra) k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
+        k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         cudaEventRecord(forks->join[1], forks->side[1]);
         if (!put) real();
         cudaStreamWaitEvent(s, forks->join[0], 0);
         cudaStreamWaitEvent(s, forks->join[1], 0);
-        k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
-        if (n) *n += (a.intra_plane ? 8 : 7) + (list_ok(a) ? 2 : 0);
+        k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), CMT, 0, s>>>(a);
+        if (n) *n += 8 + (list_ok(a) ? 2 : 0);
         return;
     }
     // the derivative: real space beside the reciprocal chain
@@ -2637,12 +2605,12 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     cudaEventRecord(forks->fork, s);
     cudaStreamWaitEvent(rs, forks->fork, 0);
     launch_ksk<float, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
-    launch_sk_reduce<float, 1>(a, rs);
+    launch_sk_reduce<1>(a, rs);
     k_kforce<float, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<float>(a.max_kmax), rs>>>(a);
     k_real<float, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
     cudaEventRecord(forks->join[0], rs);
     cudaStreamWaitEvent(s, forks->join[0], 0);
-    k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
+    k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), CMT, 0, s>>>(a);
     if (n) *n += 6;
 }
 
@@ -2734,13 +2702,15 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         else if (mixed) launch_ksk<float, 0>(a, gk, s);
         else launch_ksk64(a, s);
     } else if (n == "sk_reduce") {
-        if (mixed) launch_sk_reduce<float, 0>(a, s);
+        if (mixed && a.sk_sites) launch_sk_reduce<2>(a, s);
+        else if (mixed) launch_sk_reduce<0>(a, s);
         else launch_sk_reduce64(a, s);
     } else if (n == "kforce") {
         if (mixed) launch_kforce_f32(a, gf, s);
         else launch_kforce64(a, s);
     } else if (n == "combine") {
-        if (mixed) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), 128, 0, s>>>(a);
+        a.lj_plane = 1;
+        if (mixed) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), CMT, 0, s>>>(a);
         else launch_combine64(a, s);
     } else if (n == "lj") {
         if (mixed) {
