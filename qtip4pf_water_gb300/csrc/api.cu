@@ -228,6 +228,8 @@ struct qtg_ctx {
     int4 *sites_fix = nullptr;  // fixed-point site fractions per slot (half-interaction real space)
     long long *rfix = nullptr;  // fixed-point real-space site forces per slot (half-interaction real space)
     double *real64_tab = nullptr;  // FP64: the real-space pair-function table
+    long long *real64_int = nullptr, *real64_sys = nullptr;  // its fixed-point form; constants per system
+    float4 *sites32 = nullptr;     // FP64: wrapped FP32 charge sites
     // real-space pair list (mixed contexts with beads beyond the half-interaction
     // kernel in boxes with r_c + 2 RL_SPREAD <= L/2): rl_ok marks the context
     // eligible, rl_form 0 runs the real space over the list there, 1 over all pairs
@@ -404,6 +406,9 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.sites_fix = c->sites_fix;
     a.rfix = c->rfix;
     a.real64_tab = c->real64_tab;
+    a.real64_int = c->real64_int;
+    a.real64_sys = c->real64_sys;
+    a.sites32 = c->sites32;
     a.opos = c->opos;
     a.opos32 = c->opos32;
     a.lj64 = c->lj64;
@@ -1378,7 +1383,12 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     AL(ctx->intra, 6 * ctx->total_sites);
     AL(ctx->sites_fix, ctx->total_sites);
     AL(ctx->rfix, (ctx->mixed ? 3 : 6) * ctx->total_sites);
-    if (!ctx->mixed) AL(ctx->real64_tab, (size_t)R64_INTERVALS * 16);
+    if (!ctx->mixed) {
+        AL(ctx->real64_tab, (size_t)R64_INTERVALS * 16);
+        AL(ctx->real64_int, (size_t)RI_OCT * 64 * 12);
+        AL(ctx->real64_sys, 4 * (size_t)n_systems);
+        AL(ctx->sites32, ctx->total_sites);
+    }
     {
         // real-space pair list: rows hold the molecules whose M sites lie within
         // r_c + RL_SKIN + 2 RL_SPREAD (the prefilter radius of k_rlist_rows), at the
@@ -1465,7 +1475,16 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
             real64_table(t.data());
             return t;
         }();
+        static const std::vector<long long> itab = [] {
+            std::vector<long long> t((size_t)RI_OCT * 64 * 12);
+            real64_int_table(t.data());
+            return t;
+        }();
+        std::vector<long long> sc(4 * (size_t)n_systems);
+        for (int k = 0; k < n_systems; ++k) real64_system(ctx->sys_h[k], sc.data() + 4 * k);
         cp(ctx->real64_tab, tab.data(), sizeof(double) * tab.size());
+        cp(ctx->real64_int, itab.data(), sizeof(long long) * itab.size());
+        cp(ctx->real64_sys, sc.data(), sizeof(long long) * sc.size());
     }
     cp(ctx->charge, chg_all.data(), sizeof(double) * chg_all.size());
     cp(ctx->mass, mass_all.data(), sizeof(double) * mass_all.size());
@@ -1534,7 +1553,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->kpair, ctx->opos32, ctx->lj64, ctx->intra64};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->real64_int, ctx->real64_sys, ctx->sites32, ctx->kpair, ctx->opos32, ctx->lj64, ctx->intra64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);

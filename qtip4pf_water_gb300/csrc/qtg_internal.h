@@ -52,6 +52,7 @@ struct SysDev {
     long long mass_off; // doubles: [9N] in mass
     double box[3], inv_box[3];
     double kappa, rc_sq, ewald_pref, k_pref, self_energy;
+    double q_top, inv_q_top;  // k_real64's unit of charge, a little above the largest |charge|, and its inverse
     double q_scale, inv_q_scale;  // the power of two at or above the largest |charge|, and its inverse
     double r_cut_sq, r_skin_sq, skin_margin;
     double beta, beta_n, omega_psq, dt, halfdt, eps_sc, c1_centroid, inv_sqrt_beta_n;
@@ -80,6 +81,8 @@ inline void set_charge_scale(SysDev &S, const double *charge, int n) {
     while (top > 0.0 && 0.5 * s >= top) s *= 0.5;
     S.q_scale = s;
     S.inv_q_scale = 1.0 / s;
+    S.q_top = top > 0.0 ? top * (1.0 + 1e-6) : 1.0;
+    S.inv_q_top = 1.0 / S.q_top;
 }
 
 // The FP32 constants above, from the FP64 ones (host).
@@ -491,6 +494,8 @@ constexpr int MAX_SC = 32;   // structure-factor site chunks
 constexpr int MAX_SC2 = 2 * MAX_SC;  // the same of k_ksk2, whose partial sums are half as large
 constexpr int R64_LO = -16, R64_HI = 5;  // octaves of (kappa r)^2 in the FP64 pair-function table
 constexpr int R64_INTERVALS = (R64_HI - R64_LO) * 64;
+// the same of its fixed-point form, and the range of the high word of (kappa r)^2 2^56
+constexpr int RI_LO = -3, RI_OCT = 8, RI_BOT = 1 << (56 + RI_LO - 32), RI_TOP = 1 << (56 + RI_LO + RI_OCT - 32);
 constexpr int HALF_MAX_TILES = 64;  // half-interaction real space: beads of at most 64 x 32 sites
 constexpr int HALF_MAX_CH = 8;      // its stationary-side chunks, one site a lane
 constexpr int MAX_PART = MAX_RJ + MAX_KC + 1;  // partial site-force planes
@@ -554,6 +559,8 @@ struct EvalArgs {
     long long *rfix;
     int real_fix;
     const double *real64_tab;  // FP64: the pair-function table (real64_table)
+    const long long *real64_int, *real64_sys;  // FP64: its fixed-point form; four constants a system (real64_system)
+    float4 *sites32;       // FP64: wrapped FP32 charge sites and their molecule, per slot (null: not wanted)
     long long total_sites; // sites summed over all slots (plane stride of part)
     double2 *skp;          // partial S(k) [MAX_SC][total_k] (k_ksk2: float2 [MAX_SC2][total_k])
     int sk_sites;          // nonzero: skp holds k_ksk2's plain FP32 sums, of this many sites each
@@ -611,6 +618,17 @@ void launch_ksk2(const EvalArgs &a, cudaStream_t s);
 
 // real64.cu: real space of the FP64 form, and its pair-function table (R64_INTERVALS x 16 doubles, host)
 void real64_table(double *tab);
+void real64_int_table(long long *tab);  // RI_OCT * 64 x 12
+void real64_system(const SysDev &S, long long *out);  // four constants
+// kappa x in units of 2^-56 (modulo 2^64), correctly rounded but for a unit
+__host__ __device__ inline long long kappa_fix(double kappa, double x) {
+    const double h = kappa * x, l = fma(kappa, x, -h), i = floor(h), two56 = 72057594037927936.0;
+#ifdef __CUDA_ARCH__
+    return (long long)((unsigned long long)__double2ll_rn(i) << 56) + __double2ll_rn((h - i) * two56) + __double2ll_rn(l * two56);
+#else
+    return (long long)((unsigned long long)llrint(i) << 56) + llrint((h - i) * two56) + llrint(l * two56);
+#endif
+}
 void init_real64_attributes();
 void launch_real64(const EvalArgs &a, cudaStream_t s);
 

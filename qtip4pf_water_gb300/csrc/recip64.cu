@@ -50,7 +50,7 @@ __device__ __forceinline__ void column_factor(const int4 &x, const int4 &y, int 
 
 // ---- k_prep64 -----------------------------------------------------------------------
 // One thread per (site, dimension), blocks dimension-major as k_prep_f32: charge site
-// (M, H1, H2) wrapped into the box, wrapped oxygen, zeroed sums, and the site's row of
+// (M, H1, H2) wrapped into the box in k_real64's fixed point, wrapped oxygen, zeroed sums, and the site's row of
 // phases exp(i 2 pi m s_d), m = 0 .. k_max: powers 1, 2 and the multiples of four from
 // arguments reduced in FP64, the others as products of those in limbs (whose rounding is
 // below the FP64 sines'). The x row carries the charge over q_scale.
@@ -78,10 +78,19 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
     }
     const double t = x * S.inv_box[d], frac = t - floor(t);
     const double chg = d == 0 ? a.charge[S.chg_off + s] : 0.0;
-    double *sv = reinterpret_cast<double *>(a.sites) + 4 * ((size_t)J.site_off + s);
-    sv[d] = frac * S.box[d];
-    if (d == 0) sv[3] = chg;
-    if (a.rfix) {  // k_real64 adds into it (reciprocal space alone may have none)
+    if (a.sites32) {  // k_real64's form of the site (reciprocal space alone may have none)
+        // wrapped as frac is, with one rounding (while the quotient is exact enough for it)
+        const double w = fabs(t) < 1e9 ? fma(-floor(t), S.box[d], x) : frac * S.box[d];
+        i64 *sv = reinterpret_cast<i64 *>(a.sites) + 4 * ((size_t)J.site_off + s);
+        sv[d] = kappa_fix(S.kappa, w);
+        float *sf = reinterpret_cast<float *>(a.sites32 + (size_t)J.site_off + s);
+        sf[d] = (float)w;
+        if (d == 0) {
+            const double h = chg * S.inv_q_top, l = fma(-h, S.q_top, chg) * S.inv_q_top, two62 = 4611686018427387904.0;
+            sv[3] = __double2ll_rn(h * two62) + __double2ll_rn(l * two62);
+            sf[3] = __int_as_float(mol);
+        }
+        // its sums start from nothing
         i64 *rf = a.rfix + 6 * ((size_t)J.site_off + s) + 2 * d;
         rf[0] = rf[1] = 0;
     }

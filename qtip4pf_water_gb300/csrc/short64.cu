@@ -245,9 +245,11 @@ __global__ void __launch_bounds__(96) k_combine64(EvalArgs a) {
         const size_t at = 3 * ((size_t)J.site_off + 3 * m) + d;
         for (int p = 0; p < a.n_kc; ++p)
             for (int s = 0; s < 3; ++s) fs[s] += a.part[3 * (size_t)p * a.total_sites + at + 3 * s];
+        // units of 2^-56 q_top^2 kappa^2
+        const double unit = S.q_top * S.kappa * (S.q_top * S.kappa);
         for (int s = 0; s < 3; ++s) {
             const long long *rf = a.rfix + 2 * (at + 3 * s);
-            fs[s] += fma((double)rf[0], 0.00390625, (double)rf[1] * 8.673617379884035e-19);
+            fs[s] += unit * fma((double)rf[0], 5.960464477539063e-08, (double)rf[1] * 1.3877787807814457e-17);
         }
     }
     const size_t mol = (size_t)J.site_off / 3 + m;

@@ -43,3 +43,18 @@ def test_near_contact_pair(gpu_lib):
     ref, got, e_ref, e_got = _forces(q, 27, 1, st.box_bohr, pos, 1e-6)
     assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
     assert abs(e_got - e_ref) < 1e-9 * abs(e_ref)
+
+
+# Ewald tolerances whose pairs are beyond the fixed-point form (every pair in FP64), and a
+# pair in each of its octaves' neighbours: H...H distances around (kappa r)^2 = 2^-3
+@pytest.mark.parametrize("eps,gap", [(1e-18, None), (1e-6, 0.98), (1e-6, 1.02)])
+def test_edges_of_the_fixed_point_form(gpu_lib, eps, gap):
+    q = gpu_lib
+    st = q.seeded_start(27, 1, 298.0, seed=6)
+    pos = np.ascontiguousarray(st.q)
+    if gap is not None:
+        kappa = q.System.create(27, 1, st.box_bohr, precision=q.FP64, propagator=q.TROTTER, eps_ewald=eps).info.kappa
+        pos[0, 9 + 3: 9 + 6] = pos[0, 3:6] + gap * 2.0 ** -1.5 / kappa * np.array([0.6, 0.0, 0.8])
+    ref, got, e_ref, e_got = _forces(q, 27, 1, st.box_bohr, pos, eps)
+    assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
+    assert abs(e_got - e_ref) < 1e-9 * max(1.0, abs(e_ref))
