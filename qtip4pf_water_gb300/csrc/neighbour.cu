@@ -50,13 +50,17 @@ __device__ __forceinline__ bool pair_exact(const double *qi, const double *qj, c
     return r2 < S.r_skin_sq;
 }
 
-__device__ __forceinline__ bool pair_in(const float4 a, const float4 b, const double *qi, const double *qj,
-                                        const SysDev &S, float rs2) {
+__device__ __forceinline__ float image_r2(const float4 a, const float4 b, const SysDev &S) {
     float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     dx -= S.boxf[0] * rintf(dx * S.inv_boxf[0]);
     dy -= S.boxf[1] * rintf(dy * S.inv_boxf[1]);
     dz -= S.boxf[2] * rintf(dz * S.inv_boxf[2]);
-    float r2 = dx * dx + dy * dy + dz * dz;
+    return dx * dx + dy * dy + dz * dz;
+}
+
+__device__ __forceinline__ bool pair_in(const float4 a, const float4 b, const double *qi, const double *qj,
+                                        const SysDev &S, float rs2) {
+    const float r2 = image_r2(a, b, S);
     if (fabsf(r2 - rs2) > kBand * rs2) return r2 < rs2;
     return pair_exact(qi, qj, S);
 }
@@ -206,12 +210,34 @@ __device__ void row_bitmap(const ListArgs &a, const SysDev &S, int bead, int i, 
     };
     if (S.lc_cells == 0) {
         // every molecule in order: the 32 lanes test the 32 molecules of one bitmap
-        // word, which a ballot assembles (no atomics on a shared word)
-        for (int j0 = 0; j0 < N; j0 += 32) {
-            const int j = j0 + lane;
-            const bool in = j < N && j != i && pair_in(pi, wp[j], qb + 9 * i, qb + 9 * j, S, rs2);
-            const unsigned word = __ballot_sync(0xffffffffu, in);
-            if (lane == 0) bm[j0 >> 5] = word;
+        // word, which a ballot assembles (no atomics on a shared word). Four words at a
+        // time, as a row is a chain of loads and tests (one at a time: 205 us for the
+        // lists of 512 waters, 32 beads, 157 so)
+        for (int j0 = 0; j0 < N; j0 += 128) {
+            float4 p[4];
+            float r2[4];
+            bool in[4], near = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) p[u] = j0 + 32 * u + lane < N ? wp[j0 + 32 * u + lane] : pi;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                r2[u] = image_r2(pi, p[u], S);
+                in[u] = r2[u] < rs2;
+                near |= fabsf(r2[u] - rs2) <= kBand * rs2;
+            }
+            if (near)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = j0 + 32 * u + lane;
+                    if (j < N && fabsf(r2[u] - rs2) <= kBand * rs2) in[u] = pair_exact(qb + 9 * i, qb + 9 * j, S);
+                }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = j0 + 32 * u + lane;
+                const unsigned word = __ballot_sync(0xffffffffu, in[u] && j < N && j != i);
+                if (lane == 0 && j0 + 32 * u < N) bm[(j0 >> 5) + u] = word;
+            }
         }
     } else {
         const int *cs = a.cell_start + S.lc_off + (size_t)bead * (S.lc_cells + 1);
@@ -380,7 +406,9 @@ void launch_skin_rebuild(const ListArgs &a, cudaStream_t s, unsigned long long *
     // one block an SM, or one per 16 items of a rebuild of every bead when that is
     // more (at most eight an SM): in a step without a rebuild the blocks only read the count and exit,
     // and a wide grid holds the thread slots of the force kernels running beside
-    // it (1216 blocks cost the 512-water P = 32 step ~7 us)
+    // it (1216 blocks cost the 512-water P = 32 step ~7 us; sixteen warps a block instead of
+    // eight cost it 1.4 us and build its lists in 107 us instead of 157, once in some
+    // thousand steps)
     const int grid = (int)std::min<long long>(items, std::max<long long>(152LL, std::min<long long>(items / 16, 152LL * 8)));
     const size_t bm = (size_t)ROWS * W * sizeof(unsigned);
     k_list_rows<false><<<grid, 32 * ROWS, bm, s>>>(a, row_blocks);
