@@ -28,6 +28,7 @@
 
 #include <algorithm>
 
+#include "fixed62.h"
 #include "qtg_internal.h"
 
 namespace qtg {
@@ -110,7 +111,6 @@ void real64_system(const SysDev &S, long long *out) {
 
 namespace {
 
-typedef long long i64;
 constexpr int RROWS = 16;          // sites a warp holds
 constexpr int RW = 32 / RROWS;     // warps per block: the parts of a tile of 32 sites
 constexpr int RLANES = 32 / RROWS;  // lanes that sum a held site's pairs
@@ -128,23 +128,6 @@ struct RWarp {
     unsigned short code[RCAP];     // row, visited site and image of every packed pair
 };
 
-__device__ __forceinline__ i64 madw(int a, int b, i64 c) { return (i64)a * b + c; }
-// v in limbs: h 2^31 + l, 0 <= l < 2^31; |v| < 2^62
-struct Limbs {
-    int h, l;
-};
-__device__ __forceinline__ Limbs limbs(i64 v) { return Limbs{(int)(v >> 31), (int)v & 0x7fffffff}; }
-// x y 2^-62 to within a unit: the product of the low limbs (a quarter unit in the mean) is
-// left out and the floor takes half a unit, which the added constant makes up
-__device__ __forceinline__ i64 mul62(const Limbs &x, const Limbs &y) {
-    return (i64)x.h * y.h + (madw(x.h, y.l, madw(x.l, y.h, 0x60000000ll)) >> 31);
-}
-// the same with the low limbs' product, for a factor that many pairs share
-__device__ __forceinline__ i64 mul62x(const Limbs &x, const Limbs &y) {
-    return (i64)x.h * y.h + (madw(x.h, y.l, madw(x.l, y.h, ((i64)x.l * y.l >> 31) + 0x40000000ll)) >> 31);
-}
-__device__ __forceinline__ i64 sqr62(const Limbs &x) { return (i64)x.h * x.h + (madw(x.h, x.l, 0x30000000ll) >> 30); }
-
 // one of the two functions: t = tau in units of 2^-62
 __device__ __forceinline__ i64 horner(const longlong2 &c01, const longlong2 &c23, const int4 &c47, const Limbs &t, int t32) {
     int p = c47.w;
@@ -152,9 +135,9 @@ __device__ __forceinline__ i64 horner(const longlong2 &c01, const longlong2 &c23
     p = c47.y + (int)(((i64)p * t32) >> 32);
     p = c47.x + (int)(((i64)p * t32) >> 32);
     i64 v = c23.y + (((i64)p * t32) >> 23);
-    v = c23.x + mul62(limbs(v), t);
-    v = c01.y + mul62(limbs(v), t);
-    return c01.x + mul62(limbs(v), t);
+    v = c23.x + mul62(split62(v), t);
+    v = c01.y + mul62(split62(v), t);
+    return c01.x + mul62(split62(v), t);
 }
 
 // G and W in FP64: the FP64 table, or the functions themselves outside it
@@ -292,7 +275,7 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
             const i64 y0 = p.y[0] - s.y[0] - image[0][img & 3], y1 = p.y[1] - s.y[1] - image[1][(img >> 2) & 3],
                       y2 = p.y[2] - s.y[2] - image[2][(img >> 4) & 3];
             // u in units of 2^-56; a fixed-point pair has u in [2^RI_LO, 2^(RI_LO + RI_OCT))
-            const i64 u = sqr62(limbs(y0 * 8)) + sqr62(limbs(y1 * 8)) + sqr62(limbs(y2 * 8));
+            const i64 u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
             i64 fx = 0, fy = 0, fz = 0;
             if (u < uc && (unsigned)((int)(u >> 32) - RI_BOT) < (unsigned)(RI_TOP - RI_BOT)) {
                 const int z = __clz((int)(u >> 32));
@@ -302,17 +285,17 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
                 const longlong2 w01 = __ldg(q), w23 = __ldg(q + 1), g01 = __ldg(q + 3), g23 = __ldg(q + 4);
                 const int4 w47 = __ldg(reinterpret_cast<const int4 *>(q + 2)), g47 = __ldg(reinterpret_cast<const int4 *>(q + 5));
                 const i64 t = (i64)((unsigned long long)(n << 7) >> 2) - (1ll << 61);
-                const Limbs tl = limbs(t);
+                const Limbs tl = split62(t);
                 const int t32 = (int)(t >> 30);
-                const Limbs qq = limbs(mul62x(limbs(p.q), limbs(s.q)));
-                const i64 eg = mul62x(qq, limbs(horner(g01, g23, g47, tl, t32)));
+                const Limbs qq = split62(mul62x(split62(p.q), split62(s.q)));
+                const i64 eg = mul62x(qq, split62(horner(g01, g23, g47, tl, t32)));
                 he += eg >> 32;
                 le += (unsigned)eg;
-                const Limbs w = limbs(mul62x(qq, limbs(horner(w01, w23, w47, tl, t32))));
+                const Limbs w = split62(mul62x(qq, split62(horner(w01, w23, w47, tl, t32))));
                 const int up = oct == 0 ? 5 : 3;  // the lowest octave's W has two bits less
-                fx = mul62(w, limbs(y0 << up));
-                fy = mul62(w, limbs(y1 << up));
-                fz = mul62(w, limbs(y2 << up));
+                fx = mul62(w, split62(y0 << up));
+                fy = mul62(w, split62(y1 << up));
+                fz = mul62(w, split62(y2 << up));
             } else if (u < uc || uc < 0) {
                 i64 *rf = a.rfix + 6 * (size_t)J.site_off;
                 e += slow_pair(a, S, y0, y1, y2, p.q, s.q, rf + 6 * (i0 + ((c >> 5) & 15)),
