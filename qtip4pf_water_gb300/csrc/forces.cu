@@ -2617,13 +2617,16 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
 // Chunk counts of the FP64 reciprocal space: whole 32-site shared-memory chunks of the
 // structure factors, and blocks enough to fill the GPU; where these leave half of it idle,
 // half chunks (64 waters, 1 bead: 18.6 us with whole ones, 14.4 with halves; 216 waters, 8
-// beads, whose chunks fill it, a Suzuki-Chin call 414 and 425 us).
+// beads, whose chunks fill it, a Suzuki-Chin call 414 and 425 us). The k-force takes more
+// blocks than fit at once: its unit is a batch of columns, and few chunks of some three
+// batches end unevenly (216 waters, 32 beads: 5 chunks 131 us, 7 120, 13 109; 512 waters: 3
+// chunks 337 us, 8 315).
 void set_chunks64(EvalArgs &a) {
     const int ns = 3 * a.max_mols, tiles = (ns + 127) / 128, ktiles = (a.max_grp + KT - 1) / KT;
     const long long base = (long long)ktiles * a.n_jobs;
     const int sites = base * ((ns + CH - 1) / CH) <= 76 ? CH / 2 : CH;
     a.n_sc = chunks_or(a.tune_sc, base, std::min(MAX_SC, (ns + sites - 1) / sites), 6);
-    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 6);
+    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 16);
 }
 
 // An FP64 evaluation: real space | reciprocal chain | short-range terms on parallel
