@@ -1329,10 +1329,10 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
 // Sum of the structure-factor partials of every k in chunk order, the reciprocal-space
 // energy sum_k c_k |S(k)|^2, and the force weights 2 c_k S(k) (MODE 1, the derivative:
 // and 2 c_k dS(k)) for the k-force. One thread per k. Bound by latency: what does not
-// depend on k_ksk is read before the wait for it, and the partials come sixteen (MODE 1:
-// eight) loads at a time (four, resp. one, took 9.9 us at 216 waters, 1 bead against 7.4,
+// depend on k_ksk is read before the wait for it, and the partials come sixteen (MODEs 1
+// and 2, whose batches are larger: eight) loads at a time (four, resp. one, took 9.9 us at 216 waters, 1 bead against 7.4,
 // resp. 18 us for the derivative of 512 waters, 16 beads).
-// MODE 0: k_ksk's partials; MODE 2: k_ksk2's, which need fewer registers.
+// MODE 0: k_ksk's partials; MODE 2: k_ksk2's (sixteen loads: 48 uneven replicas 57 us, eight: 42).
 template <int MODE>
 __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
     pdl_launch_dependents();  // the k-force may start its staging of the phase rows
@@ -1375,13 +1375,13 @@ __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
             if (MODE == 2) {  // no compensation beside them
                 const int n_sc = (S.n_sites + a.sk_sites - 1) / a.sk_sites;
                 const float2 *pp = reinterpret_cast<const float2 *>(a.skp) + J.sk_off + k;
-                for (int c0 = 0; c0 < n_sc; c0 += 16) {
-                    float2 p[16];
+                for (int c0 = 0; c0 < n_sc; c0 += 8) {
+                    float2 p[8];
 #pragma unroll
-                    for (int u = 0; u < 16; ++u)
+                    for (int u = 0; u < 8; ++u)
                         if (c0 + u < n_sc) p[u] = pp[(size_t)(c0 + u) * a.total_k];
 #pragma unroll
-                    for (int u = 0; u < 16; ++u)
+                    for (int u = 0; u < 8; ++u)
                         if (c0 + u < n_sc) {
                             kahan_add(xs, xc, p[u].x);
                             kahan_add(ys, yc, p[u].y);
