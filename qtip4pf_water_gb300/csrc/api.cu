@@ -211,6 +211,10 @@ struct Table {  // a device job table plus its host copy
 
 }  // namespace
 
+// Parts of a step (step_parts): at most, and molecule-beads of a step and of each part
+constexpr int MAX_PARTS = 4;
+constexpr long long PARTS_MIN = 32000, PART_MIN = 2048;
+
 struct qtg_ctx {
     int device = 0;
     int precision = QTG_FP64;
@@ -223,6 +227,13 @@ struct qtg_ctx {
     cudaEvent_t sur_fork = nullptr, sur_join = nullptr;
     cudaEvent_t ev_fork[2] = {nullptr, nullptr}, ev_join = nullptr;
     Forks forks{};            // branches of a mixed force evaluation (real | k-space | LJ)
+    // parts of a step's systems after the first (see enqueue_parts): stream, forks and events
+    struct Part {
+        cudaStream_t stream = nullptr;
+        Forks forks{};
+        cudaEvent_t join = nullptr;
+    } part_of[MAX_PARTS - 1];
+    cudaEvent_t ring_done[MAX_PARTS] = {};
     float4 *ljf = nullptr;    // dense LJ oxygen forces per molecule and slot
     float *intra = nullptr;   // intramolecular forces, 18 floats per molecule and slot
     int4 *sites_fix = nullptr;  // fixed-point site fractions per slot (half-interaction real space)
@@ -709,7 +720,106 @@ bool rebuild_beside_forces(const qtg_ctx *c, int sys) {
     return true;
 }
 
+// The parts a step of all systems goes in (first systems; a closing entry): up to four of
+// about the same pair work for second-order systems of the mixed form with some 32,000
+// molecule-beads and more, each enough for the kernels of large batches (which lay their
+// partial sums out their own way in shared scratch); else one.
+std::vector<int> step_parts(const qtg_ctx *c) {
+    std::vector<int> lo(1, 0);
+    const auto molecules = [&](int s) { return (long long)c->sys_h[s].n_beads * c->sys_h[s].n_mols; };
+    const auto load = [&](int s) { return (double)molecules(s) * c->sys_h[s].n_mols; };
+    long long total = 0, here = 0, least = PART_MIN;
+    double work = 0.0, sum = 0.0;
+    for (int s = 0; s < c->n_sys; ++s) {
+        total += molecules(s);
+        work += load(s);
+    }
+    const bool can = c->n_sys > 1 && total >= PARTS_MIN && rebuild_beside_forces(c, -1) && c->surrogates.empty() && !lj_list_ok(c) &&
+                     !c->rl_ok;
+    for (int s = 0; can && s < c->n_sys; ++s) {
+        if (s > lo.back() && (int)lo.size() < MAX_PARTS && sum >= work * (double)lo.size() / MAX_PARTS) {
+            least = std::min(least, here);
+            here = 0;
+            lo.push_back(s);
+        }
+        sum += load(s);
+        here += molecules(s);
+    }
+    if (can && std::min(least, here) < PART_MIN) lo.resize(1);
+    lo.push_back(c->n_sys);
+    return lo;
+}
+
+// The step's ring and end-step kernels are bound by FP64 instructions, the force kernels
+// by FP32 ones. In parts of the systems on streams of their own, one ring update behind the
+// other, a part's forces run beside the next one's ring update and the one before's end
+// step. 48 uneven replicas (277,000 molecule-beads) 2409 us a step in one part, 2350 in two,
+// 2336 in four; 12 (59,000) 583, 571, 529; 4 of 216 waters, 8 beads (6,900), which fill the
+// GPU only together, 91 and 115 in two.
+void enqueue_parts(qtg_ctx *c, const std::vector<int> &lo, int nvt, bool pile_g) {
+    const int parts = (int)lo.size() - 1;
+    cudaStream_t main = c->stream;
+    const auto columns = [&](RingArgs &r, int h) {
+        const int a = lo[h], z = lo[h + 1] - 1;
+        r.work = c->colwork + c->cw_begin[a];
+        r.n_work = c->cw_begin[z] + c->cw_count[z] - c->cw_begin[a];
+    };
+    for (int h = 0; h < parts; ++h) {
+        cudaStream_t st = h ? c->part_of[h - 1].stream : main;
+        RingArgs r = ring_args(c, -1, RF_KICK | RF_FWD | RF_CAYLEY | RF_BACK | RF_DISP | (nvt ? RF_THERMO : 0));
+        columns(r, h);
+        // (its partial sums are laid out otherwise than an end step's, which may run beside it)
+        r.cw_part = c->cw_part + 4 * (size_t)c->n_colwork;
+        r.pile_g = pile_g ? 1 : 0;
+        r.n_draw = lo[h + 1] - lo[h];  // (as in enqueue_step)
+        r.draw_sys0 = lo[h];
+        if (h) cudaStreamWaitEvent(st, c->ring_done[h - 1], 0);
+        launch_ring(r, st, &c->launches);
+        cudaEventRecord(c->ring_done[h], st);
+    }
+    // every part's lists, beside the forces
+    cudaStreamWaitEvent(c->side_stream, c->ring_done[parts - 1], 0);
+    launch_skin_rebuild(list_args(c, 0, (int)c->base.h.size(), 0), c->side_stream, &c->launches);
+    cudaEventRecord(c->ev_join, c->side_stream);
+    for (int h = 0; h < parts; ++h) {
+        const SysDev &first = c->sys_h[lo[h]], &last = c->sys_h[lo[h + 1] - 1];
+        EvalArgs base = eval_args(c, c->base.d + first.job_base, last.job_base + last.n_beads - first.job_base, c->q,
+                                  c->fphys, 0, 0);
+        base.lj_full = 1;
+        base.out_prop = c->f;
+        if (h) {
+            std::swap(c->forks, c->part_of[h - 1].forks);
+            c->stream = c->part_of[h - 1].stream;
+        }
+        launch_eval(c, base);
+        FinalizeArgs fa = fin_args(c, -1, 1, 1);
+        fa.pile_g = pile_g ? 1 : 0;
+        fa.pre_drawn = 1;
+        RingArgs e = ring_args(c, -1, 0);
+        columns(e, h);
+        cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+        e.kick = 1;
+        e.fuse_fin = 1;  // the last system of all parts to finish advances the step
+        e.fin = fa;
+        e.fin.ticket = c->fin_ticket;
+        launch_end_step(e, c->stream, &c->launches);
+        if (h) {
+            cudaEventRecord(c->part_of[h - 1].join, c->stream);
+            std::swap(c->forks, c->part_of[h - 1].forks);
+            c->stream = main;
+        }
+    }
+    for (int h = 1; h < parts; ++h) cudaStreamWaitEvent(main, c->part_of[h - 1].join, 0);
+}
+
 void enqueue_step(qtg_ctx *c, int sys, int nvt, int ext_noise, bool pile_g) {
+    if (sys < 0 && !ext_noise) {
+        const std::vector<int> lo = step_parts(c);
+        if (lo.size() > 2) {
+            enqueue_parts(c, lo, nvt, pile_g);
+            return;
+        }
+    }
     RingArgs r = ring_args(c, sys, RF_KICK | RF_FWD | RF_CAYLEY | RF_BACK | RF_DISP | (nvt ? RF_THERMO : 0));
     r.noise = ext_noise ? c->noise : nullptr;
     r.pile_g = pile_g ? 1 : 0;
@@ -1313,6 +1423,15 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->sur_join, cudaEventDisableTiming);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ctx->ev_fork[k], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
+    for (int h = 0; h < MAX_PARTS && n_systems > 1 && ctx->mixed; ++h) {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ring_done[h], cudaEventDisableTiming);
+        if (h == 0) continue;
+        auto &p = ctx->part_of[h - 1];
+        for (cudaStream_t *st : {&p.stream, &p.forks.side[0], &p.forks.side[1]})
+            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+        for (cudaEvent_t *ev : {&p.join, &p.forks.fork, &p.forks.join[0], &p.forks.join[1]})
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    }
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&ctx->forks.side[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->forks.fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->forks.sc_stream, cudaStreamNonBlocking);
@@ -1454,7 +1573,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     AL(ctx->sc_sys, scs.size());
     AL(ctx->sc_bead, scb.size());
     AL(ctx->colwork, cw.size());
-    AL(ctx->cw_part, 4 * cw.size());
+    AL(ctx->cw_part, 5 * cw.size());
     AL(ctx->cw_ticket, n_systems);
     AL(ctx->fin_ticket, 1);
     AL(ctx->acc, n_systems);
@@ -1568,6 +1687,14 @@ void qtg_destroy(qtg_ctx *ctx) {
     for (cudaEvent_t ev : {ctx->ev_fork[0], ctx->ev_fork[1], ctx->ev_join, ctx->forks.fork, ctx->forks.join[0],
                            ctx->forks.join[1], ctx->sur_fork, ctx->sur_join, ctx->forks.sc_fork, ctx->forks.sc_join})
         if (ev) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : ctx->ring_done)
+        if (ev) cudaEventDestroy(ev);
+    for (auto &p : ctx->part_of) {
+        for (cudaEvent_t ev : {p.join, p.forks.fork, p.forks.join[0], p.forks.join[1]})
+            if (ev) cudaEventDestroy(ev);
+        for (cudaStream_t st : {p.stream, p.forks.side[0], p.forks.side[1]})
+            if (st) cudaStreamDestroy(st);
+    }
     for (cudaStream_t st : {ctx->forks.side[0], ctx->forks.side[1], ctx->forks.sc_stream})
         if (st) cudaStreamDestroy(st);
     delete ctx;
