@@ -1,35 +1,25 @@
 // qTIP4P/F force evaluation on GB300 (replaces forces.cpp:25-630).
 //
-// A launch evaluates a batch of "jobs" (one configuration of one system each;
-// all beads of all replicas at once). Per job:
-//   k_prep     charge sites (M, H1, H2) wrapped into the box with their charges,
-//              wrapped oxygen positions, and per-site phase tables
-//              exp(i 2 pi m s_d), m = 0..k_max, d = x,y,z (complex recursion from
-//              exp(i 2 pi s_d), charge folded into the x factor);
-//   k_real     real-space Ewald between sites of different molecules; grid =
-//              (i-site tiles) x (j-chunks) x jobs, j-sites staged through shared
-//              memory, each thread owns one i-site and writes one partial force
-//              per j-chunk (no atomics, deterministic);
-//   k_ksk      structure factors S(k) = sum_i q_i exp(i k.r_i); grid = (k tiles)
-//              x (site chunks) x jobs, one thread per k-vector, site chunks staged
-//              in shared memory, 32-site partial sums promoted to FP64;
-//   k_kforce   reciprocal-space site forces; grid = (i-site tiles) x (k-chunks)
-//              x jobs, (k, 2 c_k k, S(k)) broadcast from shared memory, S(k)
-//              summed over the site-chunk partials in fixed order;
-//   k_combine  per molecule: partial site forces summed in fixed order, same-
-//              molecule real-space pairs (erfc - 1), quartic-Morse bonds, HOH
-//              angle (FP64 difference vectors), M-site chain rule;
-//   k_lj       O-O Lennard-Jones over the CSR Verlet list, one warp per row.
-//   k_lj_dense O-O Lennard-Jones of the device stepper (mixed), all pairs from shared memory.
-// The kernels are templated on the arithmetic type: double for the parity
-// mode, float (FP64 accumulation across tiles/chunks/planes) for the mixed
-// mode. Mode-1 jobs compute the directional derivative of the intermolecular
-// Ewald forces along a per-dof direction (the Suzuki-Chin force gradient).
+// A launch evaluates a batch of "jobs" (one configuration of one system each; all beads of
+// all replicas at once). This file holds the mixed form's kernels (FP32 arithmetic with
+// compensated or FP64 sums), and the launches of both forms:
+//   k_prep_f32       charge sites (M, H1, H2) wrapped into the box, wrapped oxygens, and the
+//                    sites' phase tables exp(i 2 pi m s_d), m = 0 .. k_max;
+//   k_real_half(2)   real-space Ewald, every pair of sites once (k_real_f32: every ordered
+//                    pair, k_real_list: over a pair list, for larger beads);
+//   k_ksk, k_sk_reduce, k_kforce_f32   structure factors, their sums and weights, and the
+//                    reciprocal-space site forces (recip32.cu: k_ksk2, for large batches);
+//   k_lj_dense, k_lj_list_f32, k_lj    O-O Lennard-Jones over all pairs, the stepper's
+//                    symmetric or the caller's half list;
+//   k_intra_f32      same-molecule pairs (erfc - 1), quartic-Morse bonds, HOH angle;
+//   k_combine_f32    a molecule's partial forces in fixed order, M-site chain rule.
+// Mode-1 jobs (k_real_d, k_ksk<1>, k_sk_reduce<1>, k_kforce<1>) compute the directional
+// derivative of the intermolecular Ewald forces along a per-dof direction (the Suzuki-Chin
+// force gradient). The FP64 form's kernels are in real64.cu, recip64.cu and short64.cu.
 #include <math.h>
 
 #include <algorithm>
 #include <string>
-#include <type_traits>
 
 #include "packed.h"
 #include "qtg_internal.h"
@@ -37,28 +27,6 @@
 namespace qtg {
 
 namespace {
-
-template <typename R> struct V4;
-template <> struct __align__(16) V4<float> { float x, y, z, w; };
-template <> struct __align__(16) V4<double> { double x, y, z, w; };
-template <typename R> struct V2;
-template <> struct __align__(8) V2<float> { float x, y; };
-template <> struct __align__(16) V2<double> { double x, y; };
-
-__device__ __forceinline__ double f_erfc(double x) { return erfc(x); }
-__device__ __forceinline__ double f_exp(double x) { return exp(x); }
-__device__ __forceinline__ float f_rint(float x) { return rintf(x); }
-__device__ __forceinline__ double f_rint(double x) { return rint(x); }
-__device__ __forceinline__ double f_sqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double f_acos(double x) { return acos(x); }
-__device__ __forceinline__ void f_sincospi(double t, double *s, double *c) { sincospi(t, s, c); }
-
-template <typename R> __device__ __forceinline__ R sys_box(const SysDev &S, int d);
-template <> __device__ __forceinline__ float sys_box<float>(const SysDev &S, int d) { return S.boxf[d]; }
-template <> __device__ __forceinline__ double sys_box<double>(const SysDev &S, int d) { return S.box[d]; }
-template <typename R> __device__ __forceinline__ R sys_ibox(const SysDev &S, int d);
-template <> __device__ __forceinline__ float sys_ibox<float>(const SysDev &S, int d) { return S.inv_boxf[d]; }
-template <> __device__ __forceinline__ double sys_ibox<double>(const SysDev &S, int d) { return S.inv_box[d]; }
 
 __device__ __forceinline__ int chunk_lo(int n, int c, int nc) { return (int)(((long long)n * c) / nc); }
 
@@ -98,13 +66,6 @@ __device__ __forceinline__ void pair_terms(float r2, float kap, float kap2, floa
     *ex = e;
     *ec = t * as_poly(t) * e;
 }
-__device__ __forceinline__ void pair_terms(double r2, double kap, double kap2, double *inv, double *ex, double *ec) {
-    const double r = sqrt(r2);
-    *inv = 1.0 / r;
-    *ex = exp(-kap2 * r2);
-    *ec = erfc(kap * r);
-}
-
 // ---- k_prep_f32 (mixed; the FP64 form's k_prep64 is in recip64.cu) --------------
 // One thread per (site, dimension): each dimension of
 // the M site, the box fraction, the fixed-point fraction and the phase-table
@@ -202,31 +163,20 @@ __device__ __forceinline__ void kahan_add(R &s, R &c, R v) {
     s = t;
 }
 
-// Partial site-force planes: FP64 in the FP64 form; FP32 in the mixed form
-// (each plane is a compensated FP32 sum rounded once; k_combine_f32 adds the
-// planes with compensation), which halves their traffic and keeps the plane
-// sum off the FP64 pipe.
-template <typename R>
-__device__ __forceinline__ void store_plane(double *part, size_t at3, R x, R y, R z);
-template <>
-__device__ __forceinline__ void store_plane<double>(double *part, size_t at3, double x, double y, double z) {
-    part[at3] = x;
-    part[at3 + 1] = y;
-    part[at3 + 2] = z;
-}
-template <>
-__device__ __forceinline__ void store_plane<float>(double *part, size_t at3, float x, float y, float z) {
+// Partial site-force planes: FP32 (each a compensated FP32 sum rounded once; k_combine_f32
+// adds the planes with compensation), which keeps the plane sum off the FP64 pipe.
+__device__ __forceinline__ void store_plane(double *part, size_t at3, float x, float y, float z) {
     float *p = reinterpret_cast<float *>(part) + at3;
     p[0] = x;
     p[1] = y;
     p[2] = z;
 }
 
-// ---- k_real: intermolecular real-space Ewald ----------------------------------
+// ---- k_real_d: directional derivative of the real-space forces -------------------
+// Every ordered pair of sites; j-sites staged through shared memory, one i-site a thread.
 constexpr int RT = 128;
 
-template <typename R, int MODE>
-__global__ void __launch_bounds__(RT) k_real(EvalArgs a) {
+__global__ void __launch_bounds__(RT) k_real_d(EvalArgs a) {
     const int rj = blockIdx.y, jb = blockIdx.z;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
@@ -235,81 +185,68 @@ __global__ void __launch_bounds__(RT) k_real(EvalArgs a) {
     const int i = blockIdx.x * RT + threadIdx.x;
     const bool act = i < ns;
     const int j0 = chunk_lo(ns, rj, a.n_rj), j1 = chunk_lo(ns, rj + 1, a.n_rj);
-    const V4<R> *sites = reinterpret_cast<const V4<R> *>(a.sites) + J.site_off;
-    const V4<R> *tans = reinterpret_cast<const V4<R> *>(a.tan_sites) + J.site_off;
-    __shared__ V4<R> sj[RT];
-    __shared__ V4<R> uj[MODE == 1 ? RT : 1];
-    __shared__ double red[RT / 32];
-    const R L0 = sys_box<R>(S, 0), L1 = sys_box<R>(S, 1), L2 = sys_box<R>(S, 2);
-    const R I0 = sys_ibox<R>(S, 0), I1 = sys_ibox<R>(S, 1), I2 = sys_ibox<R>(S, 2);
-    const R rc2 = (R)S.rc_sq, kap = (R)S.kappa, kap2 = (R)(S.kappa * S.kappa), pref = (R)S.ewald_pref;
-    V4<R> si;
-    si.x = si.y = si.z = si.w = (R)0;
-    V4<R> ui = si;
+    const float4 *sites = reinterpret_cast<const float4 *>(a.sites) + J.site_off;
+    const float4 *tans = reinterpret_cast<const float4 *>(a.tan_sites) + J.site_off;
+    __shared__ float4 sj[RT];
+    __shared__ float4 uj[RT];
+    const float L0 = S.boxf[0], L1 = S.boxf[1], L2 = S.boxf[2];
+    const float I0 = S.inv_boxf[0], I1 = S.inv_boxf[1], I2 = S.inv_boxf[2];
+    const float rc2 = (float)S.rc_sq, kap = (float)S.kappa, kap2 = (float)(S.kappa * S.kappa), pref = (float)S.ewald_pref;
+    float4 si;
+    si.x = si.y = si.z = si.w = 0.f;
+    float4 ui = si;
     if (act) {
         si = sites[i];
-        if (MODE == 1) ui = tans[i];
+        ui = tans[i];
     }
     const int mlo = (i / 3) * 3;  // first site of i's molecule
-    double Fx = 0.0, Fy = 0.0, Fz = 0.0, E = 0.0;
+    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
     for (int t0 = j0; t0 < j1; t0 += RT) {
         __syncthreads();
         if (t0 + threadIdx.x < j1) {
             sj[threadIdx.x] = sites[t0 + threadIdx.x];
-            if (MODE == 1) uj[threadIdx.x] = tans[t0 + threadIdx.x];
+            uj[threadIdx.x] = tans[t0 + threadIdx.x];
         }
         __syncthreads();
         const int nj = min(RT, j1 - t0);
-        R fx = 0, fy = 0, fz = 0, e = 0;
+        float fx = 0, fy = 0, fz = 0;
         if (act) {
             for (int jj = 0; jj < nj; ++jj) {
                 if ((unsigned)(t0 + jj - mlo) < 3u) continue;  // same molecule
-                const V4<R> b = sj[jj];
-                R dx = si.x - b.x, dy = si.y - b.y, dz = si.z - b.z;
-                dx -= L0 * f_rint(dx * I0);
-                dy -= L1 * f_rint(dy * I1);
-                dz -= L2 * f_rint(dz * I2);
-                const R r2 = dx * dx + dy * dy + dz * dz;
+                const float4 b = sj[jj];
+                float dx = si.x - b.x, dy = si.y - b.y, dz = si.z - b.z;
+                dx -= L0 * rintf(dx * I0);
+                dy -= L1 * rintf(dy * I1);
+                dz -= L2 * rintf(dz * I2);
+                const float r2 = dx * dx + dy * dy + dz * dz;
                 if (r2 < rc2) {
-                    R inv, ex, ec;
+                    float inv, ex, ec;
                     pair_terms(r2, kap, kap2, &inv, &ex, &ec);
-                    const R qq = si.w * b.w;
-                    const R en = qq * inv * ec;
-                    const R hq = qq * pref * ex;
-                    const R phi = (en + hq) * inv * inv;
-                    if (MODE == 0) {
-                        e += en;
-                        fx += phi * dx;
-                        fy += phi * dy;
-                        fz += phi * dz;
-                    } else {
-                        // d/d(eps) of phi(r^2) r along u = u_i - u_j:
-                        // phi' = dphi/d(r^2) = -1.5 phi / r^2 - kappa^2 hq / r^2
-                        const V4<R> ub = uj[jj];
-                        const R ux = ui.x - ub.x, uy = ui.y - ub.y, uz = ui.z - ub.z;
-                        const R ru = dx * ux + dy * uy + dz * uz;
-                        const R dphi = (-(R)1.5 * phi - kap2 * hq) * inv * inv;
-                        const R c2 = (R)2 * dphi * ru;
-                        fx += phi * ux + c2 * dx;
-                        fy += phi * uy + c2 * dy;
-                        fz += phi * uz + c2 * dz;
-                    }
+                    const float qq = si.w * b.w;
+                    const float en = qq * inv * ec;
+                    const float hq = qq * pref * ex;
+                    const float phi = (en + hq) * inv * inv;
+                    // d/d(eps) of phi(r^2) r along u = u_i - u_j:
+                    // phi' = dphi/d(r^2) = -1.5 phi / r^2 - kappa^2 hq / r^2
+                    const float4 ub = uj[jj];
+                    const float ux = ui.x - ub.x, uy = ui.y - ub.y, uz = ui.z - ub.z;
+                    const float ru = dx * ux + dy * uy + dz * uz;
+                    const float dphi = (-1.5f * phi - kap2 * hq) * inv * inv;
+                    const float c2 = 2.0f * dphi * ru;
+                    fx += phi * ux + c2 * dx;
+                    fy += phi * uy + c2 * dy;
+                    fz += phi * uz + c2 * dz;
                 }
             }
         }
         Fx += (double)fx;
         Fy += (double)fy;
         Fz += (double)fz;
-        E += (double)e;
     }
-    if (act) store_plane<R>(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + i), (R)Fx, (R)Fy, (R)Fz);
-    if (MODE == 0) {
-        const double t = block_sum(0.5 * E, red);
-        if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
-    }
+    if (act) store_plane(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + i), (float)Fx, (float)Fy, (float)Fz);
 }
 
-// FP32 form of k_real<float, 0> (energies and forces): the pair term is
+// Real-space energies and forces of every ordered pair: the pair term is
 // q_i q_j [A, (A + B) / r^2] with A = erfc(kappa r) / r and
 // B = (2 kappa / sqrt(pi)) exp(-kappa^2 r^2); q_i is factored out of the sums,
 // the same-molecule exclusion joins the cutoff predicate, and each 128-site
@@ -371,7 +308,7 @@ __global__ void __launch_bounds__(RT) k_real_f32(EvalArgs a) {
     }
     const double qi = (double)si.w;
     if (act)
-        store_plane<float>(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + i), si.w * (Sx - Cx),
+        store_plane(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + i), si.w * (Sx - Cx),
                            si.w * (Sy - Cy), si.w * (Sz - Cz));
     const double t = block_sum(0.5 * qi * ((double)Se - (double)Ce), red);
     if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], t);
@@ -647,7 +584,7 @@ __global__ void __launch_bounds__(32 * RLW) k_real_list(EvalArgs a) {
         const float fx = lane == 0 ? f[0] : (lane == 1 ? f[3] : f[6]);
         const float fy = lane == 0 ? f[1] : (lane == 1 ? f[4] : f[7]);
         const float fz = lane == 0 ? f[2] : (lane == 1 ? f[5] : f[8]);
-        store_plane<float>(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + 3 * i + lane), q * fx, q * fy,
+        store_plane(a.part, 3 * ((size_t)rj * a.total_sites + J.site_off + 3 * i + lane), q * fx, q * fy,
                            q * fz);
     }
     __shared__ double red[RLW];
@@ -1139,13 +1076,13 @@ constexpr int CH = 32;   // sites per shared-memory chunk
 // complex product, whose third products (Ar + Ai)(Zr +- Zi) are U +- V, with T1 and
 // T2 shared by +kz and -kz): four FMAs for the pair instead of eight. Then
 // S(+kz) = T1 - T2 + i (U + V - T1 - T2) and S(-kz) = T1 + T2 + i (U - V - T1 + T2).
-template <typename R, int MODE, int KZ>
+template <int MODE, int KZ>
 __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
     const int sc = blockIdx.y, jb = blockIdx.z;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
     // the FP32 energy/force form runs over the half set (kx = 0, ky < 0 columns left out)
-    const bool half = sizeof(R) == 4 && MODE == 0;
+    constexpr bool half = MODE == 0;
     const int ng = half ? S.n_grp_half : S.n_grp, ns = S.n_sites, km1 = S.k_max + 1;
     if (blockIdx.x * KT >= ng) return;
     const int t = blockIdx.x * KT + threadIdx.x;
@@ -1153,9 +1090,8 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
     const int s0 = chunk_lo(ns, sc, a.n_sc), s1 = chunk_lo(ns, sc + 1, a.n_sc);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // two buffers (chunk i computed while chunk i + 1 is copied in)
-    V4<R> *ush = reinterpret_cast<V4<R> *>(smem_raw);      // [2][CH] (mode 1)
-    V2<R> *tab = reinterpret_cast<V2<R> *>(ush + 2 * CH);  // [2][3*km1][CH+1]
-    constexpr bool G3 = sizeof(R) == 4 && MODE == 0;
+    float4 *ush = reinterpret_cast<float4 *>(smem_raw);      // [2][CH] (mode 1)
+    float2 *tab = reinterpret_cast<float2 *>(ush + 2 * CH);  // [2][3*km1][CH+1]
     KGroup G;
     G.col = G.kz0 = G.n = 0;
     KCol C;
@@ -1165,45 +1101,39 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
         C = a.kcol[S.col_off + G.col];
     }
     const int ax = C.kx, ay = abs(C.ky);
-    const R sy = C.ky < 0 ? (R)-1 : (R)1;
-    const R bz = (R)(2.0 * PI_REF * S.inv_box[2]);
-    const R kx = (R)(2.0 * PI_REF * C.kx * S.inv_box[0]), ky = (R)(2.0 * PI_REF * C.ky * S.inv_box[1]);
+    const float sy = C.ky < 0 ? -1.f : 1.f;
+    const float bz = (float)(2.0 * PI_REF * S.inv_box[2]);
+    const float kx = (float)(2.0 * PI_REF * C.kx * S.inv_box[0]), ky = (float)(2.0 * PI_REF * C.ky * S.inv_box[1]);
     // the group's |kz| values az = kz0 .. kz0 + n - 1; each covers kz = +az and -az
     int zrow[KZ];
-    R kzr[KZ];
+    float kzr[KZ];
 #pragma unroll
     for (int g = 0; g < KZ; ++g) {
         zrow[g] = (2 * km1 + min(G.kz0 + g, km1 - 1)) * (CH + 1);
-        kzr[g] = bz * (R)(G.kz0 + g);
+        kzr[g] = bz * (float)(G.kz0 + g);
     }
     // compensated running sums over the chunk totals, [g][0] for +az, [g][1] for -az
-    R Sr[KZ][2], Si[KZ][2], Cr[KZ][2], Ci[KZ][2], dSr[KZ][2], dSi[KZ][2], dCr[KZ][2], dCi[KZ][2];
+    float Sr[KZ][2], Si[KZ][2], Cr[KZ][2], Ci[KZ][2], dSr[KZ][2], dSi[KZ][2], dCr[KZ][2], dCi[KZ][2];
 #pragma unroll
     for (int g = 0; g < KZ; ++g)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) Sr[g][h] = Si[g][h] = Cr[g][h] = Ci[g][h] = dSr[g][h] = dSi[g][h] = dCr[g][h] = dCi[g][h] = (R)0;
-    const V2<R> *ph = reinterpret_cast<const V2<R> *>(a.phase) + J.phase_off;
-    const V4<R> *tans = reinterpret_cast<const V4<R> *>(a.tan_sites) + J.site_off;
+        for (int h = 0; h < 2; ++h) Sr[g][h] = Si[g][h] = Cr[g][h] = Ci[g][h] = dSr[g][h] = dSi[g][h] = dCr[g][h] = dCi[g][h] = 0.f;
+    const float2 *ph = reinterpret_cast<const float2 *>(a.phase) + J.phase_off;
+    const float4 *tans = reinterpret_cast<const float4 *>(a.tan_sites) + J.site_off;
     const int rows = 3 * km1, nchunk = s1 > s0 ? (s1 - s0 + CH - 1) / CH : 0;
     // copies of chunk ci's phase rows (and tangents) into buffer ci & 1, zero past s1
     auto stage = [&](int ci) {
         const int c0 = s0 + ci * CH;
-        V2<R> *tb = tab + (ci & 1) * rows * (CH + 1);
+        float2 *tb = tab + (ci & 1) * rows * (CH + 1);
         for (int idx = threadIdx.x; idx < rows * CH; idx += KT) {
             const int row = idx / CH, c = idx - row * CH, s = c0 + c;
-            cp_async<sizeof(V2<R>)>(tb + row * (CH + 1) + c, ph + (size_t)row * ns + min(s, s1 - 1), s < s1);
+            cp_async<sizeof(float2)>(tb + row * (CH + 1) + c, ph + (size_t)row * ns + min(s, s1 - 1), s < s1);
         }
         if (MODE == 1 && threadIdx.x < CH) {
             const int s = c0 + threadIdx.x;
-            const V4<R> *src = tans + min(s, s1 - 1);
-            V4<R> *dst = ush + (ci & 1) * CH + threadIdx.x;
-            if constexpr (sizeof(V4<R>) == 16) {
-                cp_async<16>(dst, src, s < s1);
-            } else {
-                cp_async<16>(dst, src, s < s1);
-                cp_async<16>(reinterpret_cast<unsigned char *>(dst) + 16, reinterpret_cast<const unsigned char *>(src) + 16,
-                             s < s1);
-            }
+            const float4 *src = tans + min(s, s1 - 1);
+            float4 *dst = ush + (ci & 1) * CH + threadIdx.x;
+            cp_async<16>(dst, src, s < s1);
         }
         cp_async_commit();
     };
@@ -1215,23 +1145,23 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
         else cp_async_commit();
         cp_async_wait<1>();  // this thread's copies of chunk ci have landed
         __syncthreads();     // and every other thread's
-        const V2<R> *tab_c = tab + (ci & 1) * rows * (CH + 1);
-        const V4<R> *ush_c = ush + (ci & 1) * CH;
+        const float2 *tab_c = tab + (ci & 1) * rows * (CH + 1);
+        const float4 *ush_c = ush + (ci & 1) * CH;
         const int nc = min(CH, s1 - c0);
-        R sr[KZ][2], si[KZ][2], dsr[KZ][2], dsi[KZ][2];
+        float sr[KZ][2], si[KZ][2], dsr[KZ][2], dsi[KZ][2];
 #pragma unroll
         for (int g = 0; g < KZ; ++g)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) sr[g][h] = si[g][h] = dsr[g][h] = dsi[g][h] = (R)0;
+            for (int h = 0; h < 2; ++h) sr[g][h] = si[g][h] = dsr[g][h] = dsi[g][h] = 0.f;
         auto site = [&](int c) {
-            const V2<R> x = tab_c[ax * (CH + 1) + c], y = tab_c[(km1 + ay) * (CH + 1) + c];
-            const R yi = sy * y.y;
-            const R pr = x.x * y.x - x.y * yi, pi = x.x * yi + x.y * y.x;
-            if constexpr (G3) {
+            const float2 x = tab_c[ax * (CH + 1) + c], y = tab_c[(km1 + ay) * (CH + 1) + c];
+            const float yi = sy * y.y;
+            const float pr = x.x * y.x - x.y * yi, pi = x.x * yi + x.y * y.x;
+            if constexpr (half) {
                 const float ps = (float)(pr + pi);
 #pragma unroll
                 for (int g = 0; g < KZ; ++g) {
-                    const V2<R> z = tab_c[zrow[g] + c];
+                    const float2 z = tab_c[zrow[g] + c];
                     sr[g][0] = fmaf((float)pr, (float)z.x, sr[g][0]);  // T1
                     sr[g][1] = fmaf((float)pi, (float)z.y, sr[g][1]);  // T2
                     si[g][0] = fmaf(ps, (float)z.x, si[g][0]);         // U
@@ -1239,40 +1169,24 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
                 }
                 return;
             }
-            R kxyu = (R)0, uz = (R)0;
-            if (MODE == 1) {
-                const V4<R> u = ush_c[c];
-                kxyu = kx * u.x + ky * u.y;
-                uz = u.z;
-            }
+            const float4 u = ush_c[c];
+            const float kxyu = kx * u.x + ky * u.y, uz = u.z;
 #pragma unroll
             for (int g = 0; g < KZ; ++g) {
-                const V2<R> z = tab_c[zrow[g] + c];
-                if (MODE == 0) {
-                    // A Z (kz = +az) and A conj(Z) (kz = -az) accumulated by FMAs alone
-                    sr[g][0] = fma(pr, z.x, sr[g][0]);
-                    sr[g][0] = fma(-pi, z.y, sr[g][0]);
-                    si[g][0] = fma(pi, z.x, si[g][0]);
-                    si[g][0] = fma(pr, z.y, si[g][0]);
-                    sr[g][1] = fma(pr, z.x, sr[g][1]);
-                    sr[g][1] = fma(pi, z.y, sr[g][1]);
-                    si[g][1] = fma(pi, z.x, si[g][1]);
-                    si[g][1] = fma(-pr, z.y, si[g][1]);
-                } else {
-                    // A Z (kz = +az) and A conj(Z) (kz = -az) share their products
-                    const R t1 = pr * z.x, t2 = pi * z.x;
-                    const R erp = t1 - pi * z.y, eip = t2 + pr * z.y;
-                    const R erm = t1 + pi * z.y, eim = t2 - pr * z.y;
-                    sr[g][0] += erp;
-                    si[g][0] += eip;
-                    sr[g][1] += erm;
-                    si[g][1] += eim;
-                    const R kup = kxyu + kzr[g] * uz, kum = kxyu - kzr[g] * uz;
-                    dsr[g][0] -= kup * eip;
-                    dsi[g][0] += kup * erp;
-                    dsr[g][1] -= kum * eim;
-                    dsi[g][1] += kum * erm;
-                }
+                const float2 z = tab_c[zrow[g] + c];
+                // A Z (kz = +az) and A conj(Z) (kz = -az) share their products
+                const float t1 = pr * z.x, t2 = pi * z.x;
+                const float erp = t1 - pi * z.y, eip = t2 + pr * z.y;
+                const float erm = t1 + pi * z.y, eim = t2 - pr * z.y;
+                sr[g][0] += erp;
+                si[g][0] += eip;
+                sr[g][1] += erm;
+                si[g][1] += eim;
+                const float kup = kxyu + kzr[g] * uz, kum = kxyu - kzr[g] * uz;
+                dsr[g][0] -= kup * eip;
+                dsi[g][0] += kup * erp;
+                dsr[g][1] -= kum * eim;
+                dsi[g][1] += kum * erm;
             }
         };
         if (nc == CH) {  // a full chunk: a fixed trip count, unrolled
@@ -1303,7 +1217,7 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
                     if (h == 1 && az == 0) continue;  // kz = 0 has one entry
                     const int kz = h ? -az : az;
                     const size_t at = (size_t)sc * a.total_k + J.sk_off + C.k_begin + (kz + C.m);
-                    if constexpr (G3) {
+                    if constexpr (half) {
                         // FP32 form: the compensated pair (S, C) of S(kz) itself, from the
                         // (sum, compensation) pairs of T1, T2, U and V
                         const float t1 = (float)Sr[g][0], t2 = (float)Sr[g][1], u1 = (float)Cr[g][0], u2 = (float)Cr[g][1];
@@ -1315,11 +1229,11 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
                             o = make_float4(t1 + t2, ((us - vs) - t1) + t2, u1 + u2, ((uc - vc) - u1) + u2);
                         }
                         reinterpret_cast<float4 *>(a.skp)[at] = o;
-                    } else
+                    } else {
                         a.skp[at] = make_double2((double)Sr[g][h] - (double)Cr[g][h], (double)Si[g][h] - (double)Ci[g][h]);
-                    if (MODE == 1)
                         a.dskp[at] = make_double2((double)dSr[g][h] - (double)dCr[g][h],
                                                   (double)dSi[g][h] - (double)dCi[g][h]);
+                    }
                 }
             }
         }
@@ -1477,13 +1391,13 @@ void launch_sk_reduce(const EvalArgs &a, cudaStream_t s) {
 constexpr int FT = 128;  // threads (sites) per block
 constexpr int KB = 128;  // k-vectors per batch (at most)
 
-template <typename R, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(FT) k_kforce(EvalArgs a) {
     const int kc = blockIdx.y, jb = blockIdx.z;
     const Job J = a.jobs[jb];
     const SysDev &S = a.sys[J.sys];
     // FP32 energy/force form: the half set, whose weights k_sk_reduce writes
-    const int nb = (sizeof(R) == 4 && MODE == 0) ? S.n_batch_half : S.n_batch, ns = S.n_sites, km1 = S.k_max + 1;
+    const int nb = MODE == 0 ? S.n_batch_half : S.n_batch, ns = S.n_sites, km1 = S.k_max + 1;
     if (blockIdx.x * FT >= ns) return;
     const int i = blockIdx.x * FT + threadIdx.x;
     const bool act = i < ns;
@@ -1491,26 +1405,26 @@ __global__ void __launch_bounds__(FT) k_kforce(EvalArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // 16-byte elements first so every array stays aligned for vector access
     KCol *cs = reinterpret_cast<KCol *>(smem_raw);  // [KB]
-    V2<R> *ss = reinterpret_cast<V2<R> *>(cs + KB);  // [KB] 2 c_k S(k)
-    V2<R> *ds = ss + KB;                             // [KB] 2 c_k dS(k)
-    V2<R> *zr = ds + KB;                             // [km1][FT] my Z(kz) row
-    const V2<R> *ph = reinterpret_cast<const V2<R> *>(a.phase) + J.phase_off;
+    float2 *ss = reinterpret_cast<float2 *>(cs + KB);  // [KB] 2 c_k S(k)
+    float2 *ds = ss + KB;                             // [KB] 2 c_k dS(k)
+    float2 *zr = ds + KB;                             // [km1][FT] my Z(kz) row
+    const float2 *ph = reinterpret_cast<const float2 *>(a.phase) + J.phase_off;
     for (int m = 0; m < km1; ++m) {
-        V2<R> v;
-        v.x = v.y = (R)0;
+        float2 v;
+        v.x = v.y = 0.f;
         if (act) v = ph[(size_t)(2 * km1 + m) * ns + i];
         zr[m * FT + threadIdx.x] = v;
     }
-    V4<R> ui;
-    ui.x = ui.y = ui.z = ui.w = (R)0;
-    if (MODE == 1 && act) ui = reinterpret_cast<const V4<R> *>(a.tan_sites)[J.site_off + i];
-    const R bx = (R)(2.0 * PI_REF * S.inv_box[0]), by = (R)(2.0 * PI_REF * S.inv_box[1]),
-            bz = (R)(2.0 * PI_REF * S.inv_box[2]);
+    float4 ui;
+    ui.x = ui.y = ui.z = ui.w = 0.f;
+    if (MODE == 1 && act) ui = reinterpret_cast<const float4 *>(a.tan_sites)[J.site_off + i];
+    const float bx = (float)(2.0 * PI_REF * S.inv_box[0]), by = (float)(2.0 * PI_REF * S.inv_box[1]),
+            bz = (float)(2.0 * PI_REF * S.inv_box[2]);
     // per-batch sums added into Kahan-compensated running sums in the working precision
-    R Fx = 0, Fy = 0, Fz = 0, Cx = 0, Cy = 0, Cz = 0;
+    float Fx = 0, Fy = 0, Fz = 0, Cx = 0, Cy = 0, Cz = 0;
     const int ii = act ? i : 0;
-    const V2<R> *wsk = reinterpret_cast<const V2<R> *>(a.wsk) + J.sk_off;
-    const V2<R> *wdsk = reinterpret_cast<const V2<R> *>(a.wdsk) + J.sk_off;
+    const float2 *wsk = reinterpret_cast<const float2 *>(a.wsk) + J.sk_off;
+    const float2 *wdsk = reinterpret_cast<const float2 *>(a.wdsk) + J.sk_off;
     for (int bt = bt0; bt < bt1; ++bt) {
         const KBatch B = a.kbatch[S.batch_off + bt];
         __syncthreads();
@@ -1520,55 +1434,55 @@ __global__ void __launch_bounds__(FT) k_kforce(EvalArgs a) {
             if (MODE == 1) ds[idx] = wdsk[B.k0 + idx];
         }
         __syncthreads();
-        R fx = 0, fy = 0, fz = 0;
+        float fx = 0, fy = 0, fz = 0;
         for (int cc = 0; cc < B.c1 - B.c0; ++cc) {
             const KCol C = cs[cc];
-            const V2<R> x = ph[(size_t)C.kx * ns + ii];
-            const V2<R> y = ph[(size_t)(km1 + abs(C.ky)) * ns + ii];
-            const R yi = C.ky < 0 ? -y.y : y.y;
-            const R pr = x.x * y.x - x.y * yi, pi = x.x * yi + x.y * y.x;
-            R kxyu = (R)0;
-            if (MODE == 1) kxyu = bx * (R)C.kx * ui.x + by * (R)C.ky * ui.y;
+            const float2 x = ph[(size_t)C.kx * ns + ii];
+            const float2 y = ph[(size_t)(km1 + abs(C.ky)) * ns + ii];
+            const float yi = C.ky < 0 ? -y.y : y.y;
+            const float pr = x.x * y.x - x.y * yi, pi = x.x * yi + x.y * y.x;
+            float kxyu = 0.f;
+            if (MODE == 1) kxyu = bx * (float)C.kx * ui.x + by * (float)C.ky * ui.y;
             const int kb = C.k_begin - B.k0 + C.m;  // smem index of kz = 0
-            R v = 0, vz = 0;
+            float v = 0, vz = 0;
             {   // kz = 0: Z = 1
-                const V2<R> sk = ss[kb];
-                R val = sk.x * pi - sk.y * pr;
+                const float2 sk = ss[kb];
+                float val = sk.x * pi - sk.y * pr;
                 if (MODE == 1) {
-                    const V2<R> d = ds[kb];
+                    const float2 d = ds[kb];
                     val = (d.x * pi - d.y * pr) + kxyu * (sk.x * pr + sk.y * pi);
                 }
                 v += val;
             }
             // kz = +az and -az share the products of A Z and A conj(Z)
             for (int az = 1; az <= C.m; ++az) {
-                const V2<R> z = zr[az * FT + threadIdx.x];
-                const R t1 = pr * z.x, t2 = pi * z.x;
-                const R erp = t1 - pi * z.y, eip = t2 + pr * z.y;
-                const R erm = t1 + pi * z.y, eim = t2 - pr * z.y;
-                const V2<R> sp = ss[kb + az], sm = ss[kb - az];
-                R vp = sp.x * eip - sp.y * erp, vm = sm.x * eim - sm.y * erm;
+                const float2 z = zr[az * FT + threadIdx.x];
+                const float t1 = pr * z.x, t2 = pi * z.x;
+                const float erp = t1 - pi * z.y, eip = t2 + pr * z.y;
+                const float erm = t1 + pi * z.y, eim = t2 - pr * z.y;
+                const float2 sp = ss[kb + az], sm = ss[kb - az];
+                float vp = sp.x * eip - sp.y * erp, vm = sm.x * eim - sm.y * erm;
                 if (MODE == 1) {
-                    const V2<R> dp = ds[kb + az], dm = ds[kb - az];
-                    const R kup = kxyu + bz * (R)az * ui.z, kum = kxyu - bz * (R)az * ui.z;
+                    const float2 dp = ds[kb + az], dm = ds[kb - az];
+                    const float kup = kxyu + bz * (float)az * ui.z, kum = kxyu - bz * (float)az * ui.z;
                     vp = (dp.x * eip - dp.y * erp) + kup * (sp.x * erp + sp.y * eip);
                     vm = (dm.x * eim - dm.y * erm) + kum * (sm.x * erm + sm.y * eim);
                 }
                 v += vp + vm;
-                vz += (R)az * (vp - vm);
+                vz += (float)az * (vp - vm);
             }
-            fx += bx * (R)C.kx * v;
-            fy += by * (R)C.ky * v;
+            fx += bx * (float)C.kx * v;
+            fy += by * (float)C.ky * v;
             fz += bz * vz;
         }
         kahan_add(Fx, Cx, fx);
         kahan_add(Fy, Cy, fy);
         kahan_add(Fz, Cz, fz);
     }
-    if (act) store_plane<R>(a.part, 3 * ((size_t)(a.n_rj + kc) * a.total_sites + J.site_off + i), Fx - Cx, Fy - Cy, Fz - Cz);
+    if (act) store_plane(a.part, 3 * ((size_t)(a.n_rj + kc) * a.total_sites + J.site_off + i), Fx - Cx, Fy - Cy, Fz - Cz);
 }
 
-// FP32 form of k_kforce<float, 0> with the kz sums rearranged. Per site and
+// k_kforce<0> with the kz sums rearranged. Per site and
 // column, with A = X(kx) Y(ky) = pr + i pi, Z = Z(|kz|) = zx + i zy and the
 // column's weights W(+kz), W(-kz) (W = 2 c_k S(k)), the value summed above is
 //   vp + vm = pr [zy dx - zx sy] + pi [zx sx + zy dy],
@@ -1744,20 +1658,18 @@ __global__ void __launch_bounds__(FT) k_kforce_f32(EvalArgs a) {
 #pragma unroll
     for (int u = 0; u < SPT; ++u)
         if (site[u] < ns)
-            store_plane<float>(a.part, 3 * ((size_t)(a.n_rj + kc) * a.total_sites + J.site_off + site[u]),
+            store_plane(a.part, 3 * ((size_t)(a.n_rj + kc) * a.total_sites + J.site_off + site[u]),
                                Fx[u] - Cx[u], Fy[u] - Cy[u], Fz[u] - Cz[u]);
 }
 
-template <typename R>
 size_t kforce_smem(int kmax);
-template <typename R>
 size_t ksk_smem(int kmax);
 
 // k_ksk for the context's structure-factor group width
-template <typename R, int MODE>
+template <int MODE>
 void launch_ksk(const EvalArgs &a, dim3 grid, cudaStream_t s) {
-    if (a.kz == 3) k_ksk<R, MODE, 3><<<grid, KT, ksk_smem<R>(a.max_kmax), s>>>(a);
-    else k_ksk<R, MODE, 4><<<grid, KT, ksk_smem<R>(a.max_kmax), s>>>(a);
+    if (a.kz == 3) k_ksk<MODE, 3><<<grid, KT, ksk_smem(a.max_kmax), s>>>(a);
+    else k_ksk<MODE, 4><<<grid, KT, ksk_smem(a.max_kmax), s>>>(a);
 }
 
 // the FP32 k-force kernel for the largest |kz| of the batch (the general form beyond 32)
@@ -1772,7 +1684,7 @@ void launch_kforce_f32(const EvalArgs &a, dim3 grid, cudaStream_t s) {
     else if (a.kpk && a.max_kmax <= 16) launch_pdl(k_kforce_f32<16, 2>, g2, dim3(FT), sm, s, a);
     else if (a.kpk && a.max_kmax <= 24) launch_pdl(k_kforce_f32<24, 2>, g2, dim3(FT), sm, s, a);
     else if (a.kpk && a.max_kmax <= 32) launch_pdl(k_kforce_f32<32, 2>, g2, dim3(FT), sm, s, a);
-    else k_kforce<float, 0><<<grid, FT, kforce_smem<float>(a.max_kmax), s>>>(a);
+    else k_kforce<0><<<grid, FT, kforce_smem(a.max_kmax), s>>>(a);
 }
 
 // ---- k_combine: partial sums, short-range terms and the M-site chain rule ---------
@@ -1984,7 +1896,7 @@ __global__ void __launch_bounds__(CMT) k_combine_f32(EvalArgs a) {
 // relative band around r_cut^2, or whose separation is within rounding of
 // half a box in some dimension (where the two images tie and the rounding rule
 // picks the sign), is recomputed with exactly that arithmetic.
-template <typename R, int FULL>
+template <int FULL>
 __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     const int jb = blockIdx.y;
     const Job J = a.jobs[jb];
@@ -1997,9 +1909,8 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     double e = 0.0;
     const Consts &C = a.c;
     const double rc2 = C.r_cut_sq;
-    const R rc2r = (R)rc2;
-    const R bandr = sizeof(R) == 4 ? (R)1e-5 : (R)1e-12;
-    const R tie = sizeof(R) == 4 ? (R)1e-5 : (R)1e-12;
+    const float rc2r = (float)rc2;
+    const float bandr = (float)1e-5, tie = (float)1e-5;
     // half list: rows 0..N-2, entries j > i, forces on j by atomics; symmetric
     // list (FULL): rows 0..N-1, entries j != i, each pair seen from both ends, so
     // a row's force needs no atomics and the energy is halved
@@ -2021,56 +1932,48 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
             n0 = max(0, min(n0, cap));
             n1 = max(n0, min(n1, cap));
         }
-        R xi[3];
-        const V4<R> *opos = reinterpret_cast<const V4<R> *>(a.opos) + J.site_off / 3;
-        if (sizeof(R) == 4) {
-            const V4<R> o = opos[i];
-            xi[0] = o.x;
-            xi[1] = o.y;
-            xi[2] = o.z;
-        } else {
-            for (int d = 0; d < 3; ++d) xi[d] = (R)q[9 * i + d];
-        }
-        const R s6c = (R)C.sigmalj6, s12c = (R)C.sigmalj12, eps4 = (R)(4.0 * C.epslj), eps24 = (R)(24.0 * C.epslj);
-        R fi0 = 0, fi1 = 0, fi2 = 0, el = 0;
+        float xi[3];
+        const float4 *opos = reinterpret_cast<const float4 *>(a.opos) + J.site_off / 3;
+        const float4 o = opos[i];
+        xi[0] = o.x;
+        xi[1] = o.y;
+        xi[2] = o.z;
+        const float s6c = (float)C.sigmalj6, s12c = (float)C.sigmalj12, eps4 = (float)(4.0 * C.epslj), eps24 = (float)(24.0 * C.epslj);
+        float fi0 = 0, fi1 = 0, fi2 = 0, el = 0;
         for (int n = n0 + lane; n < n1; n += 32) {
             const int j = ls[n];
             if ((FULL ? j == i : j <= i) || j < 0 || j >= N) {
                 atomicOr(a.status, (unsigned)ST_LIST_OVERFLOW);
                 continue;
             }
-            R r[3];
-            if (sizeof(R) == 4) {
-                const V4<R> o = opos[j];
-                r[0] = xi[0] - o.x;
-                r[1] = xi[1] - o.y;
-                r[2] = xi[2] - o.z;
-            } else {
-                for (int d = 0; d < 3; ++d) r[d] = xi[d] - (R)q[9 * j + d];
-            }
+            float r[3];
+            const float4 o = opos[j];
+            r[0] = xi[0] - o.x;
+            r[1] = xi[1] - o.y;
+            r[2] = xi[2] - o.z;
             bool exact = false;
             for (int d = 0; d < 3; ++d) {
-                const R t = r[d] * sys_ibox<R>(S, d);
-                const R fr = fabs(t - trunc(t));
-                if (fabs(fr - (R)0.5) < tie) exact = true;
-                r[d] -= sys_box<R>(S, d) * f_rint(t);
+                const float t = r[d] * S.inv_boxf[d];
+                const float fr = fabs(t - trunc(t));
+                if (fabs(fr - 0.5f) < tie) exact = true;
+                r[d] -= S.boxf[d] * rintf(t);
             }
-            R r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+            float r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
             if (exact || fabs(r2 - rc2r) <= bandr * rc2r) {
                 double rd[3];
                 const double r2d = lj_exact_disp(q + 9 * i, q + 9 * j, S, rd);
-                for (int d = 0; d < 3; ++d) r[d] = (R)rd[d];
-                r2 = (R)r2d;
+                for (int d = 0; d < 3; ++d) r[d] = (float)rd[d];
+                r2 = (float)r2d;
                 exact = r2d < rc2;
             } else {
-                exact = r2 < (R)rc2;
+                exact = r2 < (float)rc2;
             }
             if (exact) {
-                const R i2 = (R)1 / r2, i6 = i2 * i2 * i2;
-                const R s6 = i6 * s6c, s12 = i6 * i6 * s12c;
-                const R en = s12 - s6;
-                el += en * eps4 - (R)C.e_cut;
-                const R ff = (en + s12) * eps24 * i2;
+                const float i2 = 1.0f / r2, i6 = i2 * i2 * i2;
+                const float s6 = i6 * s6c, s12 = i6 * i6 * s12c;
+                const float en = s12 - s6;
+                el += en * eps4 - (float)C.e_cut;
+                const float ff = (en + s12) * eps24 * i2;
                 fi0 += ff * r[0];
                 fi1 += ff * r[1];
                 fi2 += ff * r[2];
@@ -2420,16 +2323,13 @@ __global__ void __launch_bounds__(256) k_fp64_probe(double *out, int iters) {
     if (t == 12345.0) out[0] = t;  // keeps the chains live
 }
 
-template <typename R>
 size_t ksk_smem(int kmax) {
-    return 2 * (CH * sizeof(V4<R>) + (size_t)3 * (kmax + 1) * (CH + 1) * sizeof(V2<R>));
+    return 2 * (CH * sizeof(float4) + (size_t)3 * (kmax + 1) * (CH + 1) * sizeof(float2));
 }
-template <typename R>
 size_t kforce_smem(int kmax) {
-    return (size_t)KB * (sizeof(KCol) + 2 * sizeof(V2<R>)) + (size_t)(kmax + 1) * FT * sizeof(V2<R>);
+    return (size_t)KB * (sizeof(KCol) + 2 * sizeof(float2)) + (size_t)(kmax + 1) * FT * sizeof(float2);
 }
 
-template <typename R>
 void set_attrs() {
     const int big = 200 * 1024;
     cudaFuncSetAttribute(k_kforce_f32<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -2438,12 +2338,12 @@ void set_attrs() {
     cudaFuncSetAttribute(k_kforce_f32<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_kforce_f32<24, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_kforce_f32<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_ksk<R, 0, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_ksk<R, 1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_ksk<R, 0, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_ksk<R, 1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_kforce<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    cudaFuncSetAttribute(k_kforce<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_ksk<0, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_ksk<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_ksk<0, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_ksk<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_kforce<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_kforce<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 }
 
 // Chunk counts so that each force kernel launches enough 4-warp blocks to keep
@@ -2464,7 +2364,7 @@ void launch_lj_dense(const EvalArgs &a, cudaStream_t s) {
         return;
     }
     if (a.lj_list) {
-        k_lj<float, 1><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
+        k_lj<1><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
         return;
     }
     const long long blocks8 = (long long)((a.max_mols + 15) / 16) * a.n_jobs;
@@ -2539,7 +2439,7 @@ void set_ksk2_chunks(EvalArgs &a) {
 void launch_recip(const EvalArgs &a, cudaStream_t s) {
     const int ns = 3 * a.max_mols, tiles = (ns + FT - 1) / FT, ktiles = (a.max_grp + KT - 1) / KT;
     if (ksk2_ok(a)) launch_ksk2(a, s);
-    else launch_ksk<float, 0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
+    else launch_ksk<0>(a, dim3(ktiles, a.n_sc, a.n_jobs), s);
     if (a.sk_sites) launch_sk_reduce<2>(a, s);
     else launch_sk_reduce<0>(a, s);
     launch_kforce_f32(a, dim3(tiles, a.n_kc, a.n_jobs), s);
@@ -2587,7 +2487,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             forks->put_lists(forks->put_arg, forks->side[1]);
         }
         if (a.lj_full) launch_lj_dense(a, forks->side[1]);
-        else k_lj<float, 0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
+        else k_lj<0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         cudaEventRecord(forks->join[1], forks->side[1]);
         if (!put) real();
@@ -2604,10 +2504,10 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
     cudaStream_t rs = forks->side[0];
     cudaEventRecord(forks->fork, s);
     cudaStreamWaitEvent(rs, forks->fork, 0);
-    launch_ksk<float, 1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
+    launch_ksk<1>(a, dim3(ktiles, a.n_sc, a.n_jobs), rs);
     launch_sk_reduce<1>(a, rs);
-    k_kforce<float, 1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem<float>(a.max_kmax), rs>>>(a);
-    k_real<float, 1><<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
+    k_kforce<1><<<dim3(tiles, a.n_kc, a.n_jobs), FT, kforce_smem(a.max_kmax), rs>>>(a);
+    k_real_d<<<dim3(tiles, a.n_rj, a.n_jobs), RT, 0, s>>>(a);
     cudaEventRecord(forks->join[0], rs);
     cudaStreamWaitEvent(s, forks->join[0], 0);
     k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), CMT, 0, s>>>(a);
@@ -2706,7 +2606,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         else launch_real64(a, s);
     } else if (n == "ksk") {
         if (mixed && ksk2_ok(a)) launch_ksk2(a, s);
-        else if (mixed) launch_ksk<float, 0>(a, gk, s);
+        else if (mixed) launch_ksk<0>(a, gk, s);
         else launch_ksk64(a, s);
     } else if (n == "sk_reduce") {
         if (mixed && a.sk_sites) launch_sk_reduce<2>(a, s);
@@ -2723,7 +2623,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         if (mixed) {
             if (a.lj_full && a.ljf) a.lj_plane = 1;  // as the stepper's forked evaluation
             if (a.lj_full) launch_lj_dense(a, s);
-            else k_lj<float, 0><<<gl, 128, 0, s>>>(a);
+            else k_lj<0><<<gl, 128, 0, s>>>(a);
         } else {
             launch_lj64(a, s);
         }
@@ -2731,7 +2631,7 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
 }
 
 void init_force_kernel_attributes() {
-    set_attrs<float>();
+    set_attrs();
     init_recip32_attributes();
     init_recip64_attributes();
     init_real64_attributes();
