@@ -207,7 +207,7 @@ qtg_status qtg_reset_estimators(qtg_ctx *ctx);
  * that own the GPU memory budget and pass preallocated buffers to their force
  * routines (an allocation of their own would escape that budget or fail under
  * its cap). It calls no cudaMalloc/cudaFree and needs no qtg_ctx: all scratch
- * lives in one static device array of 3.29 MiB (3,453,952 bytes) that every GPU loading the
+ * lives in one static device array of 3.25 MiB (3,404,800 bytes) that every GPU loading the
  * library holds until exit.
  *   sites   device, double[3 n_sites]: charge sites (M, H1, H2 per molecule)
  *   charge  device, double[n_sites]

@@ -12,7 +12,7 @@
 // allocates all of its memory up front.
 //
 // Limits: at most QTG_NOALLOC_MAX_SITES charge sites and k_max <=
-// QTG_NOALLOC_MAX_KMAX; the array is 3.29 MiB (3,453,952 bytes) and every GPU that loads the
+// QTG_NOALLOC_MAX_KMAX; the array is 3.25 MiB (3,404,800 bytes) and every GPU that loads the
 // library holds it until the process exits.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -42,8 +42,7 @@ constexpr size_t OFF_KVEC = OFF_JOB + al256(sizeof(Job));
 constexpr size_t OFF_KCOL = OFF_KVEC + al256(sizeof(KVec) * NA_MAX_K);
 constexpr size_t OFF_KGRP = OFF_KCOL + al256(sizeof(KCol) * NA_COLS);
 constexpr size_t OFF_KBATCH = OFF_KGRP + al256(sizeof(KGroup) * NA_MAX_GRP);
-constexpr size_t OFF_SITES = OFF_KBATCH + al256(sizeof(KBatch) * NA_MAX_BATCH);
-constexpr size_t OFF_PHASE = OFF_SITES + al256(4 * sizeof(double) * NA_MAX_SITES);
+constexpr size_t OFF_PHASE = OFF_KBATCH + al256(sizeof(KBatch) * NA_MAX_BATCH);
 constexpr size_t OFF_SKP = OFF_PHASE + al256(2 * sizeof(double) * 3 * (NA_MAX_KMAX + 1) * NA_MAX_SITES);
 constexpr size_t OFF_WSK = OFF_SKP + al256(2 * sizeof(double) * NA_SC * NA_MAX_K);
 constexpr size_t OFF_PART = OFF_WSK + al256(2 * sizeof(double) * NA_MAX_K);
@@ -57,7 +56,7 @@ constexpr size_t NA_BYTES = OFF_STATUS + 256;
 // stand-in for the symbol: the device address comes from cudaGetSymbolAddress.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 static_assert(NA_MAX_KMAX <= 15, "the packed weights' |kz| needs a shift beyond k_max 15");
-static_assert(NA_BYTES == 3453952, "the scratch size stated in the header and comments is out of date");
+static_assert(NA_BYTES == 3404800, "the scratch size stated in the header and comments is out of date");
 
 constexpr int NA_MAX_DEVICES = 64;
 unsigned char *g_scratch_ptr[NA_MAX_DEVICES] = {nullptr};
@@ -330,7 +329,6 @@ extern "C" qtg_status qtg_kwald_noalloc(const double *sites, const double *charg
     a.kcol = reinterpret_cast<const KCol *>(base + OFF_KCOL);
     a.kgrp = reinterpret_cast<const KGroup *>(base + OFF_KGRP);
     a.kbatch = reinterpret_cast<const KBatch *>(base + OFF_KBATCH);
-    a.sites = base + OFF_SITES;
     a.phase = base + OFF_PHASE;
     a.skp = reinterpret_cast<double2 *>(base + OFF_SKP);
     a.total_k = NA_MAX_K;
