@@ -754,7 +754,7 @@ std::vector<int> step_parts(const qtg_ctx *c) {
 // by FP32 ones. In parts of the systems on streams of their own, one ring update behind the
 // other, a part's forces run beside the next one's ring update and the one before's end
 // step. 48 uneven replicas (277,000 molecule-beads) 2409 us a step in one part, 2350 in two,
-// 2336 in four; 12 (59,000) 583, 571, 529; 4 of 216 waters, 8 beads (6,900), which fill the
+// 2321 in four; 12 (59,000) 583, 571, 525; 4 of 216 waters, 8 beads (6,900), which fill the
 // GPU only together, 91 and 115 in two.
 void enqueue_parts(qtg_ctx *c, const std::vector<int> &lo, int nvt, bool pile_g) {
     const int parts = (int)lo.size() - 1;

@@ -1244,8 +1244,9 @@ __global__ void __launch_bounds__(KT) k_ksk(EvalArgs a) {
 // energy sum_k c_k |S(k)|^2, and the force weights 2 c_k S(k) (MODE 1, the derivative:
 // and 2 c_k dS(k)) for the k-force. One thread per k. Bound by latency: what does not
 // depend on k_ksk is read before the wait for it, and the partials come sixteen (MODEs 1
-// and 2, whose batches are larger: eight) loads at a time (four, resp. one, took 9.9 us at 216 waters, 1 bead against 7.4,
-// resp. 18 us for the derivative of 512 waters, 16 beads).
+// and 2, whose batches are larger: eight) loads at a time. 216 waters, 1 bead, cold caches:
+// 9.9 us with four at a time, 7.4 here; the derivative of 512 waters, 16 beads: 18 us with
+// one at a time, 15 here.
 // MODE 0: k_ksk's partials; MODE 2: k_ksk2's (sixteen loads: 48 uneven replicas 57 us, eight: 42).
 template <int MODE>
 __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
@@ -2531,8 +2532,8 @@ void set_chunks64(EvalArgs &a) {
 
 // An FP64 evaluation: real space | reciprocal chain | short-range terms on parallel
 // streams after the preparation. The first two share the FP64 and integer pipes little, and
-// in a small batch each leaves most of the GPU idle (64 waters, 1 bead: some 31, 48 and
-// 44 us).
+// in a small batch each leaves most of the GPU idle (64 waters, 1 bead: some 17, 43 and
+// 30 us).
 void launch_ewald64(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks *forks) {
     set_chunks64(a);
     a.n_rj = 0;  // no real-space planes: the combine reads the fixed-point sums
