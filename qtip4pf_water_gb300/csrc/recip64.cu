@@ -287,6 +287,15 @@ __global__ void __launch_bounds__(KT64) k_ksk64(EvalArgs a) {
     }
 }
 
+// v 2^(58 - ex) rounded, for |v| < 2^ex, by shifts (an FP64 product and conversion take
+// sixteen cycles of an SM each)
+__device__ __forceinline__ i64 fix58(double v, int ex) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff, s = e - 1017 - ex;
+    const i64 m = (i64)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(v);
+    const i64 u = e == 0 || s < -54 ? 0 : s >= 0 ? m << s : (m + (1ll << (-s - 1))) >> -s;
+    return hi < 0 ? -u : u;
+}
+
 // ---- k_sk_reduce64 --------------------------------------------------------------------
 // A block per force batch (whole columns, at most 128 vectors), a thread per k: S(k) from
 // the site chunks' partials in order, the batch's energy, and the weights W = 2 c_k S(k)
@@ -294,7 +303,9 @@ __global__ void __launch_bounds__(KT64) k_ksk64(EvalArgs a) {
 // of (s.x, d.y, d.x, s.y) and of kz / 2^kshift times (d.x, s.y, s.x, d.y), all over the
 // power of two above the batch's largest |s|, |d|, whose worth goes to wsk[k0]. (kshift
 // keeps kz / 2^kshift below 16 and its sum over a column below 121, so that the limbs
-// and k_kforce64's sums fit; it is 0 for k_max <= 15.)
+// and k_kforce64's sums fit; it is 0 for k_max <= 15.) Bound by FP64 issue, so that only the
+// sums and the weights themselves are FP64 (the packing too: 14.5 us at 216 waters, 32 beads,
+// 10.2 here; 512 waters 18.6 and 10.4).
 __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
     const Job J = a.jobs[blockIdx.y];
     const SysDev &S = a.sys[J.sys];
@@ -303,7 +314,8 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
     const int k = B.k0 + threadIdx.x;
     const bool on = k < B.k1;
     __shared__ double2 wl[128];
-    __shared__ double red[4], top[4];
+    __shared__ double red[4];
+    __shared__ unsigned top[4];
     double e = 0.0;
     int code = -1;
     if (on) {
@@ -329,25 +341,40 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
         dx = wp.x - wm.x;
         dy = wp.y - wm.y;
     }
-    double m = fmax(fmax(fabs(sx), fabs(sy)), fmax(fabs(dx), fabs(dy)));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    // the largest magnitude's exponent, from the high words
+    const auto high = [](double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; };
+    unsigned m = max(max(high(sx), high(sy)), max(high(dx), high(dy)));
+    m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
     const double te = block_sum(e, red);  // (its barriers also publish top)
     if (threadIdx.x == 0) atomicAdd(&a.energy[J.slot], te);
-    m = fmax(fmax(top[0], top[1]), fmax(top[2], top[3]));
-    // m < 2^ex; tiny batches (all weights zero or subnormal) take the smallest scale kept
-    const int ex = max(((__double2hiint(m) >> 20) & 0x7ff) - 1022, -900);
+    m = max(max(top[0], top[1]), max(top[2], top[3]));
+    // every value < 2^ex; tiny batches (all weights zero or subnormal) take the smallest scale kept
+    const int ex = max((int)(m >> 20) - 1022, -900);
     const double scale = __hiloint2double((1023 + ex) << 20, 0), inv = __hiloint2double((1023 - ex) << 20, 0);
     if (threadIdx.x == 0) a.wsk64[J.sk_off + B.k0] = make_double2(scale, 0.0);
     if (code < 0) return;
     int4 *o = reinterpret_cast<int4 *>(a.wpk) + 4 * ((size_t)J.sk_off + B.k0 + (code >> 8));
+    const i64 isx = fix58(sx, ex), isy = fix58(sy, ex);
+    const auto pack = [](i64 re, i64 im) {
+        int4 v;
+        limbs((re + 4) >> 3, v.x, v.y);
+        limbs((im + 4) >> 3, v.z, v.w);
+        return v;
+    };
     if (az == 0) {
-        o[0] = complex_limbs(sx * inv, sy * inv);
+        o[0] = pack(isx, isy);
+        return;
+    }
+    const i64 idx = fix58(dx, ex), idy = fix58(dy, ex);
+    o[0] = pack(isx, idy);
+    o[1] = pack(idx, isy);
+    if (a.kshift == 0) {  // az <= 15
+        o[2] = pack(idx * az, isy * az);
+        o[3] = pack(isx * az, idy * az);
         return;
     }
     const double f = inv * az * __hiloint2double((1023 - a.kshift) << 20, 0);
-    o[0] = complex_limbs(sx * inv, dy * inv);
-    o[1] = complex_limbs(dx * inv, sy * inv);
     o[2] = complex_limbs(dx * f, sy * f);
     o[3] = complex_limbs(sx * f, dy * f);
 }
