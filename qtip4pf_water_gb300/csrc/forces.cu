@@ -2498,9 +2498,13 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
         if (n) *n += 8 + (list_ok(a) ? 2 : 0);
         return;
     }
-    // the derivative: real space beside the reciprocal chain
-    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC);
-    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC);
+    // the derivative: real space beside the reciprocal chain, and both beside the FP64
+    // finite differences, so that few long chunks (two blocks an SM for the structure
+    // factors, eight for the k-force; alone a kernel wants twelve) run best and leave
+    // k_sk_reduce less to add: Suzuki-Chin steps of 512 waters, 16 beads 367 -> 332 us, 216
+    // waters, 32 beads 296 -> 264, 8 beads 187 -> 157, 64 waters, 16 beads 156 -> 127
+    a.n_sc = chunks_or(a.tune_sc, (long long)ktiles * a.n_jobs, MAX_SC, 2);
+    a.n_kc = chunks_or(a.tune_kc, (long long)tiles * a.n_jobs, MAX_KC, 8);
     launch_prep_f32(a, s);
     cudaStream_t rs = forks->side[0];
     cudaEventRecord(forks->fork, s);
