@@ -19,7 +19,8 @@
 // way instead.
 // 216 waters, 32 beads: 3283 us for the all-pairs FP64 form with library functions, 337 us
 // with the same split and the polynomials in FP64 (37 FP64 instructions a pair), 121 us here
-// (512 waters, 32 beads: 1228 us in FP64 arithmetic, 442 here). Eight sites a warp run the
+// (143 with the fewer blocks that launch_real64 gives it for the sake of the kernels beside
+// it; 512 waters, 32 beads: 1228 us in FP64 arithmetic, 442 here, 498 so). Eight sites a warp run the
 // kernel alone 11 % faster but the FP64 steps and calls, where it shares the GPU, no faster.
 // The error against 80-bit sums is below the FP64 form's: 2.2e-15 of the real-space forces
 // against 3.8e-15 at 64 waters, 1.2e-15 against 3.4e-15 at 216, 0.9e-15 against 6.5e-15 at 512.
@@ -357,11 +358,13 @@ void init_real64_attributes() {
     cudaFuncSetAttribute(k_real64, cudaFuncAttributeMaxDynamicSharedMemorySize, RW * (int)sizeof(RWarp));
 }
 
-// Chunks of ring distances: enough blocks for a few waves of the six that fit an SM, so
-// that small beads spread over the GPU and the last wave is short.
+// Chunks of ring distances: some eight blocks an SM, about a wave. More and shorter ones
+// keep their slots from the kernels beside this one (with twenty-four: a Suzuki-Chin call of
+// 216 waters, 8 beads 407 us against 390, FP64 forces of 336 waters, 8 beads 281 against 267, a
+// step of 216 waters, 32 beads 411 against 398; with four the last two 284 and 409).
 void launch_real64(const EvalArgs &a, cudaStream_t s) {
     const int T = (3 * a.max_mols + 31) / 32;
-    const long long blocks = (long long)T * a.n_jobs, want = 152LL * 24;
+    const long long blocks = (long long)T * a.n_jobs, want = 152LL * 8;
     int n_ch = a.tune_rj > 0 ? a.tune_rj : (int)std::min<long long>(MAX_RJ, (want + blocks - 1) / blocks);
     n_ch = std::max(1, std::min(n_ch, T / 2 + 1));
     k_real64<<<dim3(T, n_ch, a.n_jobs), 32 * RW, RW * sizeof(RWarp), s>>>(a, n_ch);
