@@ -2385,7 +2385,9 @@ void launch_real_half(EvalArgs &a, cudaStream_t s) {
     const int T2 = (3 * a.max_mols + 63) / 64, units = half_units(T2);
     if ((long long)T2 * units * a.n_jobs >= 152LL * 16) {
         const int gx = (T2 + HW - 1) / HW;
-        int n_ch = chunks_or(a.tune_rj, (long long)gx * a.n_jobs, units, 20);
+        // (ten blocks an SM: 512 waters, 32 beads 192.5 us a step, 48 replicas 2300; with twenty
+        // 195.5 and 2324, with seven 194.7 and 2298)
+        int n_ch = chunks_or(a.tune_rj, (long long)gx * a.n_jobs, units, 10);
         if (a.tune_rj <= 0) {  // whole units: as many chunks as hold units / n_ch (rounded) each
             const int per = std::max(1, (units + n_ch / 2) / n_ch);
             n_ch = (units + per - 1) / per;
@@ -2427,11 +2429,12 @@ bool ksk2_ok(const EvalArgs &a) {
            (long long)a.max_mols * a.n_jobs >= 2048;
 }
 // Its site chunks, of the same size for every system of the batch: at most 192 sites, and
-// about a block an SM (the real-space kernel runs beside it). 512 waters, 32 beads: 8 chunks
-// 199.5 us a step, 16 chunks 201.0; 343 waters, 16 beads: 8 chunks 104.5, 28 chunks 110.8.
+// about two blocks an SM (the real-space kernel runs beside it). 512 waters, 32 beads: one
+// an SM 195.5 us a step, two 193.2, three 196.8; 343 waters, 16 beads: 99.0, 95.3, 93.4; 216
+// waters, 32 beads: 95.3, 93.9, 96.9.
 void set_ksk2_chunks(EvalArgs &a) {
     const int ns = 3 * a.max_mols;
-    a.n_sc = std::max(chunks_or(a.tune_sc, (long long)ksk2_blocks(a) * a.n_jobs, MAX_SC2, 1), (ns + 191) / 192);
+    a.n_sc = std::max(chunks_or(a.tune_sc, (long long)ksk2_blocks(a) * a.n_jobs, MAX_SC2, 2), (ns + 191) / 192);
     a.sk_sites = std::max(16, ((ns + a.n_sc - 1) / a.n_sc + 15) / 16 * 16);
     a.n_sc = (ns + a.sk_sites - 1) / a.sk_sites;
 }
