@@ -2431,10 +2431,13 @@ bool ksk2_ok(const EvalArgs &a) {
 // Its site chunks, of the same size for every system of the batch: at most 192 sites, and
 // about two blocks an SM (the real-space kernel runs beside it). 512 waters, 32 beads: one
 // an SM 195.5 us a step, two 193.2, three 196.8; 343 waters, 16 beads: 99.0, 95.3, 93.4; 216
-// waters, 32 beads: 95.3, 93.9, 96.9.
+// waters, 32 beads: 95.3, 93.9, 96.9. A batch that fills the SMs with whole beads keeps
+// them whole.
 void set_ksk2_chunks(EvalArgs &a) {
     const int ns = 3 * a.max_mols;
-    a.n_sc = std::max(chunks_or(a.tune_sc, (long long)ksk2_blocks(a) * a.n_jobs, MAX_SC2, 2), (ns + 191) / 192);
+    const long long base = (long long)ksk2_blocks(a) * a.n_jobs, two = 2 * 152;
+    const int n_sc = a.tune_sc > 0 ? a.tune_sc : (int)std::max(1LL, (two + base / 2) / base);  // (to the nearest)
+    a.n_sc = std::max(std::min(n_sc, MAX_SC2), (ns + 191) / 192);
     a.sk_sites = std::max(16, ((ns + a.n_sc - 1) / a.n_sc + 15) / 16 * 16);
     a.n_sc = (ns + a.sk_sites - 1) / a.sk_sites;
 }
