@@ -78,10 +78,10 @@ inline void set_charge_scale(SysDev &S, const double *charge, int n) {
     double top = 0.0, s = 1.0;
     for (int i = 0; i < n; ++i) top = charge[i] > top ? charge[i] : -charge[i] > top ? -charge[i] : top;
     while (s < top && s < 1e300) s *= 2.0;
-    while (top > 0.0 && 0.5 * s >= top) s *= 0.5;
+    while (top > 0.0 && 0.5 * s >= top && s > 1e-300) s *= 0.5;
     S.q_scale = s;
     S.inv_q_scale = 1.0 / s;
-    S.q_top = top > 0.0 ? top * (1.0 + 1e-6) : 1.0;
+    S.q_top = top > 1e-300 ? top * (1.0 + 1e-6) : 1.0;
     S.inv_q_top = 1.0 / S.q_top;
 }
 

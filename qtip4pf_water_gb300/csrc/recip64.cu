@@ -180,8 +180,10 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
 // Ar Zr, Ai Zi, Ar Zi, Ai Zr, from which S(+kz) = T1 - T2 + i (T3 + T4) and S(-kz) =
 // T1 + T2 + i (T4 - T3). Sites come through shared memory in chunks of CH64, double-
 // buffered by cp.async; mid holds CARRY chunks before its high part moves into hh, and
-// hh FLUSH chunks (512 sites) before it goes to FP64.
-constexpr int KT64 = 128, CH64 = 32, CARRY = 4, FLUSH = 16;
+// hh FLUSH chunks (256 sites) before it goes to FP64: a high limb reaches 2^27 (a scaled
+// charge within 2^-28 of 1), so 512 sites in phase would make 2^63.
+constexpr int KT64 = 128, CH64 = 32, CARRY = 4, FLUSH = 8;
+static_assert((long long)FLUSH * CH64 << 54 <= 1ll << 62, "k_ksk64's high sums overflow");
 
 __device__ __forceinline__ void copy16(void *dst, const void *src, bool valid) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
