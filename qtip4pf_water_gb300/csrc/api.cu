@@ -241,6 +241,7 @@ struct qtg_ctx {
     double *real64_tab = nullptr;  // FP64: the real-space pair-function table
     long long *real64_int = nullptr, *real64_sys = nullptr;  // its fixed-point form; constants per system
     float4 *sites32 = nullptr;     // FP64: wrapped FP32 charge sites
+    int *nonfinite = nullptr;      // FP64: sites that are not finite, a word per slot and preparation block
     // real-space pair list (mixed contexts with beads beyond the half-interaction
     // kernel in boxes with r_c + 2 RL_SPREAD <= L/2): rl_ok marks the context
     // eligible, rl_form 0 runs the real space over the list there, 1 over all pairs
@@ -420,6 +421,7 @@ EvalArgs eval_args(qtg_ctx *c, const Job *jobs, int n_jobs, const double *pos, d
     a.real64_int = c->real64_int;
     a.real64_sys = c->real64_sys;
     a.sites32 = c->sites32;
+    a.nonfinite = c->nonfinite;
     a.opos = c->opos;
     a.opos32 = c->opos32;
     a.lj64 = c->lj64;
@@ -1507,6 +1509,7 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         AL(ctx->real64_int, (size_t)RI_OCT * 64 * 12);
         AL(ctx->real64_sys, 4 * (size_t)n_systems);
         AL(ctx->sites32, ctx->total_sites);
+        AL(ctx->nonfinite, ctx->total_slots * 3 * ((3 * (size_t)ctx->max_mols + 127) / 128));
     }
     {
         // real-space pair list: rows hold the molecules whose M sites lie within
@@ -1672,7 +1675,7 @@ void qtg_destroy(qtg_ctx *ctx) {
                     ctx->sc_bead, ctx->colwork, ctx->acc, ctx->run, ctx->est, ctx->step, ctx->records,
                     ctx->status, ctx->red_out, ctx->rebuilt, ctx->cw_part, ctx->cw_ticket, ctx->kpk, ctx->ljf, ctx->fin_ticket, ctx->sites_fix, ctx->intra, ctx->kfc, ctx->kfb, ctx->wpk,
                     ctx->wpos, ctx->cnt_half, ctx->cnt_full, ctx->cell_start, ctx->cell_mol,
-                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->real64_int, ctx->real64_sys, ctx->sites32, ctx->kpair, ctx->opos32, ctx->lj64, ctx->intra64};
+                    ctx->rb_jobs, ctx->rb_count, ctx->rl_list, ctx->rl_cnt, ctx->rl_ref, ctx->rl_jobs, ctx->rl_count, ctx->rl_wide, ctx->rl_state, ctx->rfix, ctx->real64_tab, ctx->real64_int, ctx->real64_sys, ctx->sites32, ctx->nonfinite, ctx->kpair, ctx->opos32, ctx->lj64, ctx->intra64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->box) cudaFreeHost(ctx->box);

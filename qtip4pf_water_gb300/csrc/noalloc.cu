@@ -50,7 +50,9 @@ constexpr size_t OFF_WPK = OFF_PART + al256(3 * sizeof(double) * NA_KC * NA_MAX_
 constexpr size_t OFF_KPK = OFF_WPK + al256(4 * sizeof(int4) * NA_MAX_K);
 constexpr size_t OFF_KFC = OFF_KPK + al256(sizeof(int) * NA_MAX_K);
 constexpr size_t OFF_STATUS = OFF_KFC + al256(sizeof(int4) * NA_COLS);
+constexpr size_t OFF_NONFINITE = OFF_STATUS + 64;  // k_prep64's words, one a block
 constexpr size_t NA_BYTES = OFF_STATUS + 256;
+static_assert(3 * ((NA_MAX_SITES + 127) / 128) * sizeof(int) <= 192, "k_prep64's words fit beside the status word");
 
 // All scratch of qtg_kwald_noalloc. In host code this name is only a host-side
 // stand-in for the symbol: the device address comes from cudaGetSymbolAddress.
@@ -213,7 +215,8 @@ __global__ void __launch_bounds__(512) k_noalloc_setup(NAParams p, const double 
         }
         SysDev S = p.S;
         for (int k = 0; k < 16; ++k) qm = fmax(qm, top[k]);
-        const int ex = qm > 0.0 ? ((__double2hiint(qm) >> 20) & 0x7ff) - 1022 : 0;  // qm < 2^ex
+        // qm < 2^ex, kept where 2^-ex is a normal number too
+        const int ex = qm > 0.0 ? max(-1000, min(((__double2hiint(qm) >> 20) & 0x7ff) - 1022, 1000)) : 0;
         S.q_scale = __hiloint2double((1023 + ex) << 20, 0);
         S.inv_q_scale = __hiloint2double((1023 - ex) << 20, 0);
         S.n_kvec = nk;
@@ -337,6 +340,7 @@ extern "C" qtg_status qtg_kwald_noalloc(const double *sites, const double *charg
     a.kpk = reinterpret_cast<const int *>(base + OFF_KPK);
     a.kfc = reinterpret_cast<const int4 *>(base + OFF_KFC);
     a.kshift = 0;  // k_max <= 15
+    a.nonfinite = reinterpret_cast<int *>(base + OFF_NONFINITE);
     a.part = reinterpret_cast<double *>(base + OFF_PART);
     a.total_sites = NA_MAX_SITES;
     a.energy = energy;

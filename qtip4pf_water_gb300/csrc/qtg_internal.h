@@ -567,6 +567,7 @@ struct EvalArgs {
     double2 *dskp;         // partial dS(k) along the tangent direction
     void *wsk, *wdsk;      // mixed: 2 c_k S(k) and 2 c_k dS(k), per slot
     double2 *wsk64;        // FP64: per force batch (at its first k) the worth of its packed weights' unit
+    int *nonfinite;        // FP64: per slot and block of k_prep64, whether it met a site that is not finite
     int kshift;            // FP64: the packed |kz|-weighted force weights carry kz / 2^kshift
     long long total_k;     // k-vectors summed over all slots (plane stride of skp)
     double *energy;        // per slot

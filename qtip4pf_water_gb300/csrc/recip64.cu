@@ -104,6 +104,9 @@ __device__ __forceinline__ int4 turn_limbs(unsigned long long a) {
     return o;
 }
 
+__device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+__host__ __device__ __forceinline__ int prep64_blocks(int max_mols) { return 3 * ((3 * max_mols + 127) / 128); }
+
 // ---- k_prep64 -----------------------------------------------------------------------
 // One thread per (site, dimension), blocks dimension-major as k_prep_f32: charge site
 // (M, H1, H2) wrapped into the box in k_real64's fixed point, wrapped oxygen, zeroed sums, and the site's row of
@@ -112,6 +115,9 @@ __device__ __forceinline__ int4 turn_limbs(unsigned long long a) {
 // limbs. The x row carries the charge over q_scale. (With the FP64 sincospi the kernel was
 // bound by its FP64 instructions: 216 waters, 32 beads 30 us, 14.4 here; 64 waters, 1 bead,
 // all latency, 12.4 and 8.3. The force's error against 80-bit sums falls from 2.0e-15 to 6.4e-16.)
+// Fixed point has no NaN: a block that met a coordinate or charge that is not finite says so
+// in its word of a.nonfinite, from which k_sk_reduce64 makes the whole configuration's
+// reciprocal energy and forces NaN, as sums of such phases are.
 __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
     const Job J = a.jobs[blockIdx.y];
     const SysDev &S = a.sys[J.sys];
@@ -119,12 +125,12 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
     const int tiles = (3 * a.max_mols + 127) / 128;
     const int d = blockIdx.x / tiles, s = (blockIdx.x - d * tiles) * 128 + threadIdx.x;
     if (s == 0 && d == 0) a.energy[J.slot] = 0.0;
-    if (s >= ns) return;
     const int mol = s / 3, kind = s - 3 * mol;
     const double *q = a.pos + J.pos_off;
     const double g = a.c.gamma_vs;
-    double x;
-    if (a.sites_are_input || kind != 0) {
+    double x = 0.0;
+    if (s >= ns) {
+    } else if (a.sites_are_input || kind != 0) {
         x = q[3 * s + d];
     } else {
         // M site (forces.cpp:558-564)
@@ -134,6 +140,10 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
         reinterpret_cast<float *>(a.opos32)[at] = (float)((t - floor(t)) * S.box[d]);
         a.lj64[at] = 0.0;  // k_lj64's forces
     }
+    const double chg = d == 0 && s < ns ? a.charge[S.chg_off + s] : 0.0;
+    const int bad = __syncthreads_or(not_finite(x) || not_finite(chg));
+    if (threadIdx.x == 0) a.nonfinite[(size_t)J.slot * gridDim.x + blockIdx.x] = bad;
+    if (s >= ns) return;
     // wrapped with one rounding (while the quotient is exact enough for it), and the 64-bit
     // fraction of the box
     const double t = x * S.inv_box[d];
@@ -141,7 +151,6 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
     const double fh = wr * S.inv_box[d], fl = fma(-fh, S.box[d], wr) * S.inv_box[d];
     const unsigned long long frac = ((unsigned long long)__double2ll_rn(fh * 4611686018427387904.0) << 2) +
                                     (unsigned long long)__double2ll_rn(fl * 18446744073709551616.0);
-    const double chg = d == 0 ? a.charge[S.chg_off + s] : 0.0;
     if (a.sites32) {  // k_real64's form of the site (reciprocal space alone may have none)
         i64 *sv = reinterpret_cast<i64 *>(a.sites) + 4 * ((size_t)J.site_off + s);
         sv[d] = kappa_fix(S.kappa, wr);
@@ -320,6 +329,9 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
     __shared__ unsigned top[4];
     double e = 0.0;
     int code = -1;
+    bool bad = false;  // a site of the configuration is not finite (k_prep64)
+    const int words = prep64_blocks(a.max_mols);
+    for (int i = threadIdx.x; i < words; i += 128) bad |= a.nonfinite[(size_t)J.slot * words + i] != 0;
     if (on) {
         const KVec kv = a.kvec[S.kvec_off + k];
         const double w = 2.0 * kv.coef * (kv.twin ? 2.0 : 1.0);  // kx = 0, ky > 0: its conjugate partner too
@@ -333,7 +345,9 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
         wl[threadIdx.x] = make_double2(w * sr, w * si);
         code = a.kpk[S.kvec_off + k];
     }
-    __syncthreads();
+    const double nan = __hiloint2double(0x7ff80000, 0);
+    bad = __syncthreads_or(bad);
+    if (bad) e = nan;
     const int az = code & 255;
     double sx = 0.0, sy = 0.0, dx = 0.0, dy = 0.0;
     if (code >= 0) {
@@ -354,7 +368,7 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
     // every value < 2^ex; tiny batches (all weights zero or subnormal) take the smallest scale kept
     const int ex = max((int)(m >> 20) - 1022, -900);
     const double scale = __hiloint2double((1023 + ex) << 20, 0), inv = __hiloint2double((1023 - ex) << 20, 0);
-    if (threadIdx.x == 0) a.wsk64[J.sk_off + B.k0] = make_double2(scale, 0.0);
+    if (threadIdx.x == 0) a.wsk64[J.sk_off + B.k0] = make_double2(bad ? nan : scale, 0.0);
     if (code < 0) return;
     int4 *o = reinterpret_cast<int4 *>(a.wpk) + 4 * ((size_t)J.sk_off + B.k0 + (code >> 8));
     const i64 isx = fix58(sx, ex), isy = fix58(sy, ex);
@@ -485,8 +499,7 @@ void init_recip64_attributes() {
 }
 
 void launch_prep64(const EvalArgs &a, cudaStream_t s) {
-    const int tiles = (3 * a.max_mols + 127) / 128;
-    k_prep64<<<dim3(3 * tiles, a.n_jobs), 128, 0, s>>>(a);
+    k_prep64<<<dim3(prep64_blocks(a.max_mols), a.n_jobs), 128, 0, s>>>(a);
 }
 // 216 waters, 32 beads: 430 us with FP64 multiply-adds, 99 us here; 512 waters: 309 us.
 // Against a long-double sum the forces are as near as before (64 waters: 2.0e-15 and
