@@ -192,14 +192,15 @@ __device__ __noinline__ double slow_pair(const EvalArgs &a, const SysDev &S, i64
 __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     RWarp &W = reinterpret_cast<RWarp *>(smem_raw)[threadIdx.x >> 5];
-    __shared__ i64 image[3][4];  // n kappa L_d at n + 1
+    __shared__ i64 image[3][4];  // n kappa L_d at n + 1, n = -1 .. 1; kappa L_d / 2 at 3
     const int lane = threadIdx.x & 31;
     const Job J = a.jobs[blockIdx.z];
     const SysDev &S = a.sys[J.sys];
     const i64 *sysc = a.real64_sys + 4 * J.sys;
     if (threadIdx.x < 12) {
         const int d = threadIdx.x >> 2, n = (threadIdx.x & 3) - 1;
-        image[d][n + 1] = n * sysc[d];
+        // (sides that r_c does not reach across need no second image, see below)
+        image[d][n + 1] = n < 2 ? n * sysc[d] : S.kappa * S.box[d] < 64.0 ? sysc[d] >> 1 : 0x7fffffffffffffffll;
     }
     __syncthreads();
     const int ns = S.n_sites, T = (ns + 31) / 32, tI = blockIdx.x;
@@ -273,10 +274,20 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
         for (int b = lane; b < cnt; b += 32) {
             const int c = W.code[b], img = c >> 9;
             const RSite &p = W.si[(c >> 5) & 15], &s = W.sj[c & 31];
-            const i64 y0 = p.y[0] - s.y[0] - image[0][img & 3], y1 = p.y[1] - s.y[1] - image[1][(img >> 2) & 3],
-                      y2 = p.y[2] - s.y[2] - image[2][(img >> 4) & 3];
+            i64 y0 = p.y[0] - s.y[0] - image[0][img & 3], y1 = p.y[1] - s.y[1] - image[1][(img >> 2) & 3],
+                y2 = p.y[2] - s.y[2] - image[2][(img >> 4) & 3];
             // u in units of 2^-56; a fixed-point pair has u in [2^RI_LO, 2^(RI_LO + RI_OCT))
-            const i64 u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
+            i64 u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
+            if (u >= uc) {
+                // beyond r_c: the screen's FP32 image of a pair some 1e-7 of a side from half
+                // a box may be the farther one, and r_c reaches half the shortest side (the
+                // screen's margin lets in one pair in 10^5 that comes here)
+                const auto nearer = [](i64 y, const i64 *im) { return y > im[3] ? y - im[2] : y < -im[3] ? y + im[2] : y; };
+                y0 = nearer(y0, image[0]);
+                y1 = nearer(y1, image[1]);
+                y2 = nearer(y2, image[2]);
+                u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
+            }
             i64 fx = 0, fy = 0, fz = 0;
             if (u < uc && (unsigned)((int)(u >> 32) - RI_BOT) < (unsigned)(RI_TOP - RI_BOT)) {
                 const int z = __clz((int)(u >> 32));

@@ -58,3 +58,21 @@ def test_edges_of_the_fixed_point_form(gpu_lib, eps, gap):
     ref, got, e_ref, e_got = _forces(q, 27, 1, st.box_bohr, pos, eps)
     assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
     assert abs(e_got - e_ref) < 1e-9 * max(1.0, abs(e_ref))
+
+
+# r_c is half the side of boxes of this size: an H of another molecule just inside it along
+# one axis, where FP32 cannot tell the nearer image
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("gap", [1e-9, 1e-8, 3e-8])
+def test_pair_at_half_a_side(gpu_lib, axis, gap):
+    q = gpu_lib
+    st = q.seeded_start(8, 1, 298.0, seed=9, density_g_cm3=0.2)
+    for k in range(24):
+        pos = np.ascontiguousarray(st.q).copy()
+        i, j = k % 8, (k + 1 + k // 8) % 8
+        x = pos.reshape(8, 3, 3)
+        x[j] += x[i, 1] - x[j, 1]
+        x[j, :, axis] += (1.0 if k % 2 else -1.0) * (0.5 - gap) * st.box_bohr[axis]
+        ref, got, e_ref, e_got = _forces(q, 8, 1, st.box_bohr, pos, 1e-4)
+        assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
+        assert abs(e_got - e_ref) < 1e-9 * max(1.0, abs(e_ref))
