@@ -814,9 +814,11 @@ __global__ void __launch_bounds__(32 * HW) k_real_half(EvalArgs a, int n_ch) {
 //
 // What bounds it is instruction issue (two thirds of the pairs lie beyond r_c and cost
 // the same). The two pairs of a step share the visited site's load and its accumulators'
-// shuffles, and their arithmetic is packed (fma / mul .f32x2): 35 issue slots a pair,
-// 51 with one site a lane; the scalar form of the same loop has 45 and is 5 % slower, as
-// a packed instruction holds its port for two slots. 512 waters, 32 beads: 70.0 -> 59.6 us.
+// shuffles, and their arithmetic is packed (fma / mul .f32x2): 37 issue slots a pair,
+// 51 with one site a lane; the scalar form of the same loop has some 45 and is 5 % slower, as
+// a packed instruction holds its port for two slots. 512 waters, 32 beads: 70.0 -> 61.5 us
+// (59.4 with both pairs multiplied straight onto the visited site's sum, whose 64 roundings
+// a visit were twice k_real_half's).
 // 1 where a < b, else 0
 __device__ __forceinline__ float below(float a, float b) {
     float r;
@@ -884,12 +886,14 @@ __device__ __forceinline__ void half_visit(const int4 *vr, const int4 &a, const 
         fz = fma2(w, dz, fz);
         float wa, wb, da, db;
         unpk(w, wa, wb);
+        // (the two pairs' forces are added first: 32 roundings of a visited site's sum a
+        // visit, as with one site a lane)
         unpk(dx, da, db);
-        mx = fmaf(-wa, da, fmaf(-wb, db, mx));
+        mx -= fmaf(wa, da, __fmul_rn(wb, db));
         unpk(dy, da, db);
-        my = fmaf(-wa, da, fmaf(-wb, db, my));
+        my -= fmaf(wa, da, __fmul_rn(wb, db));
         unpk(dz, da, db);
-        mz = fmaf(-wa, da, fmaf(-wb, db, mz));
+        mz -= fmaf(wa, da, __fmul_rn(wb, db));
         mx = __shfl_sync(0xffffffffu, mx, nx);
         my = __shfl_sync(0xffffffffu, my, nx);
         mz = __shfl_sync(0xffffffffu, mz, nx);
@@ -941,7 +945,7 @@ __global__ void __launch_bounds__(32 * HW) k_real_half2(EvalArgs a, int n_ch) {
         w = qq * fmaf(K.pref, ex, A) * (iv * iv);
         return qq * A;
     };
-    float Fa[3] = {0.f, 0.f, 0.f}, Fb[3] = {0.f, 0.f, 0.f}, Ca[3] = {0.f, 0.f, 0.f}, Cb[3] = {0.f, 0.f, 0.f}, e = 0.f;
+    float Fa[3] = {0.f, 0.f, 0.f}, Fb[3] = {0.f, 0.f, 0.f}, Ca[3] = {0.f, 0.f, 0.f}, Cb[3] = {0.f, 0.f, 0.f}, e = 0.f, ce = 0.f;
     for (int u = u0; u < u1; ++u) {
         if (u == 1) continue;  // (part of visit 0)
         const int v = u ? u - 1 : 0, d = (v + 1) >> 1, half = v ? (v - 1) & 1 : 0;
@@ -1051,8 +1055,9 @@ __global__ void __launch_bounds__(32 * HW) k_real_half2(EvalArgs a, int n_ch) {
             kahan_add(Fa[k], Ca[k], fa[k] * fscale);
             kahan_add(Fb[k], Cb[k], fb[k] * fscale);
         }
-        e = fmaf(ev, escale, e);
+        kahan_add(e, ce, ev * escale);
     }
+    e -= ce;
     if (va) rfix_add(a.rfix + 3 * ((size_t)J.site_off + sa), Fa[0] - Ca[0], Fa[1] - Ca[1], Fa[2] - Ca[2]);
     if (vb) rfix_add(a.rfix + 3 * ((size_t)J.site_off + sb), Fb[0] - Cb[0], Fb[1] - Cb[1], Fb[2] - Cb[2]);
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
@@ -2376,7 +2381,7 @@ void launch_lj_dense(const EvalArgs &a, cudaStream_t s) {
 // The half-interaction real-space kernels apply to beads of at most HALF_MAX_TILES tiles
 // of 32 sites. Two sites a lane where that leaves some 16 warps an SM with one work unit
 // each: 216 waters, 32 beads (4224 warps) 27.1 -> 26.8 us, 512 waters, 32 beads 70.0 ->
-// 59.6 us. Smaller batches leave SMs idle either way, and the shorter chains of one
+// 61.5 us. Smaller batches leave SMs idle either way, and the shorter chains of one
 // site a lane end sooner: 216 waters, 1 bead 15.3 us against 16.5 us.
 bool half_ok(const EvalArgs &a) { return (3 * a.max_mols + 31) / 32 <= HALF_MAX_TILES; }
 void launch_real_half(EvalArgs &a, cudaStream_t s) {
