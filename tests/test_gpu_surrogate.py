@@ -148,3 +148,27 @@ def test_adam_training_reduces_the_loss(gpu_lib):
                     3e-3, dev.wbf.data_ptr(), q.MLP_NW)
     assert q.surrogate_status() == 0
     assert losses[1] < 0.2 * losses[0], losses
+
+
+# the training kernel's own forward pass is the forward kernel's to the bit: with that kernel's
+# outputs as targets nothing is left to learn (one ragged tile, one tile a CTA, several)
+@pytest.mark.parametrize("m", [100, 20000, 100001])
+def test_training_forward_is_the_forward_pass(gpu_lib, m):
+    torch = _torch()
+    q = gpu_lib
+    rng = np.random.default_rng(m)
+    p = so.init_params(5)
+    for k in ("b1", "b2", "b3"):
+        p[k] = rng.standard_normal(p[k].shape) * 0.5
+    p["b3"][9:] = 0.0
+    dev = _weights(torch, p)
+    x = (2.0 * torch.randn((m, 96), device="cuda", generator=torch.Generator(device="cuda").manual_seed(m))).to(torch.bfloat16)
+    w = q.MlpWeights(*[dev[k].data_ptr() for k in ("w1", "w2", "w3", "b1", "b2", "b3")])
+    y = torch.zeros((m, 16), device="cuda")
+    q.mlp_forward(w, x.data_ptr(), m, y.data_ptr())
+    part = torch.zeros((512, q.MLP_NPARAMS + 1), device="cuda")
+    grad = torch.full((q.MLP_NPARAMS + 1,), float("nan"), device="cuda")
+    q.mlp_train_batch(w, x.data_ptr(), y.data_ptr(), m, 1.0, part.data_ptr(), 512, grad.data_ptr())
+    assert q.surrogate_status() == 0
+    assert float(y[:, :9].abs().max()) > 0.1
+    assert bool((grad == 0).all())
