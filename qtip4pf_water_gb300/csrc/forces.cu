@@ -1856,8 +1856,8 @@ __global__ void __launch_bounds__(CMT) k_combine_f32(EvalArgs a) {
             fi[k] = in[3 * k];
             fa[k] = in[9 + 3 * k];
         }
-        if (a.lj_plane) lj = (double)reinterpret_cast<const float *>(a.ljf + mol)[d];
-        else if (a.lj_half) lj = a.lj64[4 * mol + d];
+        if (a.lj_full) lj = (double)reinterpret_cast<const float *>(a.ljf + mol)[d];
+        else lj = a.lj64[4 * mol + d];
     }
     if (o < 9 * nm) {
         const int np = a.n_rj + a.n_kc;
@@ -1894,7 +1894,7 @@ __global__ void __launch_bounds__(CMT) k_combine_f32(EvalArgs a) {
     }
 }
 
-// ---- k_lj: O-O Lennard-Jones over the Verlet list (forces.cpp:489-515) -----------
+// ---- k_lj: O-O Lennard-Jones over the caller's Verlet list (forces.cpp:489-515), mixed --
 // One warp per CSR row; lanes over the row's entries. The pair's displacement
 // and the cutoff decision r^2 < r_cut^2 must be the reference's (FP64,
 // x - L*round(x/L) with a true division and round-half-away-from-zero, each
@@ -1902,7 +1902,6 @@ __global__ void __launch_bounds__(CMT) k_combine_f32(EvalArgs a) {
 // relative band around r_cut^2, or whose separation is within rounding of
 // half a box in some dimension (where the two images tie and the rounding rule
 // picks the sign), is recomputed with exactly that arithmetic.
-template <int FULL>
 __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     const int jb = blockIdx.y;
     const Job J = a.jobs[jb];
@@ -1917,19 +1916,14 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
     const double rc2 = C.r_cut_sq;
     const float rc2r = (float)rc2;
     const float bandr = (float)1e-5, tie = (float)1e-5;
-    // half list: rows 0..N-2, entries j > i, forces on j by atomics; symmetric
-    // list (FULL): rows 0..N-1, entries j != i, each pair seen from both ends, so
-    // a row's force needs no atomics and the energy is halved
-    if (i < (FULL ? N : N - 1)) {
+    // half list: rows 0..N-2, entries j > i, forces on both by atomics into their own array
+    // (zeroed by k_prep_f32, read by k_combine_f32: the kernel runs beside the others)
+    if (i < N - 1) {
         const double *q = a.pos + J.pos_off;
-        // the forces, or their own array (lj_half: the kernel runs beside the others)
-        double *f = !FULL && a.lj_half ? a.lj64 + 4 * ((size_t)J.site_off / 3) : a.out + J.out_off;
-        const int fs = !FULL && a.lj_half ? 4 : 9;
-        const int cap = FULL ? 2 * S.list_size : S.list_size;
-        const int *pt = FULL ? a.point_full + S.pf_off + (size_t)J.bead * (N + 1)
-                             : a.point + S.pt_off + (size_t)J.bead * N;
-        const int *ls = FULL ? a.list_full + S.lf_off + (size_t)J.bead * cap
-                             : a.list + S.ls_off + (size_t)J.bead * S.list_size;
+        double *f = a.lj64 + 4 * ((size_t)J.site_off / 3);
+        const int cap = S.list_size;
+        const int *pt = a.point + S.pt_off + (size_t)J.bead * N;
+        const int *ls = a.list + S.ls_off + (size_t)J.bead * cap;
         // a row outside [0, capacity] (overflowed or caller-corrupted list) or an index
         // outside the row's range is skipped and flagged instead of being read out of bounds
         int n0 = pt[i], n1 = pt[i + 1];
@@ -1948,7 +1942,7 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
         float fi0 = 0, fi1 = 0, fi2 = 0, el = 0;
         for (int n = n0 + lane; n < n1; n += 32) {
             const int j = ls[n];
-            if ((FULL ? j == i : j <= i) || j < 0 || j >= N) {
+            if (j <= i || j >= N) {
                 atomicOr(a.status, (unsigned)ST_LIST_OVERFLOW);
                 continue;
             }
@@ -1983,27 +1977,17 @@ __global__ void __launch_bounds__(128) k_lj(EvalArgs a) {
                 fi0 += ff * r[0];
                 fi1 += ff * r[1];
                 fi2 += ff * r[2];
-                if (!FULL) {
-                    atomicAdd(&f[fs * j], -(double)(ff * r[0]));
-                    atomicAdd(&f[fs * j + 1], -(double)(ff * r[1]));
-                    atomicAdd(&f[fs * j + 2], -(double)(ff * r[2]));
-                }
+                atomicAdd(&f[4 * j], -(double)(ff * r[0]));
+                atomicAdd(&f[4 * j + 1], -(double)(ff * r[1]));
+                atomicAdd(&f[4 * j + 2], -(double)(ff * r[2]));
             }
         }
         const double d0 = warp_sum((double)fi0), d1 = warp_sum((double)fi1), d2 = warp_sum((double)fi2);
-        e = warp_sum((double)el) * (FULL ? 0.5 : 1.0);
+        e = warp_sum((double)el);
         if (lane == 0) {
-            if (FULL && a.lj_plane) {  // the mixed combine adds the oxygen force
-                a.ljf[J.site_off / 3 + i] = make_float4((float)d0, (float)d1, (float)d2, 0.f);
-            } else if (FULL) {
-                f[9 * i] += d0;
-                f[9 * i + 1] += d1;
-                f[9 * i + 2] += d2;
-            } else {
-                atomicAdd(&f[fs * i], d0);
-                atomicAdd(&f[fs * i + 1], d1);
-                atomicAdd(&f[fs * i + 2], d2);
-            }
+            atomicAdd(&f[4 * i], d0);
+            atomicAdd(&f[4 * i + 1], d1);
+            atomicAdd(&f[4 * i + 2], d2);
         } else {
             e = 0.0;
         }
@@ -2160,14 +2144,7 @@ __global__ void __launch_bounds__(128) k_lj_dense(EvalArgs a) {
     }
     float e = 0.f;
     if (act && sub == 0) {
-        if (a.lj_plane) {
-            a.ljf[J.site_off / 3 + i] = make_float4(fx, fy, fz, 0.f);
-        } else {
-            double *f = a.out + J.out_off;
-            f[9 * i] += (double)fx;
-            f[9 * i + 1] += (double)fy;
-            f[9 * i + 2] += (double)fz;
-        }
+        a.ljf[J.site_off / 3 + i] = make_float4(fx, fy, fz, 0.f);
         e = 0.5f * el;
     }
     // the block's FP32 partial (as the real-space warp partials), added to the FP64 energy
@@ -2365,12 +2342,8 @@ int chunks_or(int tuned, long long base_blocks, int maxc, int per_sm = 12) {
 }
 
 void launch_lj_dense(const EvalArgs &a, cudaStream_t s) {
-    if (a.lj_list && a.lj_plane) {  // large beads: the symmetric Verlet list instead of every pair
+    if (a.lj_list) {  // large beads: the symmetric Verlet list instead of every pair
         k_lj_list_f32<<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
-        return;
-    }
-    if (a.lj_list) {
-        k_lj<1><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, s>>>(a);
         return;
     }
     const long long blocks8 = (long long)((a.max_mols + 15) / 16) * a.n_jobs;
@@ -2475,8 +2448,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             a.real_fix = 1;
         }
         else if (list_ok(a)) a.n_rj = list_chunks(a);  // k_kforce_f32's planes follow the real-space ones
-        if (a.lj_full) a.lj_plane = 1;
-        else a.lj_half = 1;
+        a.lj_half = !a.lj_full;
         launch_prep_f32(a, s);
         // capture order: the reciprocal chain (the critical path: three dependent
         // kernels) first, then the Lennard-Jones branch, the real-space kernel last
@@ -2499,7 +2471,7 @@ void launch_ewald(EvalArgs a, cudaStream_t s, unsigned long long *n, const Forks
             forks->put_lists(forks->put_arg, forks->side[1]);
         }
         if (a.lj_full) launch_lj_dense(a, forks->side[1]);
-        else k_lj<0><<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
+        else k_lj<<<dim3((a.max_mols + 3) / 4, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         k_intra_f32<<<dim3((a.max_mols + 127) / 128, a.n_jobs), 128, 0, forks->side[1]>>>(a);
         cudaEventRecord(forks->join[1], forks->side[1]);
         if (!put) real();
@@ -2610,7 +2582,6 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
     else if (ksk2_ok(a)) set_ksk2_chunks(a);
     const dim3 gr(tiles, a.n_rj, a.n_jobs);
     const dim3 gk(ktiles, a.n_sc, a.n_jobs), gf(tiles, a.n_kc, a.n_jobs);
-    const dim3 gl((a.max_mols + 3) / 4, a.n_jobs);
     const std::string n(name);
     if (n == "prep") {
         if (mixed) launch_prep_f32(a, s);
@@ -2632,17 +2603,11 @@ void launch_ewald_kernel(const EvalArgs &a0, bool mixed, const char *name, cudaS
         if (mixed) launch_kforce_f32(a, gf, s);
         else launch_kforce64(a, s);
     } else if (n == "combine") {
-        a.lj_plane = 1;
         if (mixed) k_combine_f32<<<dim3((a.max_mols + CMB - 1) / CMB, a.n_jobs), CMT, 0, s>>>(a);
         else launch_combine64(a, s);
     } else if (n == "lj") {
-        if (mixed) {
-            if (a.lj_full && a.ljf) a.lj_plane = 1;  // as the stepper's forked evaluation
-            if (a.lj_full) launch_lj_dense(a, s);
-            else k_lj<0><<<gl, 128, 0, s>>>(a);
-        } else {
-            launch_lj64(a, s);
-        }
+        if (mixed) launch_lj_dense(a, s);  // (lj_full, as the stepper evaluates)
+        else launch_lj64(a, s);
     }
 }
 

@@ -522,7 +522,7 @@ struct EvalArgs {
     const double *charge;
     const int *point, *list;
     const int *point_full, *list_full;  // symmetric lists built by the stepper's rebuild
-    int lj_full;                        // 1: Lennard-Jones over the symmetric list (no atomics)
+    int lj_full;                        // 1: Lennard-Jones over the symmetric list or every pair (no atomics)
     int lj_list;                        // mixed, symmetric lists valid: k_lj over them instead of every pair
     const KVec *kvec;
     const KCol *kcol;
@@ -542,10 +542,9 @@ struct EvalArgs {
     void *opos;            // mixed: wrapped oxygen positions, 4 floats per molecule, per slot
     float4 *opos32;        // FP64 evaluations: the same, for k_lj64's screening
     double *lj64;          // FP64 evaluations: Lennard-Jones oxygen forces, 4 doubles per molecule, per slot
-    int lj_half;           // mixed, forked, half lists: 1: k_lj adds into lj64 (zeroed by k_prep_f32)
+    int lj_half;           // mixed forces over half lists: 1: k_prep_f32 zeroes lj64, k_lj adds into it
     double *intra64;       // FP64 evaluations: intramolecular site and atom forces, 18 doubles per molecule, per slot
-    float4 *ljf;           // dense Lennard-Jones oxygen forces, per molecule, per slot (lj_plane)
-    int lj_plane;          // 1: k_lj_dense writes ljf and k_combine_f32 adds it to the O force
+    float4 *ljf;           // mixed, lj_full: Lennard-Jones oxygen forces, per molecule, per slot
     float *intra;          // mixed: intramolecular site and atom forces, 18 floats per molecule and slot
     void *phase;           // complex phase tables, per slot
     void *tan_sites;       // tangent of the site positions (mode 1), per slot
