@@ -46,3 +46,38 @@ def test_parts_match_systems_alone(gpu_lib, sizes):
         assert len(e["pot"]) == before + 50
         assert all(np.all(np.isfinite(v)) for v in e.values())
     ctx.close()
+
+
+# NVT: the parts draw the centroid's random numbers for their own systems and add the ring's
+# heat in a range of their own. A last system of the Suzuki-Chin kind, which keeps the step
+# in one part, leaves the others' systems, seeds and so random numbers as they are. The bound
+# is as above, on the impulse and on the heat, whose terms are the kinetic energy's size.
+@pytest.mark.parametrize("sizes,thermostat", [([(343, 32), (216, 32), (512, 32), (125, 32)], "PILE_G"), ([(512, 32)] * 2, "PILE_L"),
+                                              ([(216, 8)] * 4, "PILE_G")])
+def test_thermostatted_parts_match_one(gpu_lib, sizes, thermostat):
+    q = gpu_lib
+    st = [q.seeded_start(n, p, 298.0, seed=k, density_g_cm3=0.9) for k, (n, p) in enumerate(sizes + [(8, 2)])]
+    got, launches = [], []
+    for whole in (False, True):
+        kinds = [q.TROTTER] * len(sizes) + [q.SUZUKI_CHIN] * whole
+        ctx = q.Context([q.system_desc(s.n_mols, s.n_beads, s.box_bohr, seed=k, propagator=kind, thermostat=getattr(q, thermostat))
+                         for k, (s, kind) in enumerate(zip(st, kinds))], q.MIXED)
+        for s, t in zip(ctx.systems, st):
+            s.set_state(t.q, t.p)
+        ctx.init_forces()
+        ctx.sync()
+        before = ctx.kernel_launches()
+        ctx.run_steps(STEPS, is_nvt=True)
+        ctx.sync()
+        launches.append((ctx.kernel_launches() - before) // STEPS)
+        got.append([(s.get_state(), s.estimators()) for s in ctx.systems[:len(sizes)]])
+        ctx.close()
+    split = sum(n * p for n, p in sizes) >= 32000
+    assert (launches[0] > 20) == split  # a part's launches are some ten, a whole step's fourteen
+    dt = 0.25 * 41.341374575751
+    for (a, ea), (b, eb), (n, p) in zip(*got, sizes):
+        assert np.linalg.norm(a["p"] - b["p"]) <= 1e-4 * STEPS * dt * np.linalg.norm(b["f"])
+        assert len(ea["pot"]) == len(eb["pot"])
+        assert np.allclose(ea["heat"], eb["heat"], rtol=0, atol=1e-4 * eb["kin"][0])
+        assert np.allclose(ea["kin"], eb["kin"], rtol=1e-4)
+        assert np.allclose(ea["pot"], eb["pot"], rtol=0, atol=1e-4 * max(1.0, abs(eb["pot"][0])))
