@@ -1486,23 +1486,32 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         AL(tmp, 4 * ctx->total_sites);
         ctx->sites = tmp;
         tmp = nullptr;
-        AL(tmp, 4 * ctx->total_sites);
-        ctx->tan_sites = tmp;
-        tmp = nullptr;
         AL(tmp, 2 * ctx->total_phase);
         ctx->phase = tmp;
     }
-    {
+    // each form's own scratch; the force gradient's (of systems with odd beads) takes both:
+    // the derivative in FP32, the short-range finite differences in FP64
+    const bool gradient = !ctx->fd.h.empty();
+    AL(ctx->lj64, 4 * (ctx->total_sites / 3));
+    if (!ctx->mixed || gradient) {
+        AL(ctx->opos32, ctx->total_sites / 3);
+        AL(ctx->intra64, 6 * ctx->total_sites);
+    }
+    if (ctx->mixed) {
         float4 *tmp = nullptr;
         AL(tmp, ctx->total_sites / 3);
         ctx->opos = tmp;
+        AL(ctx->ljf, ctx->total_sites / 3);
+        AL(ctx->intra, 6 * ctx->total_sites);
+        AL(ctx->sites_fix, ctx->total_sites);
     }
-    AL(ctx->opos32, ctx->total_sites / 3);
-    AL(ctx->lj64, 4 * (ctx->total_sites / 3));
-    AL(ctx->intra64, 6 * ctx->total_sites);
-    AL(ctx->ljf, ctx->total_sites / 3);
-    AL(ctx->intra, 6 * ctx->total_sites);
-    AL(ctx->sites_fix, ctx->total_sites);
+    if (ctx->mixed && gradient) {
+        float4 *tmp = nullptr;
+        AL(tmp, ctx->total_sites);
+        ctx->tan_sites = tmp;
+        AL(ctx->dskp, (size_t)MAX_SC * ctx->total_k);
+        AL(ctx->wdsk, ctx->total_k);
+    }
     AL(ctx->rfix, (ctx->mixed ? 3 : 6) * ctx->total_sites);
     if (!ctx->mixed) {
         AL(ctx->real64_tab, (size_t)R64_INTERVALS * 16);
@@ -1539,10 +1548,8 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
     }
     AL(ctx->part, (size_t)MAX_PART * 3 * ctx->total_sites);
     AL(ctx->skp, (size_t)MAX_SC * ctx->total_k);
-    AL(ctx->dskp, (size_t)MAX_SC * ctx->total_k);
     AL(ctx->wsk, ctx->total_k);
     AL(ctx->wpk, (ctx->mixed ? 2 : 4) * ctx->total_k);
-    AL(ctx->wdsk, ctx->total_k);
     AL(ctx->energy, ctx->total_slots);
     AL(ctx->energy_aux, ctx->total_slots);
     AL(ctx->base.d, ctx->base.h.size());
