@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(128) k_sk_reduce(EvalArgs a) {
         if (half) {
             // the site chunks' sums, in chunk order with compensation in FP32
             float xs = 0.f, xc = 0.f, ys = 0.f, yc = 0.f;
-            if (MODE == 2) {  // compensated sums, rounded once
+            if (MODE == 2) {  // no compensation beside them
                 const int n_sc = (S.n_sites + a.sk_sites - 1) / a.sk_sites;
                 const float2 *pp = reinterpret_cast<const float2 *>(a.skp) + J.sk_off + k;
                 for (int c0 = 0; c0 < n_sc; c0 += 8) {
@@ -2401,21 +2401,21 @@ void launch_real_list(EvalArgs &a, cudaStream_t s) {
 
 // Whether a mixed evaluation's structure factors come from k_ksk2: batches of some 2000
 // waters' sites and more (one bead of 216 waters leaves either kernel mostly latency:
-// 6.2 us), of beads up to 4096 waters.
+// 6.2 us), with at most 192 sites a block within its planes.
 bool ksk2_ok(const EvalArgs &a) {
-    return a.mode == 0 && a.kpair && a.max_mols <= 4096 && a.max_kmax <= 32 &&
+    return a.mode == 0 && a.kpair && 3 * a.max_mols <= MAX_SC2 * 192 && a.max_kmax <= 32 &&
            (long long)a.max_mols * a.n_jobs >= 2048;
 }
-// Its site chunks, of the same size for every system of the batch: about two blocks an SM
-// (the real-space kernel runs beside it), of at most 512 sites. Steps by number of chunks:
-// 512 waters, 32 beads two 189.6 us, three 187.4, eight 189.6, sixteen 190.8; 343 waters, 16
-// beads four 96.5, six 90.3, sixteen 90.1; 216 waters, 32 beads two 106.0, six 93.1, sixteen
-// 91.9; 4096 waters sixteen 155, thirty-two 128, sixty-four 118.
+// Its site chunks, of the same size for every system of the batch: at most 192 sites, and
+// about two blocks an SM (the real-space kernel runs beside it). 512 waters, 32 beads: one
+// an SM 195.5 us a step, two 193.2, three 196.8; 343 waters, 16 beads: 99.0, 95.3, 93.4; 216
+// waters, 32 beads: 95.3, 93.9, 96.9. A batch that fills the SMs with whole beads keeps
+// them whole.
 void set_ksk2_chunks(EvalArgs &a) {
     const int ns = 3 * a.max_mols;
     const long long base = (long long)ksk2_blocks(a) * a.n_jobs, two = 2 * 152;
     const int n_sc = a.tune_sc > 0 ? a.tune_sc : (int)std::max(1LL, (two + base / 2) / base);  // (to the nearest)
-    a.n_sc = std::max(std::min(n_sc, MAX_SC2), (ns + 511) / 512);
+    a.n_sc = std::max(std::min(n_sc, MAX_SC2), (ns + 191) / 192);
     a.sk_sites = std::max(16, ((ns + a.n_sc - 1) / a.n_sc + 15) / 16 * 16);
     a.n_sc = (ns + a.sk_sites - 1) / a.sk_sites;
 }

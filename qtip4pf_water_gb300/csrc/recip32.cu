@@ -23,14 +23,15 @@ namespace {
 // + i (T3 + T4), S(-kz) = T1 + T2 + i (T4 - T3). Sites lie in shared memory a record each
 // (X, Y, Zr, Zi), so that the lanes of a warp, on neighbouring (kx, ky) and mostly one
 // group of |kz|, read one or two 128-byte lines an access; CH2 sites at a time, double-
-// buffered by cp.async. Sums: 16 sites in FP32, three of these a chunk, the chunks with
-// compensation (Kahan, in shared memory: the 64 registers would cost a third of the warps),
-// and so the blocks (k_sk_reduce); k_ksk adds 32 sites before it compensates. Without the
-// compensation (192 sites in a plain sum) the kernel took 34.9 us instead of 38.3 at 512
-// waters, 32 beads, but sites in phase, as in a crystal, summed with a larger error: forces of
-// like ions on a lattice 8.4e-5 off, 7.3e-5 with it (k_ksk 1.1e-4), random sites 2.3e-7 (2.6e-7).
-// Compensating every second chunk instead gains 0.5 % of a step at most.
-constexpr int CH2 = 48, SUB2 = 16;
+// buffered by cp.async. Sums: 16 sites in FP32, six of these HELD chunks, the two halves of a
+// block (at most 192 sites, see set_ksk2_chunks in forces.cu; the first half's sums wait in
+// shared memory), the blocks with compensation (k_sk_reduce). Errors against FP64 sums of the
+// same factors, 1536 sites: random phases 1.05e-7 of S (k_ksk's 32 sites and compensation from
+// there on 1.60e-7), sites in phase as in a crystal 3.34e-8 (k_ksk 3.6e-8 in four blocks, 3.3e-8
+// in sixteen); with 192 sites in a plain sum 3.5e-8. Kahan's compensation after each chunk (3.2e-8)
+// takes as much shared memory again: 512 waters, 32 beads 34.9 -> 38.3 us, 1000 waters, 16 beads 5 %
+// of a step.
+constexpr int CH2 = 48, SUB2 = 16, HELD = 2;
 
 __host__ __device__ constexpr int ksk2_km4(int km1) { return (km1 + 3) & ~3; }
 // floats a site record takes: an odd number of 16-byte units, so that the 16-byte
@@ -84,10 +85,16 @@ __global__ void __launch_bounds__(256) k_ksk2(EvalArgs a) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) T[h][k][0] = T[h][k][1] = zero;
     stage(0);
-    // this thread's running sums over the chunks and their compensations, 16 bytes each
-    ulonglong2 *sum = reinterpret_cast<ulonglong2 *>(rec + 2 * CH2 * R) + threadIdx.x, *comp = sum + 8 * blockDim.x;
-    const F2 minus = pk(-1.f, -1.f);
+    ulonglong2 *held = reinterpret_cast<ulonglong2 *>(rec + 2 * CH2 * R) + threadIdx.x;  // the first half's sums
     for (int ci = 0; ci < nchunk; ++ci) {
+        if (ci == HELD) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                F2 *c = T[k >> 2][k & 3];
+                held[k * blockDim.x] = make_ulonglong2(c[0].v, c[1].v);
+                c[0] = c[1] = zero;
+            }
+        }
         __syncthreads();  // every thread is done with buffer (ci + 1) & 1
         if (ci + 1 < nchunk) stage(ci + 1);
         else cp_async_commit();
@@ -135,36 +142,17 @@ __global__ void __launch_bounds__(256) k_ksk2(EvalArgs a) {
                     T[h][k][1] = add2(T[h][k][1], v[h][k][1]);
                 }
         }
-        // the chunk's sums join the running ones (Kahan; after the last chunk T holds them)
-        const bool more = ci + 1 < nchunk;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            F2 *c = T[k >> 2][k & 3];
-            F2 s0 = c[0], s1 = c[1], e0 = zero, e1 = zero;
-            if (ci > 0) {
-                const ulonglong2 o = sum[k * blockDim.x];
-                if (ci > 1) {
-                    const ulonglong2 q = comp[k * blockDim.x];
-                    e0 = F2{q.x};
-                    e1 = F2{q.y};
-                }
-                const F2 y0 = add2(c[0], e0), y1 = add2(c[1], e1);
-                s0 = add2(F2{o.x}, y0);
-                s1 = add2(F2{o.y}, y1);
-                e0 = add2(fma2(s0, minus, F2{o.x}), y0);
-                e1 = add2(fma2(s1, minus, F2{o.y}), y1);
-            }
-            if (more) {
-                sum[k * blockDim.x] = make_ulonglong2(s0.v, s1.v);
-                if (ci > 0) comp[k * blockDim.x] = make_ulonglong2(e0.v, e1.v);
-                c[0] = c[1] = zero;
-            } else {
-                c[0] = add2(s0, e0);
-                c[1] = add2(s1, e1);
-            }
-        }
     }
     if (t >= np) return;
+    if (nchunk > HELD) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const ulonglong2 o = held[k * blockDim.x];
+            F2 *c = T[k >> 2][k & 3];
+            c[0] = add2(c[0], F2{o.x});
+            c[1] = add2(c[1], F2{o.y});
+        }
+    }
     float2 *skp = reinterpret_cast<float2 *>(a.skp) + (size_t)sc * a.total_k + J.sk_off;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -189,7 +177,7 @@ __global__ void __launch_bounds__(256) k_ksk2(EvalArgs a) {
 }
 
 size_t ksk2_smem(int kmax, int threads) {
-    return (size_t)2 * CH2 * ksk2_record(kmax + 1) * sizeof(float) + (size_t)threads * 16 * sizeof(ulonglong2);
+    return (size_t)2 * CH2 * ksk2_record(kmax + 1) * sizeof(float) + (size_t)threads * 8 * sizeof(ulonglong2);
 }
 
 }  // namespace

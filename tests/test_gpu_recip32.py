@@ -4,8 +4,8 @@ phase (ions on a lattice, whose Bragg vectors add every site's charge in one dir
 
 The bound on a site's force is the sum over the vectors of 2 c |k| |q| (|S| 2^-24 n + |dS|):
 n = 24 roundings between S and the force (weights, column factors, phases to two powers, |kz|
-sums and the closing products), and dS = 2^-24 (30 sum |q|) for the chains of 16 and 3 site
-sums, their compensated sums, the phases and the column factors of each of them."""
+sums and the closing products), and dS = 2^-24 (30 sum |q|) for the chains of 16 sites and
+six such sums, the halves and blocks they join, the phases and the column factors."""
 import numpy as np
 import pytest
 
