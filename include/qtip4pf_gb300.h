@@ -82,7 +82,9 @@ typedef struct qtg_system_info {
 
 /* ---- context --------------------------------------------------------------- */
 /* Creates a context on the current CUDA device holding n_systems systems.
- * All device memory is allocated here; no later call allocates. */
+ * All device memory is allocated here; no later call allocates. QTG_ERR_ARG: a field
+ * out of range, or a cell so long (or a tolerance so small) that k_max exceeds 63 (QTG_MIXED:
+ * 63 along z, 127 along x and y). */
 qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precision, qtg_ctx **out);
 void qtg_destroy(qtg_ctx *ctx);
 const char *qtg_last_error(const qtg_ctx *ctx);

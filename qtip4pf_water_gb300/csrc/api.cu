@@ -1142,6 +1142,12 @@ qtg_status qtg_create(const qtg_system_desc *systems, int n_systems, int precisi
         S.rc_sq = rc * rc;
         const double kc = 2.0 * acc * kappa;
         S.k_max = (int)(kc * max_box / (2.0 * PI_REF));
+        // a column of 2 |kz| + 1 vectors has to fit a force batch (128), and the phase rows of
+        // all three dimensions the shared memory of the structure factors (half the entries FP64)
+        if ((int)(kc * S.box[2] / (2.0 * PI_REF)) > 63 || S.k_max > (ctx->mixed ? 127 : 63)) {
+            qtg_destroy(ctx);
+            return QTG_ERR_ARG;
+        }
         S.ewald_pref = 2.0 * kappa / sqrt(PI_REF);
         S.kappaf = (float)kappa;
         S.kappa_sqf = (float)(kappa * kappa);

@@ -56,3 +56,35 @@ def test_coherent_sites_at_the_charge_scale(gpu_lib, top):
     e_got = s.kwald(sites, got, charge)
     assert np.linalg.norm(got - ref) < 1e-9 * np.linalg.norm(ref)
     assert abs(e_got - e_ref) < 1e-9 * abs(e_ref)
+
+
+# cells so long that k_max reaches the kernels' limit: 2 |kz| + 1 vectors a column in a batch of
+# 128, and phase rows of k_max + 1 entries in shared memory. Beyond it the cell is refused.
+@pytest.mark.parametrize("axis,ratio,kmax", [(2, 7.1, 62), (0, 7.1, 62), (2, 7.5, 65), (0, 7.5, 65)])
+def test_long_cells(gpu_lib, axis, ratio, kmax):
+    from oracle.binding import Oracle
+
+    q = gpu_lib
+    st = q.seeded_start(27, 1, 298.0, seed=4)
+    stretch = np.ones(3)
+    stretch[axis] = ratio
+    box = st.box_bohr * stretch
+    x = st.q.reshape(27, 3, 3)
+    pos = np.ascontiguousarray((x - x[:, :1] + x[:, :1] * stretch).reshape(1, -1))
+    o = Oracle(27, 1, box, 298.0, 0.25, eps_ewald=1e-6)
+    point, lst, _ = o.build_lists(pos)
+    ref = np.zeros_like(pos)
+    e_ref, _ = o.force_eval_trotter(pos, ref, point, lst)
+    for prec, tol in ((q.FP64, 1e-9), (q.MIXED, 1e-4)):
+        if kmax > 63 and (prec == q.FP64 or axis == 2):
+            with pytest.raises(q.QtgError) as ei:
+                q.System.create(27, 1, box, precision=prec, propagator=q.TROTTER)
+            assert ei.value.status == 1
+            continue
+        s = q.System.create(27, 1, box, precision=prec, propagator=q.TROTTER)
+        assert s.info.k_max == kmax
+        got = np.zeros_like(pos)
+        e_got, _ = s.force_eval_trotter(pos, got, s.charges(), point, lst)
+        assert np.linalg.norm(got - ref) < tol * np.linalg.norm(ref)
+        self_e = s.info.kappa / np.sqrt(np.pi) * float((s.charges() ** 2).sum())
+        assert abs(e_got - e_ref) < (1e-9 if prec == q.FP64 else 1e-6) * max(abs(e_ref), self_e)
