@@ -321,7 +321,9 @@ struct qtg_ctx {
     int n_sc_odd = 0;
     ColWork *colwork = nullptr;
     int n_colwork = 0;
-    double *cw_part = nullptr;    // [n_colwork][4] block partials of the ordered system sums
+    // block partials of the ordered system sums, [n_colwork][4], and [n_colwork] for the ring's
+    // heat in a step of parts (enqueue_parts)
+    double *cw_part = nullptr;
     unsigned *fin_ticket = nullptr;  // systems closed by a fused end step
     unsigned *cw_ticket = nullptr;  // [n_sys] arrival tickets of those sums
     // run state
@@ -725,7 +727,12 @@ bool rebuild_beside_forces(const qtg_ctx *c, int sys) {
 // The parts a step of all systems goes in (first systems; a closing entry): up to four of
 // about the same pair work for second-order systems of the mixed form with some 32,000
 // molecule-beads and more, each enough for the kernels of large batches (which lay their
-// partial sums out their own way in shared scratch); else one.
+// partial sums out their own way in shared scratch); else one. Steps in one part and in
+// parts, by molecule-beads: 8 x (512, 8) 32,800: 339 and 324 us; 2 x (512, 32) the same: 350 and
+// 336; 24 x (216, 8) 41,500: 319 and 322; 8 x (216, 32) 55,300: 462 and 426; below the limit
+// 4 x (216, 32) 27,600: 252 and 241; 32 x (64, 8) 16,400: 157 and 160; 4 x (512, 8) 16,400: 186 and
+// 204; 8 x (216, 8) 13,800: 137 and 173; 4 x (64, 32) 8,200: 97 and 147. Between some 20,000 and 32,000
+// parts gain a few percent or nothing, below they lose.
 std::vector<int> step_parts(const qtg_ctx *c) {
     std::vector<int> lo(1, 0);
     const auto molecules = [&](int s) { return (long long)c->sys_h[s].n_beads * c->sys_h[s].n_mols; };
@@ -754,8 +761,9 @@ std::vector<int> step_parts(const qtg_ctx *c) {
 
 // The step's ring and end-step kernels are bound by FP64 instructions, the force kernels
 // by FP32 ones. In parts of the systems on streams of their own, one ring update behind the
-// other, a part's forces run beside the next one's ring update and the one before's end
-// step. 48 uneven replicas (277,000 molecule-beads) 2409 us a step in one part, 2350 in two,
+// other, a part's forces run beside the next ones' ring updates, and the end steps, once every
+// ring update and the lists are done, beside the forces of the parts that are still at them.
+// 48 uneven replicas (277,000 molecule-beads) 2409 us a step in one part, 2350 in two,
 // 2321 in four; 12 (59,000) 583, 571, 525; 4 of 216 waters, 8 beads (6,900), which fill the
 // GPU only together, 91 and 115 in two.
 void enqueue_parts(qtg_ctx *c, const std::vector<int> &lo, int nvt, bool pile_g) {
@@ -770,7 +778,8 @@ void enqueue_parts(qtg_ctx *c, const std::vector<int> &lo, int nvt, bool pile_g)
         cudaStream_t st = h ? c->part_of[h - 1].stream : main;
         RingArgs r = ring_args(c, -1, RF_KICK | RF_FWD | RF_CAYLEY | RF_BACK | RF_DISP | (nvt ? RF_THERMO : 0));
         columns(r, h);
-        // (its partial sums are laid out otherwise than an end step's, which may run beside it)
+        // (its partial sums are laid out otherwise than an end step's: a range of their own, so
+        // that neither depends on the other's parts being done)
         r.cw_part = c->cw_part + 4 * (size_t)c->n_colwork;
         r.pile_g = pile_g ? 1 : 0;
         r.n_draw = lo[h + 1] - lo[h];  // (as in enqueue_step)

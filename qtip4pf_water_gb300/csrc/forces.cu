@@ -1678,7 +1678,13 @@ void launch_ksk(const EvalArgs &a, dim3 grid, cudaStream_t s) {
     else k_ksk<MODE, 4><<<grid, KT, ksk_smem(a.max_kmax), s>>>(a);
 }
 
-// the FP32 k-force kernel for the largest |kz| of the batch (the general form beyond 32)
+// The FP32 k-force kernel for the largest |kz| of the batch (the general form beyond 32). An
+// instance keeps its Z rows in registers: 8, 10 (96 and 103 registers) and 14 (128) are the last
+// that fit four or five blocks an SM, straight bodies end there (a switch of fourteen), and
+// 16, 24 and 32 loop with a test a |kz|. Against the looping form with X in shared memory, alone:
+// k_max 9 to 11 as fast or 3 % slower (1000 waters, 16 beads 50.4 -> 52.4 us), 12 (1300 waters, 12
+// beads) 88.6 -> 58.2, 13 64.8 -> 46.7, 14 44.0 -> 33.1, 15 57.2 -> 42.6, 16 91.2 -> 63.6; long cells 17
+// 27.0 -> 24.5, 24 34.7 -> 30.7, 28 102.9 -> 59.1. An instance of 12 is no faster than 14 at 11 and 12.
 void launch_kforce_f32(const EvalArgs &a, dim3 grid, cudaStream_t s) {
     // two sites a thread (the block covers 2 FT sites: grid.x halves)
     const size_t sm = (size_t)(a.max_kmax + 1) * 2 * FT * sizeof(float2);

@@ -553,8 +553,8 @@ struct EvalArgs {
     // (units of 2^-40 Hartree/bohr, [total_sites][3]; zeroed by k_prep_f32, summed by
     // integer atomics, so the sum does not depend on their order), read by
     // k_combine_f32 when real_fix is set
-    // FP64: the same of k_real64, [total_sites][3][2]: a high limb in units of 2^-8 and a
-    // low limb in units of 2^-60 (zeroed by k_prep64, read by k_combine64)
+    // FP64: k_real64's, [total_sites][3][2], in units of q_top^2 kappa^2: a high limb worth
+    // 2^-24 and a low limb worth 2^-56 a unit (zeroed by k_prep64, read by k_combine64)
     long long *rfix;
     int real_fix;
     const double *real64_tab;  // FP64: the pair-function table (real64_table)

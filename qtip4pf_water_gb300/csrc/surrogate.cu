@@ -595,8 +595,7 @@ __device__ __forceinline__ void store16(uint8_t *rows, int K, uint8_t *cols, int
 // TMEM quadrant w mod 4 and the 16 columns from 16 (w / 4) on of every layer. SiLU's
 // derivative is kept in registers from the forward pass, the transposed copies are stored
 // two rows at a time, and the next tile's inputs are loaded while this one is worked on.
-// 442368 rows: 800 us with four warps, one row a thread and two-byte stores; see
-// qtg_mlp_train_batch's launch.
+// 442368 rows: 800 us with four warps, one row a thread and two-byte stores, 240 so.
 __global__ void __launch_bounds__(TT, 1) k_mlp_train(TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
