@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
     const i64 *sysc = a.real64_sys + 4 * J.sys;
     if (threadIdx.x < 12) {
         const int d = threadIdx.x >> 2, n = (threadIdx.x & 3) - 1;
-        // (sides that r_c does not reach across need no second image, see below)
+        // (sides of which r_c does not reach half need no second image, see below)
         image[d][n + 1] = n < 2 ? n * sysc[d] : S.kappa * S.box[d] < 64.0 ? sysc[d] >> 1 : 0x7fffffffffffffffll;
     }
     __syncthreads();
@@ -276,20 +276,10 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
         for (int b = lane; b < cnt; b += 32) {
             const int c = W.code[b], img = c >> 9;
             const RSite &p = W.si[(c >> 5) & 15], &s = W.sj[c & 31];
-            i64 y0 = p.y[0] - s.y[0] - image[0][img & 3], y1 = p.y[1] - s.y[1] - image[1][(img >> 2) & 3],
-                y2 = p.y[2] - s.y[2] - image[2][(img >> 4) & 3];
+            const i64 y0 = p.y[0] - s.y[0] - image[0][img & 3], y1 = p.y[1] - s.y[1] - image[1][(img >> 2) & 3],
+                      y2 = p.y[2] - s.y[2] - image[2][(img >> 4) & 3];
             // u in units of 2^-56; a fixed-point pair has u in [2^RI_LO, 2^(RI_LO + RI_OCT))
-            i64 u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
-            if (u >= uc) {
-                // beyond r_c: the screen's FP32 image of a pair some 1e-7 of a side from half
-                // a box may be the farther one, and r_c reaches half the shortest side (the
-                // screen's margin lets in one pair in 10^5 that comes here)
-                const auto nearer = [](i64 y, const i64 *im) { return y > im[3] ? y - im[2] : y < -im[3] ? y + im[2] : y; };
-                y0 = nearer(y0, image[0]);
-                y1 = nearer(y1, image[1]);
-                y2 = nearer(y2, image[2]);
-                u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
-            }
+            const i64 u = sqr62(split62(y0 * 8)) + sqr62(split62(y1 * 8)) + sqr62(split62(y2 * 8));
             i64 fx = 0, fy = 0, fz = 0;
             if (u < uc && (unsigned)((int)(u >> 32) - RI_BOT) < (unsigned)(RI_TOP - RI_BOT)) {
                 const int z = __clz((int)(u >> 32));
@@ -310,10 +300,14 @@ __global__ void __launch_bounds__(32 * RW) k_real64(EvalArgs a, int n_ch) {
                 fx = mul62(w, split62(y0 << up));
                 fy = mul62(w, split62(y1 << up));
                 fz = mul62(w, split62(y2 << up));
-            } else if (u < uc || uc < 0) {
+            } else {
+                // too near, or beyond r_c: the screen's margin lets in some pairs (one in 10^5),
+                // and of a pair 1e-7 of a side from half a box its FP32 image may be the farther
+                // one, where r_c reaches half the shortest side. Decided in FP64
+                const auto nearer = [](i64 y, const i64 *im) { return y > im[3] ? y - im[2] : y < -im[3] ? y + im[2] : y; };
                 i64 *rf = a.rfix + 6 * (size_t)J.site_off;
-                e += slow_pair(a, S, y0, y1, y2, p.q, s.q, rf + 6 * (i0 + ((c >> 5) & 15)),
-                               rf + 6 * (((tI + d) % T) * 32 + (c & 31)));
+                e += slow_pair(a, S, nearer(y0, image[0]), nearer(y1, image[1]), nearer(y2, image[2]), p.q, s.q,
+                               rf + 6 * (i0 + ((c >> 5) & 15)), rf + 6 * (((tI + d) % T) * 32 + (c & 31)));
             }
             W.f[0][b] = fx;
             W.f[1][b] = fy;

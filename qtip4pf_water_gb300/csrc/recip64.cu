@@ -329,9 +329,10 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
     __shared__ unsigned top[4];
     double e = 0.0;
     int code = -1;
-    bool bad = false;  // a site of the configuration is not finite (k_prep64)
+    // whether a site of the configuration is not finite (k_prep64): on its way during the sums
     const int words = prep64_blocks(a.max_mols);
-    for (int i = threadIdx.x; i < words; i += 128) bad |= a.nonfinite[(size_t)J.slot * words + i] != 0;
+    const int *nf = a.nonfinite + (size_t)J.slot * words;
+    int word = (int)threadIdx.x < words ? nf[threadIdx.x] : 0;
     if (on) {
         const KVec kv = a.kvec[S.kvec_off + k];
         const double w = 2.0 * kv.coef * (kv.twin ? 2.0 : 1.0);  // kx = 0, ky > 0: its conjugate partner too
@@ -346,7 +347,8 @@ __global__ void __launch_bounds__(128) k_sk_reduce64(EvalArgs a) {
         code = a.kpk[S.kvec_off + k];
     }
     const double nan = __hiloint2double(0x7ff80000, 0);
-    bad = __syncthreads_or(bad);
+    for (int i = threadIdx.x + 128; i < words; i += 128) word |= nf[i];
+    const bool bad = __syncthreads_or(word);
     if (bad) e = nan;
     const int az = code & 255;
     double sx = 0.0, sy = 0.0, dx = 0.0, dy = 0.0;
