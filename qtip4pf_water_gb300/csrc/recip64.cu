@@ -128,11 +128,11 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
     const int mol = s / 3, kind = s - 3 * mol;
     const double *q = a.pos + J.pos_off;
     const double g = a.c.gamma_vs;
+    const bool own = s < ns;
     double x = 0.0;
-    if (s >= ns) {
-    } else if (a.sites_are_input || kind != 0) {
+    if (own && (a.sites_are_input || kind != 0)) {
         x = q[3 * s + d];
-    } else {
+    } else if (own) {
         // M site (forces.cpp:558-564)
         x = g * q[9 * mol + d] + 0.5 * (1.0 - g) * (q[9 * mol + 3 + d] + q[9 * mol + 6 + d]);
         const double t = q[9 * mol + d] * S.inv_box[d];
@@ -140,10 +140,10 @@ __global__ void __launch_bounds__(128) k_prep64(EvalArgs a) {
         reinterpret_cast<float *>(a.opos32)[at] = (float)((t - floor(t)) * S.box[d]);
         a.lj64[at] = 0.0;  // k_lj64's forces
     }
-    const double chg = d == 0 && s < ns ? a.charge[S.chg_off + s] : 0.0;
+    const double chg = d == 0 && own ? a.charge[S.chg_off + s] : 0.0;
     const int bad = __syncthreads_or(not_finite(x) || not_finite(chg));
     if (threadIdx.x == 0) a.nonfinite[(size_t)J.slot * gridDim.x + blockIdx.x] = bad;
-    if (s >= ns) return;
+    if (!own) return;
     // wrapped with one rounding (while the quotient is exact enough for it), and the 64-bit
     // fraction of the box
     const double t = x * S.inv_box[d];
